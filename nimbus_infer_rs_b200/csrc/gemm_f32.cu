@@ -1,0 +1,246 @@
+// Matrix product of fp32 rows with fp32 weights, out[M,N] = act(X W^T + bias) (+ residual): the
+// prompts of the true 32-bit path.  Every product and sum is an fp32 multiply-add.
+//
+// Bound by the rate of those multiply-adds.  They are issued two at a time (fma.rn.f32x2): an
+// accumulator is a pair, the sum over the even and the sum over the odd places of K, so both
+// operands of the packed instruction are two neighbouring numbers of a row as they lie in
+// memory and nothing has to be duplicated into pairs.  Shared memory holds a block of K as
+// [pair of K][row], filled with 8-byte cp.async straight from the rows; a thread owns 8 x 8
+// outputs and reads 4 + 4 16-byte words for its 64 packed multiply-adds.  A CTA is 64 threads and
+// a 64 x 64 tile: small enough that the tiles of a prompt of a small model deal out evenly
+// over 148 SMs, and several of them to an SM hide each other's barriers.  Where even those are
+// too few, K is cut among the CTAs of a cluster, whose sums meet in distributed shared memory.
+//
+// Measured against the kernels of gemm_simt.cu (us, rows x columns x K): 2024x2304x768 178 (190),
+// 2024x3072x768 257 (378), 2024x768x3072 323 (329), 333x2304x768 49 (60), 333x768x3072 70 (133),
+// 65x768x768 17 (35), 65x768x3072 29 (139).  At 40 TFLOP/s it is bound by what shared memory hands
+// out: a packed multiply-add needs 2 bytes a lane, 64 outputs a thread allow no less.
+//
+// Reference analogue: Mat::gemm_into (src/model.rs:88-133): y[i][j] = dot(x[i], Wt[j]).
+#include "gemm_f32.cuh"
+
+namespace {
+
+constexpr int TM = 64, TN = 64;
+constexpr int KP = 8;                 // pairs of K in a block (16 numbers)
+constexpr int LD = TM + 4;            // in pairs: the eight pairs of a row fall into different banks
+constexpr int STAGES = 3;
+constexpr int THREADS = 64;
+constexpr int STAGE_PAIRS = 2 * KP * LD;
+
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float pair_sum(unsigned long long v) {
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(lo), "=f"(hi) : "l"(v));
+  return lo + hi;
+}
+// eight bytes into shared memory, or zeros where `live` is false (the address is then not read)
+__device__ __forceinline__ void copy8(uint32_t dst, const float* src, bool live) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src), "r"(live ? 8 : 0)
+               : "memory");
+}
+
+// SPLITS: CTAs of a cluster (along x) that share a tile, each with its part of K.
+template <int SPLITS, typename TOut>
+__global__ void __launch_bounds__(THREADS, 4)
+gemm_f32_kernel(const float* X, const float* __restrict__ W, const float* __restrict__ bias,
+                const float* residual, TOut* out, int M, int N, int K, int act, int k_part,
+                int n_tiles) {
+  __shared__ __align__(16) unsigned long long tiles[STAGES * STAGE_PAIRS];
+  const int tid = threadIdx.x;
+  const int tile = blockIdx.x / SPLITS, part = blockIdx.x % SPLITS;
+  const int m0 = (tile / n_tiles) * TM, n0 = (tile % n_tiles) * TN;
+  const int k_lo = part * k_part, k_hi = min(K, k_lo + k_part);
+  const int n_blocks = k_hi > k_lo ? (k_hi - k_lo + 2 * KP - 1) / (2 * KP) : 0;
+  // loads: eight neighbouring lanes take the eight pairs of a row's block, eight rows a pass
+  const int lp = tid & 7, lr = tid >> 3;
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(tiles);
+
+  auto fetch = [&](int block) {
+    const int k = k_lo + block * 2 * KP + lp * 2;
+    const bool k_ok = k < k_hi;           // K is even: a pair is in or out as a whole
+    const uint32_t dst = base + (uint32_t)(((block % STAGES) * STAGE_PAIRS + lp * LD + lr) * 8);
+#pragma unroll
+    for (int i = 0; i < TM / 8; ++i) {
+      const int r = m0 + lr + i * 8;
+      const bool ok = k_ok && r < M;
+      copy8(dst + i * 64, X + (ok ? (size_t)r * K + k : 0), ok);
+    }
+#pragma unroll
+    for (int i = 0; i < TN / 8; ++i) {
+      const int r = n0 + lr + i * 8;
+      const bool ok = k_ok && r < N;
+      copy8(dst + KP * LD * 8 + i * 64, W + (ok ? (size_t)r * K + k : 0), ok);
+    }
+  };
+
+  const int ty = tid >> 3, tx = tid & 7;
+  unsigned long long acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
+
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) {
+    if (s < n_blocks) fetch(s);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  }
+  for (int b = 0; b < n_blocks; ++b) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();            // the block is there for all, and all are done with the one before
+    if (b + STAGES - 1 < n_blocks) fetch(b + STAGES - 1);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    const unsigned long long* xs = tiles + (b % STAGES) * STAGE_PAIRS + ty * 2;
+    const unsigned long long* ws = tiles + (b % STAGES) * STAGE_PAIRS + KP * LD + tx * 2;
+#pragma unroll
+    for (int p = 0; p < KP; ++p) {
+      // rows c*16 + ty*2 + {0, 1}: a warp's reads are one broadcast and one unbroken line
+      ulonglong2 a[4], w[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        a[c] = *reinterpret_cast<const ulonglong2*>(xs + p * LD + c * 16);
+        w[c] = *reinterpret_cast<const ulonglong2*>(ws + p * LD + c * 16);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          fma2(acc[i][j], (i & 1) ? a[i >> 1].y : a[i >> 1].x, (j & 1) ? w[j >> 1].y : w[j >> 1].x);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+
+  float v[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[i][j] = pair_sum(acc[i][j]);
+
+  // Parts of K: every CTA leaves its sums in its own shared memory ([place][thread]: conflict
+  // free), then finishes 8 / SPLITS of each thread's rows from all of them.
+  int i_lo = 0, i_hi = 8;
+  if constexpr (SPLITS > 1) {
+    float* mine = reinterpret_cast<float*>(tiles);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) mine[(i * 8 + j) * THREADS + tid] = v[i][j];
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    i_lo = part * (8 / SPLITS);
+    i_hi = i_lo + 8 / SPLITS;
+    uint32_t peer[SPLITS];
+#pragma unroll
+    for (int s = 0; s < SPLITS; ++s)
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(peer[s]) : "r"(base), "r"(s));
+#pragma unroll
+    for (int i = 0; i < 8 / SPLITS; ++i) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float sum = 0.0f;
+#pragma unroll
+        for (int s = 0; s < SPLITS; ++s) {
+          float t;
+          asm volatile("ld.shared::cluster.f32 %0, [%1];\n"
+                       : "=f"(t)
+                       : "r"(peer[s] + (uint32_t)((((i_lo + i) * 8 + j) * THREADS + tid) * 4))
+                       : "memory");
+          sum += t;
+        }
+        v[i][j] = sum;          // this CTA's rows move to the front
+      }
+    }
+    // nobody leaves while another still reads its shared memory
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  }
+
+  const bool pairs = (N % 2 == 0) && (uintptr_t)out % 8 == 0 && (uintptr_t)residual % 8 == 0;
+#pragma unroll
+  for (int i = 0; i < 8 / SPLITS; ++i) {
+    const int place = i_lo + i;
+    const int m = m0 + (place >> 1) * 16 + ty * 2 + (place & 1);
+    if (m >= M) continue;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int n = n0 + c * 16 + tx * 2;
+      if (n >= N) continue;
+      const size_t o = (size_t)m * N + n;
+      const bool two = n + 1 < N;
+      float r0 = 0.0f, r1 = 0.0f;
+      if (residual) {
+        if (pairs) {
+          const float2 r = *reinterpret_cast<const float2*>(residual + o);
+          r0 = r.x;
+          r1 = r.y;
+        } else {
+          r0 = residual[o];
+          if (two) r1 = residual[o + 1];
+        }
+      }
+      float y0 = v[i][2 * c], y1 = v[i][2 * c + 1];
+      if (bias) {
+        y0 += bias[n];
+        if (two) y1 += bias[n + 1];
+      }
+      y0 = nb_apply_act(y0, act) + r0;
+      y1 = nb_apply_act(y1, act) + r1;
+      if (pairs && sizeof(TOut) == 4) {
+        *reinterpret_cast<float2*>(out + o) = make_float2(y0, y1);
+      } else {
+        out[o] = nb_from_f32<TOut>(y0);
+        if (two) out[o + 1] = nb_from_f32<TOut>(y1);
+      }
+    }
+  }
+}
+
+template <int SPLITS, typename TOut>
+cudaError_t launch(const float* X, const float* W, const float* bias, const float* residual, TOut* out,
+                   int M, int N, int K, int act, long long tiles, cudaStream_t stream) {
+  const int blocks = (K + 2 * KP - 1) / (2 * KP);
+  const int k_part = (blocks + SPLITS - 1) / SPLITS * 2 * KP;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * SPLITS));
+  cfg.blockDim = dim3(THREADS);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = SPLITS;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = SPLITS > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, gemm_f32_kernel<SPLITS, TOut>, X, W, bias, residual, out, M, N, K,
+                            act, k_part, (N + TN - 1) / TN);
+}
+
+}  // namespace
+
+template <typename TOut>
+bool nb_gemm_f32_tiles(const float* X, const float* W, const float* bias, const float* residual,
+                       TOut* out, int M, int N, int K, int act, cudaStream_t stream,
+                       cudaError_t* err) {
+  // pairs of K are copied as 8-byte words
+  if (K % 2 || (uintptr_t)X % 8 || (uintptr_t)W % 8) return false;
+  const long long tiles = (long long)((M + TM - 1) / TM) * ((N + TN - 1) / TN);
+  if (tiles * 8 > 0x7fffffffLL) return false;
+  // K is cut until there are two CTAs an SM, but not into parts of less than 128 numbers
+  int splits = 1;
+  while (splits < 8 && tiles * splits < 2 * 148 && K / (2 * splits) >= 128) splits *= 2;
+  switch (splits) {
+    case 1: *err = launch<1, TOut>(X, W, bias, residual, out, M, N, K, act, tiles, stream); break;
+    case 2: *err = launch<2, TOut>(X, W, bias, residual, out, M, N, K, act, tiles, stream); break;
+    case 4: *err = launch<4, TOut>(X, W, bias, residual, out, M, N, K, act, tiles, stream); break;
+    default: *err = launch<8, TOut>(X, W, bias, residual, out, M, N, K, act, tiles, stream); break;
+  }
+  return true;
+}
+
+template bool nb_gemm_f32_tiles<float>(const float*, const float*, const float*, const float*, float*,
+                                       int, int, int, int, cudaStream_t, cudaError_t*);
+template bool nb_gemm_f32_tiles<__nv_bfloat16>(const float*, const float*, const float*, const float*,
+                                               __nv_bfloat16*, int, int, int, int, cudaStream_t,
+                                               cudaError_t*);

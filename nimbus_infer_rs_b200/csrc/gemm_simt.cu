@@ -5,7 +5,7 @@
 //
 // Reference analogue: Mat::gemm_into / gemv_into (src/model.rs:65-133): y[i][j] = dot(x[i],
 // Wt[j]) with Wt stored (out, in).
-#include "common.cuh"
+#include "gemm_f32.cuh"
 
 namespace {
 
@@ -230,6 +230,14 @@ gemm_simt_large_kernel(const TIn* __restrict__ X, const TW* __restrict__ W,
 template <typename TIn, typename TW, typename TOut>
 int launch(const void* X, const void* W, const float* bias, const float* residual, void* out,
            int M, int N, int K, int act, cudaStream_t stream) {
+  if constexpr (sizeof(TIn) == 4 && sizeof(TW) == 4) {
+    cudaError_t err = cudaSuccess;
+    if (nb_gemm_f32_tiles<TOut>((const float*)X, (const float*)W, bias, residual, (TOut*)out, M, N, K,
+                                act, stream, &err)) {
+      NB_CUDA(err);
+      return 0;
+    }
+  }
   // four consecutive elements are fetched with one load when every row start is aligned
   const bool x_vec = (K % 4 == 0) && ((uintptr_t)X % (4 * sizeof(TIn)) == 0);
   const bool w_vec = (K % 4 == 0) && ((uintptr_t)W % (4 * sizeof(TW)) == 0);

@@ -12,7 +12,7 @@
 // (true 32-bit path).
 //
 // Reference analogue: Mat::gemv_into (src/model.rs:65-86), one dot product per output.
-#include "common.cuh"
+#include "gemm_f32.cuh"
 
 namespace {
 
@@ -520,6 +520,14 @@ template <typename TX, bool LN, typename TOut>
 int launch_f32(const void* X, const float* gamma, const float* beta, float eps, const void* W,
                const float* bias, const float* residual, void* out, int M, int N, int K, int act,
                cudaStream_t stream) {
+  if constexpr (!LN && sizeof(TX) == 4) {
+    cudaError_t err = cudaSuccess;
+    if (nb_gemm_f32_rows<TOut>((const float*)X, (const float*)W, bias, residual, (TOut*)out, M, N, K,
+                               act, stream, &err)) {
+      NB_CUDA(err);
+      return 0;
+    }
+  }
   const size_t smem = (size_t)F32_ROWS * K * sizeof(float);
   NB_REQUIRE(smem <= 220 * 1024, NB_ERR_UNSUPPORTED,
              "gemm_skinny: width %d needs %zu bytes of shared memory", K, smem);

@@ -113,6 +113,30 @@ def test_linear_against_float64(ops, M, N, K, xdt, wdt):
     assert (stream.double() - ref).abs().max() <= tol + 1e-6 * float(ref.abs().max())
 
 
+# the edges of the 32-bit kernels: 8-row passes, 4 and 8 columns a CTA, one to three 16-byte pieces
+# of K a thread (up to 64 rows); 64 x 64 tiles, blocks of 16 of K, K cut among 1, 2, 4 and 8 CTAs
+F32_SHAPES = [(1, 1183, 1024), (8, 1184, 1028), (9, 1185, 4), (16, 7, 3072), (17, 50, 2052), (64, 1201, 2048),
+              (65, 64, 2), (65, 63, 4096), (128, 65, 1026), (129, 1999, 510), (1025, 640, 256), (66, 64, 300)]
+
+
+@pytest.mark.parametrize("M, N, K", F32_SHAPES)
+def test_32_bit_products_at_the_edges_of_their_kernels(ops, M, N, K):
+    torch.manual_seed(M + N + K)
+    x = torch.randn(M, K, device=DEV)
+    w = torch.randn(N, K, device=DEV) / math.sqrt(K)
+    bias = torch.randn(N, device=DEV)
+    res = torch.randn(M, N, device=DEV)
+    ref = x.double() @ w.double().t() + bias.double()
+    # a sum of K fp32 products in any order: each addition rounds by 2^-24 of a partial sum
+    tol = 2.0 ** -24 * math.sqrt(K) * 4 * float(ref.abs().max()) + 1e-6
+    stream = res.clone()
+    ops.linear(x, w, bias, stream, 0, stream)
+    assert (stream.double() - ref - res.double()).abs().max() <= tol + 2.0 ** -22 * float(res.abs().max())
+    out = torch.full((M, N), float("nan"), device=DEV)
+    ops.linear(x, w, bias, out, 1)
+    assert (out.double() - _gelu(ref, 1)).abs().max() <= 2 * tol
+
+
 @pytest.mark.parametrize("M, N, K, out_dtype", [
     (45, 4800, 1600, torch.bfloat16), (192, 4800, 1600, torch.bfloat16), (192, 1600, 6400, torch.float32),
     (64, 768, 768, torch.float32), (130, 20001, 1600, torch.float32), (700, 2304, 776, torch.bfloat16),
