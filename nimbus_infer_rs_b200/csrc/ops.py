@@ -133,6 +133,9 @@ class CudaBackend:
         # CTAs of a cluster: never / where it is the faster one (a long K over few columns) /
         # wherever it applies
         self.use_rows = int(os.environ.get("NIMBUS_B200_ROWS", "1") or 1)
+        # NIMBUS_B200_MID=0/1/2: products of up to 128 rows on the kernel that cuts columns and K
+        # finely: never / where it is the fastest / wherever it applies
+        self.use_mid = int(os.environ.get("NIMBUS_B200_MID", "1") or 1)
         # NIMBUS_B200_DECODE_CLUSTERS=0: the splits of the bfloat16 decode attention merge through
         # scratch memory and a counter instead of a thread-block cluster's shared memory
         self._cluster_limit = int(self.lib.nb_attention_decode_cluster_limit())
@@ -359,6 +362,14 @@ class CudaBackend:
                 raise KernelError("linear: residual shape does not match")
         tensor_core = (x.dtype == torch.bfloat16 or norm is not None and norm[3] == torch.bfloat16) \
             and w.dtype == torch.bfloat16 and K % 8 == 0 and self.use_tcgen05
+        # 17 to 128 rows over few columns, and 9 to 16 rows with a long K: all rows and a few columns
+        # a CTA, K cut among a cluster
+        if norm is None and self.use_tcgen05 and self.use_mid and self.use_rows == 1 and M <= ROWS_MAX_ROWS \
+                and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and (
+                    self.lib.nb_gemm_mid_preferred(M, N, K) if self.use_mid == 1
+                    else self.lib.nb_gemm_mid_supported(M, N, K)):
+            self._gemm_mid(x, w, bias, residual, out, act)
+            return
         # few rows: the weight-streaming kernel; from 17 rows on the tensor-core kernel streams
         # weights faster (TMA ring), where it applies
         skinny = (M <= FUSED_NORM_MAX_ROWS or (M <= SKINNY_MAX_ROWS and not tensor_core)) \
@@ -394,7 +405,8 @@ class CudaBackend:
         if norm is not None:
             h = torch.empty((M, K), device=x.device, dtype=norm[3])
             self.layernorm(x, norm[0], norm[1], norm[2], h)
-            x = h
+            self.linear(h, w, bias, out, act, residual)
+            return
         # up to 128 rows with a long K over few columns (the MLP's second product of a decode
         # step of a larger batch or of a short prompt): weights as the 128-row operand, K cut
         # among the CTAs of a cluster
@@ -416,10 +428,14 @@ class CudaBackend:
                    dtype_code(out.dtype), M, N, K, act,
                    self._stream())
 
+    def _gemm_mid(self, x, w, bias, residual, out, act) -> None:
+        self._call("nb_gemm_mid", _ptr(x), _ptr(w), _ptr(bias), _ptr(residual), _ptr(out),
+                   dtype_code(out.dtype), x.shape[0], w.shape[0], x.shape[1], act, self._stream())
+
     # A kernel whose bounded wait on a barrier ran out says so in a word of pinned host memory
     # (one per kernel family); its results are not valid.
     _ERROR_WORDS = {0: "gemm_tcgen05", 1: "attention_prefill_tc", 2: "wait_probe", 3: "gemm_stream",
-                    4: "gemm_tc_rows", 5: "attention_differential_tc"}
+                    4: "gemm_tc_rows", 5: "attention_differential_tc", 6: "gemm_mid"}
 
     def raise_device_errors(self) -> None:
         """Raise if a kernel that has finished reported a timed-out wait.  Reads host memory
@@ -442,7 +458,8 @@ class CudaBackend:
         cycles = 4_000_000_000 if cycles is None else int(cycles)
         for fn in ("nb_gemm_tcgen05_set_wait_budget", "nb_attention_prefill_tc_set_wait_budget",
                    "nb_gemm_stream_set_wait_budget", "nb_gemm_tc_rows_set_wait_budget",
-                   "nb_moe_gemm_tc_set_wait_budget", "nb_attention_differential_tc_set_wait_budget"):
+                   "nb_moe_gemm_tc_set_wait_budget", "nb_attention_differential_tc_set_wait_budget",
+                   "nb_gemm_mid_set_wait_budget"):
             rc = getattr(self.lib, fn)(cycles)
             if rc != 0:
                 raise KernelError(f"{fn} failed ({rc}): "

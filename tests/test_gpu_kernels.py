@@ -220,6 +220,47 @@ def test_products_of_17_to_128_rows(ops, M, N, K, split):
         ops.use_rows = was_rows
 
 
+MID_SHAPES = [(17, 768, 768), (32, 2304, 768), (33, 70, 72), (64, 1600, 6400), (65, 768, 3072), (128, 333, 200),
+              (48, 2050, 520), (128, 1601, 1600), (16, 768, 3072), (3, 64, 8), (20, 5, 64)]
+
+
+@pytest.mark.parametrize("M, N, K", MID_SHAPES)
+@pytest.mark.parametrize("columns, split", [(0, 0), (16, 1), (32, 3), (64, 8), (16, 5), (64, 2)])
+def test_products_of_up_to_128_rows_in_fine_cuts(ops, M, N, K, columns, split):
+    """The kernel that cuts columns and K finely: the layout it chooses, and forced ones (sums met
+    in one CTA and in clusters whose size divides nothing); the edges of its row tiles, columns
+    that are no multiple of 4, of a tile, fewer than one; K of a part of a block and of a hundred."""
+    was = ops.use_mid
+    ops.use_mid = 2
+    ops.lib.nb_gemm_mid_force(columns, split)
+    try:
+        if not ops.lib.nb_gemm_mid_supported(M, N, K):
+            pytest.skip("this layout leaves a CTA without a block of K")
+        torch.manual_seed(M + N + K)
+        x = torch.randn(M, K, device=DEV).to(torch.bfloat16)
+        w = (torch.randn(N, K, device=DEV) / math.sqrt(K)).to(torch.bfloat16)
+        bias = torch.randn(N, device=DEV)
+        ref0 = x.double() @ w.double().t() + bias.double()
+        tol = 3e-6 * float(ref0.abs().max()) * math.sqrt(max(K, 64) / 64)      # fp32 sums, as above
+        res = torch.randn(M, N, device=DEV)
+        streams = [res.clone() for _ in range(3)]
+        for s in streams:                                  # back to back, overlapping
+            before = ops.launches
+            ops.linear(x, w, bias, s, 0, s)
+            assert ops.launches == before + 1
+        o = torch.full((M, N), 9.0, device=DEV, dtype=torch.bfloat16)
+        ops.linear(x, w, bias, o, 1)
+        ops.check_device_errors()
+        ref = ref0 + res.double()
+        assert (streams[0].double() - ref).abs().max() <= tol + 1e-6 * float(ref.abs().max())
+        assert all(torch.equal(s, streams[0]) for s in streams[1:])
+        ref = _gelu(ref0, 1)
+        assert (o.double() - ref).abs().max() <= tol + 8e-3 * float(ref.abs().max())
+    finally:
+        ops.use_mid = was
+        ops.lib.nb_gemm_mid_force(0, 0)
+
+
 def _paged_cache(n_seqs, lens, Hk, hd, dtype, seed, extra_pages=3, page=PAGE, stale_nan=False):
     """A cache with shuffled pages, filled with random keys/values for the given lengths; what
     lies in the unused part of every page is random too, or (``stale_nan``) not a number."""
