@@ -236,11 +236,11 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         }
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (n + j >= N) break;
-        if (bias != nullptr) y[j] += __ldg(bias + n + j);
-        y[j] = nb_apply_act_fast(y[j], act) + r[j];
-      }
+      for (int j = 0; j < 4; ++j)
+        if (bias != nullptr && n + j < N) y[j] += __ldg(bias + n + j);
+      nb_apply_act_fast_all(y, act);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) y[j] += r[j];
       if (vec) {
         if constexpr (sizeof(TOut) == 4) {
           *reinterpret_cast<float4*>(out + o) = make_float4(y[0], y[1], y[2], y[3]);

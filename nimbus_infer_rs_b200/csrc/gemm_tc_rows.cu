@@ -81,10 +81,12 @@ __device__ __forceinline__ void st_async_v4(uint32_t remote, uint32_t remote_bar
 template <typename TOut>
 __device__ __forceinline__ void finish_rows4(const float (&a)[4], const float (&r)[4], int m0, int m_end,
                                              int n, int N, float b, int act, TOut* out) {
+  float f[4] = {a[0] + b, a[1] + b, a[2] + b, a[3] + b};
+  nb_apply_act_fast_all(f, act);
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     if (m0 + j >= m_end) break;
-    const float y = nb_apply_act_fast(a[j] + b, act) + r[j];
+    const float y = f[j] + r[j];
     if constexpr (sizeof(TOut) == 4) reinterpret_cast<float*>(out)[(size_t)(m0 + j) * N + n] = y;
     else reinterpret_cast<bf16*>(out)[(size_t)(m0 + j) * N + n] = __float2bfloat16_rn(y);
   }

@@ -8,7 +8,8 @@
 // allocation and one of its threads issues `tcgen05.mma` (M=128, N=BN, K=16; four per stage)
 // with shared-memory matrix descriptors; `tcgen05.commit` hands a stage back to the producer
 // and, after the last K block of a tile, signals that tile's accumulator (there are two, used
-// in turn).  The other 8 or 16 warps are the epilogue: each reads its share of the columns of
+// in turn).  The last warp brings the rows of W where the tiles are large (see `split_xw`).
+// The other 4 to 16 warps are the epilogue: each reads its share of the columns of
 // its 32-lane quarter of the accumulator with `tcgen05.ld`, hands the accumulator back, applies bias / GELU / residual in fp32 and
 // stores its rows while the MMAs of the next tile already run.  Edges need no special code on the load side: TMA
 // zero-fills rows beyond M or N and columns beyond K.
@@ -27,8 +28,8 @@ typedef __nv_bfloat16 bf16;
 
 // Tuning (nb_gemm_tcgen05_tune): whether a CTA with one tile and a long K has two MMA-issuing
 // threads, and whether the producer is more than one lane.  What a launch passes to the
-// kernel: bit 0: two issuing threads; bits 1-2: the producer is 0 one lane, 1 a lane for X and
-// a lane for W (large tiles), 2 lanes that share out the ring's stages (a single row tile).
+// kernel: bit 0: two issuing threads; bits 1-2: the producer is 0 one lane, 1 a warp for X and
+// a warp for W (large tiles), 2 lanes that share out the ring's stages (a single row tile).
 bool g_dual = true, g_lanes = true;
 
 constexpr int BM = 128;
@@ -45,7 +46,7 @@ __host__ __device__ constexpr int epi_warps(int bn, int epi) {
 __host__ __device__ constexpr int acc_stride(int bn) {
   return bn <= 64 ? 64 : (bn <= 128 ? 128 : 256);
 }
-__host__ __device__ constexpr int cta_threads(int bn, int epi) { return 64 + 32 * epi_warps(bn, epi); }
+__host__ __device__ constexpr int cta_threads(int bn, int epi) { return 96 + 32 * epi_warps(bn, epi); }
 
 // One CTA per SM walks over tiles; two accumulators in tensor memory let the epilogue of one
 // tile overlap the main loop of the next.  EPI 1 adds a staging area for the epilogue: 4 KB
@@ -220,19 +221,25 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   // stage's barrier would pass for the one it waits for), in whatever order two issuing
   // threads consume the stages.
   const int PRODUCERS = (tune >> 1) == 2 ? L::PRODUCERS : 1;
-  // Large tiles: one lane brings
-  // the rows of X, the other the rows of W, both block after block in order, so the ring
-  // fills in the order the MMAs read it at twice one thread's issue rate.  The lane of X arms
+  // Large tiles: warp 0 brings
+  // the rows of X, the last warp the rows of W, both block after block in order, so the ring
+  // fills in the order the MMAs read it at twice one thread's issue rate.  (As two lanes of one
+  // warp they still took turns: 997 x 768 x 3072 16.6 us, as two warps 14.5; 997 x 1024 x 4096
+  // 20.8 and 17.8.)  The warp of X arms
   // the stage's barrier with the bytes of both boxes; bytes of W that land before that only
   // take the count below zero for a while (the phase cannot end before the arming arrives).
-  const bool split_xw = !PAIR && (tune >> 1) == 1;
-  if (warp == 0 && split_xw) {
-    if (lane < 2) {
+  const bool split_xw = (tune >> 1) == 1;
+  if (warp == 2 + EW && !split_xw) {
+    // nothing to bring in
+  } else if (split_xw && (warp == 0 || warp == 2 + EW)) {
+    const bool rows_of_x = warp == 0;
+    if (lane == 0) {
+      if constexpr (!PAIR) pre_kb = walker < num_tiles ? (num_kb < L::STAGES ? num_kb : L::STAGES) : 0;
       uint32_t it = 0;
       bool ok = true;
       for (int tile = walker; tile < num_tiles && ok; tile += n_walkers) {
         const int m0 = (tile / tiles_n) * TILE_M + m_off;
-        const int n0 = (tile % tiles_n) * BN;
+        const int n0 = (tile % tiles_n) * BN + (PAIR ? (int)rank * (BN / 2) : 0);
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = it % L::STAGES;
           const uint32_t phase = (it / L::STAGES) & 1u;
@@ -240,7 +247,18 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
           if (!early) ok = mbar_wait(empty_bar(s), phase ^ 1u, abort_flag);
           if (!ok) break;
           const uint32_t a_dst = base + s * L::STAGE_BYTES;
-          if (lane == 0) {
+          if constexpr (PAIR) {
+            // both CTAs' bytes are counted on the leader's barrier, which the leader arms
+            const uint32_t lead_bar = cluster_addr(full_bar(s), 0);
+            if (rows_of_x) {
+              if (rank == 0) mbar_expect_tx(full_bar(s), 2u * ((uint32_t)a_box_bytes + L::B_BYTES));
+              tma_load_2d_pair(a_dst, &map_x, kb * BK, m0, lead_bar);
+            } else {
+              tma_load_2d_pair(a_dst + L::A_BYTES, &map_w, kb * BK, n0, lead_bar);
+            }
+            continue;
+          }
+          if (rows_of_x) {
             if (!early) mbar_expect_tx(full_bar(s), (uint32_t)a_box_bytes + L::B_BYTES);
             tma_load_2d(a_dst, &map_x, kb * BK, m0, full_bar(s));
           } else if (!early) {
@@ -255,8 +273,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       uint32_t it_tile = 0;
       bool ok = true;
       for (int tile = walker; tile < num_tiles && ok; tile += n_walkers, it_tile += (uint32_t)num_kb) {
-        const int m0 = (tile / tiles_n) * TILE_M + m_off;
-        const int n0 = (tile % tiles_n) * BN + (PAIR ? (int)rank * (BN / 2) : 0);
+        const int m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN;
         // a lane takes every PRODUCERS-th block of the CTA's whole walk (across its tiles)
         const int kb_first = (int)(((uint32_t)lane + PRODUCERS - it_tile % PRODUCERS) % PRODUCERS);
         for (int kb = kb_first; kb < num_kb; kb += PRODUCERS) {
@@ -266,13 +283,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
           if (!(tile == walker && kb < pre_kb)) ok = mbar_wait(empty_bar(s), phase ^ 1u, abort_flag);
           if (!ok) break;
           const uint32_t a_dst = base + s * L::STAGE_BYTES;
-          if constexpr (PAIR) {
-            // both CTAs' bytes are counted on the leader's barrier, which the leader arms
-            if (rank == 0) mbar_expect_tx(full_bar(s), 2u * ((uint32_t)a_box_bytes + L::B_BYTES));
-            const uint32_t lead_bar = cluster_addr(full_bar(s), 0);
-            tma_load_2d_pair(a_dst, &map_x, kb * BK, m0, lead_bar);
-            tma_load_2d_pair(a_dst + L::A_BYTES, &map_w, kb * BK, n0, lead_bar);
-          } else if (tile == walker && kb < pre_kb) {
+          if (tile == walker && kb < pre_kb) {
             // the stage was armed and its weights asked for before the wait: the rows follow
             tma_load_2d(a_dst, &map_x, kb * BK, m0, full_bar(s));
           } else {
@@ -404,9 +415,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         float f[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
-          const float x = __uint_as_float(v[j]) + __shfl_sync(0xffffffffu, bias_l, j);
-          f[j] = nb_apply_act_fast(x, act);
+          f[j] = __uint_as_float(v[j]) + __shfl_sync(0xffffffffu, bias_l, j);
         }
+        nb_apply_act_fast_all(f, act);
         if constexpr (F32) {
           const uint32_t buf = my_row + c * 4096u;
           if (residual != nullptr) {
@@ -538,6 +549,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         const int col = nb + lane;
         const int row0 = m0 + quarter * 32;
         if (col < N) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) f[i] += bias_l;
+          nb_apply_act_fast_all(f, act);
           float rs[32];   // `residual` may be `out` itself: all of it before the first store
 #pragma unroll
           for (int i = 0; i < 32; ++i)
@@ -545,7 +559,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
             if (row0 + i >= M) break;
-            const float y = nb_apply_act_fast(f[i] + bias_l, act) + rs[i];
+            const float y = f[i] + rs[i];
             if constexpr (sizeof(TOut) == 4) reinterpret_cast<float*>(out)[(size_t)(row0 + i) * N + col] = y;
             else reinterpret_cast<bf16*>(out)[(size_t)(row0 + i) * N + col] = __float2bfloat16_rn(y);
           }
@@ -665,14 +679,14 @@ int launch(const void* X, const void* W, const float* bias, const float* residua
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     NB_CUDA(cudaLaunchKernelEx(&cfg, kern, mx, mw, mo, bias, residual, (TOut*)out, M, N, K, act, tiles_n,
-                               (int)num_tiles, a_rows * BK * 2, error_word(), 0));
+                               (int)num_tiles, a_rows * BK * 2, error_word(), 1 << 1));
     return 0;
   }
   const int grid = (int)(num_tiles < sms ? num_tiles : sms);   // one CTA per SM walks the tiles
   // Several producer lanes only for a single row tile (a decode step, a short prompt): its
   // boxes are small and the producer's issue rate bounds the kernel.  With large tiles the
   // MMAs bound it, and lanes that fill the ring out of order only delay the stage the MMAs
-  // wait for (a 2,048-token prefill: 1.16 -> 1.28 ms with four lanes); there one lane brings X
+  // wait for (a 2,048-token prefill: 1.16 -> 1.28 ms with four lanes); there one warp brings X
   // and one W, both in order (the kernel's `split_xw`).
   const int tune = (g_dual ? 1 : 0) | ((g_lanes ? (M <= BM ? 2 : 1) : 0) << 1);
   NB_CUDA(nb_launch(kern, dim3(grid), dim3(cta_threads(BN, EPI)), (size_t)smem, stream, mx, mw, mo, bias,

@@ -221,8 +221,8 @@ moe_mma_kernel(const TX* x, int x_stride, const int* order, int row_div, const i
         for (int c = 0; c < 2; ++c) {
           v[c] = acc[mi][nt][2 * half + c];
           if (DUAL) v[c] = nb_gate_up<true>(v[c], acc2[mi][nt][2 * half + c], act, act_param);
-          else v[c] = nb_apply_act_fast(v[c], act);
         }
+        if (!DUAL) nb_apply_act_fast_all(v, act);
         if (each != nullptr) {
           if (n < N) v[0] *= nb_sigmoid(each[n]);
           if (n + 1 < N) v[1] *= nb_sigmoid(each[n + 1]);
