@@ -136,6 +136,9 @@ class CudaBackend:
         # NIMBUS_B200_MID=0/1/2: products of up to 128 rows on the kernel that cuts columns and K
         # finely: never / where it is the fastest / wherever it applies
         self.use_mid = int(os.environ.get("NIMBUS_B200_MID", "1") or 1)
+        # NIMBUS_B200_F32_TC=0/1/2: 32-bit products as six products of bf16 pieces on the tensor
+        # cores: never / where that is the faster way / wherever it applies
+        self.use_f32_tc = int(os.environ.get("NIMBUS_B200_F32_TC", "1") or 1)
         # NIMBUS_B200_DECODE_CLUSTERS=0: the splits of the bfloat16 decode attention merge through
         # scratch memory and a counter instead of a thread-block cluster's shared memory
         self._cluster_limit = int(self.lib.nb_attention_decode_cluster_limit())
@@ -423,6 +426,15 @@ class CudaBackend:
                        dtype_code(out.dtype), M, N, K, act,
                        self._stream())
             return
+        # a prompt in 32-bit: three bf16 pieces of every number on the tensor cores
+        if self.use_f32_tc and self.use_tcgen05 and x.dtype == torch.float32 and w.dtype == torch.float32 \
+                and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 \
+                and (self.lib.nb_gemm_f32_tc_preferred(M, N, K) if self.use_f32_tc == 1
+                     else self.lib.nb_gemm_f32_tc_supported(M, N, K)):
+            scratch = torch.empty(self.lib.nb_gemm_f32_tc_scratch(M, N, K), device=x.device, dtype=torch.uint8)
+            self._call("nb_gemm_f32_tc", _ptr(x), _ptr(w), _ptr(bias), _ptr(residual), _ptr(out),
+                       dtype_code(out.dtype), M, N, K, act, _ptr(scratch), self._stream())
+            return
         self._call("nb_gemm_simt", _ptr(x), dtype_code(x.dtype), _ptr(w),
                    dtype_code(w.dtype), _ptr(bias), _ptr(residual), _ptr(out),
                    dtype_code(out.dtype), M, N, K, act,
@@ -435,7 +447,7 @@ class CudaBackend:
     # A kernel whose bounded wait on a barrier ran out says so in a word of pinned host memory
     # (one per kernel family); its results are not valid.
     _ERROR_WORDS = {0: "gemm_tcgen05", 1: "attention_prefill_tc", 2: "wait_probe", 3: "gemm_stream",
-                    4: "gemm_tc_rows", 5: "attention_differential_tc", 6: "gemm_mid"}
+                    4: "gemm_tc_rows", 5: "attention_differential_tc", 6: "gemm_mid", 7: "gemm_f32_tc"}
 
     def raise_device_errors(self) -> None:
         """Raise if a kernel that has finished reported a timed-out wait.  Reads host memory
@@ -459,7 +471,7 @@ class CudaBackend:
         for fn in ("nb_gemm_tcgen05_set_wait_budget", "nb_attention_prefill_tc_set_wait_budget",
                    "nb_gemm_stream_set_wait_budget", "nb_gemm_tc_rows_set_wait_budget",
                    "nb_moe_gemm_tc_set_wait_budget", "nb_attention_differential_tc_set_wait_budget",
-                   "nb_gemm_mid_set_wait_budget"):
+                   "nb_gemm_mid_set_wait_budget", "nb_gemm_f32_tc_set_wait_budget"):
             rc = getattr(self.lib, fn)(cycles)
             if rc != 0:
                 raise KernelError(f"{fn} failed ({rc}): "

@@ -119,6 +119,66 @@ F32_SHAPES = [(1, 1183, 1024), (8, 1184, 1028), (9, 1185, 4), (16, 7, 3072), (17
               (65, 64, 2), (65, 63, 4096), (128, 65, 1026), (129, 1999, 510), (1025, 640, 256), (66, 64, 300)]
 
 
+@pytest.mark.parametrize("M, N, K", [(128, 128, 64), (129, 127, 8), (65, 50, 72), (300, 2304, 768), (257, 130, 136),
+                                     (1000, 333, 1600), (100, 768, 3072)])
+@pytest.mark.parametrize("size", [1.0, 1e-15])
+def test_32_bit_products_in_bf16_pieces(ops, M, N, K, size):
+    """The tensor-core product of 32-bit rows: edges of its tiles, of its blocks of K and of the two
+    blocks between takings-out; never further from 64 bits than the multiply-adds of the CUDA
+    cores are (in their worst form, one sequence: 2^-24 of each partial sum)."""
+    torch.manual_seed(M + N + K)
+    x = torch.randn(M, K, device=DEV) * size
+    w = torch.randn(N, K, device=DEV) / math.sqrt(K)
+    bias = torch.randn(N, device=DEV) * size
+    res = torch.randn(M, N, device=DEV) * size
+    ref = x.double() @ w.double().t()
+    was = ops.use_f32_tc
+    ops.use_f32_tc = 2
+    try:
+        out = torch.full((M, N), float("nan"), device=DEV)
+        ops.linear(x, w, None, out)
+        stream = res.clone()
+        ops.linear(x, w, bias, stream, 0, stream)
+        act = torch.full((M, N), float("nan"), device=DEV, dtype=torch.bfloat16)
+        ops.linear(x, w, bias, act, 1)
+        ops.check_device_errors()
+    finally:
+        ops.use_f32_tc = was
+    tol = 2.0 ** -24 * max(4.0, 0.5 * math.sqrt(K))
+    assert float((out.double() - ref).norm() / ref.norm()) <= tol
+    want = ref + bias.double() + res.double()
+    assert float((stream.double() - want).norm() / want.norm()) <= 2 * tol
+    want = _gelu(ref + bias.double(), 1)
+    assert (act.double() - want).abs().max() <= 8e-3 * float(want.abs().max())
+
+
+def test_32_bit_products_in_bf16_pieces_of_numbers_that_have_none(ops):
+    """Rows with infinities or NaN, and rows of numbers too small for three pieces, are multiplied
+    as they are."""
+    torch.manual_seed(5)
+    x, w = torch.randn(130, 256, device=DEV), torch.randn(140, 256, device=DEV)
+    x[3, 7], x[5, 9], x[10, 0] = math.inf, math.nan, 3.0e38
+    w[11, 3] = -math.inf
+    x[7] *= 1e-36
+    x[9], w[13] = 0.0, 0.0
+    w[12] *= 1e-30
+    outs = []
+    was = ops.use_f32_tc
+    try:
+        for ops.use_f32_tc in (0, 2):
+            outs.append(torch.empty(130, 140, device=DEV))
+            ops.linear(x, w, None, outs[-1])
+    finally:
+        ops.use_f32_tc = was
+    a, b = (o.double() for o in outs)
+    assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+    assert torch.equal(a[a.isinf()], b[b.isinf()])
+    fine = a.isfinite()
+    # 256 fp32 products in two orders: each addition rounds by 2^-24 of a sum of the terms' sizes
+    size = x.double().nan_to_num(0, 0, 0).abs() @ w.double().nan_to_num(0, 0, 0).abs().t()
+    assert ((a - b).abs()[fine] <= 2.0 ** -23 * 16 * size[fine] + 1e-44).all()
+
+
 @pytest.mark.parametrize("M, N, K", F32_SHAPES)
 def test_32_bit_products_at_the_edges_of_their_kernels(ops, M, N, K):
     torch.manual_seed(M + N + K)
