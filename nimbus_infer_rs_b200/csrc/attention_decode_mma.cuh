@@ -133,14 +133,18 @@ attention_decode_mma_kernel(const __nv_bfloat16* q, int q_stride, int q_col,
     bf16* kdst = tiles + (size_t)stage * 2 * STILE;
     bf16* vdst = kdst + STILE;
     constexpr int CPR = HD / 8;   // 16-byte pieces per row
+    // only the rows that hold keys: a sequence's last page is half empty on average (64 sequences of
+    // 9 to 233 tokens bring 20 % less).  What the rest of the staged page holds is masked (keys) or
+    // cleared (values) below.
+    const int rows = min(PAGE_TOKENS, kv_len - page_idx * PAGE_TOKENS);
     if constexpr (MIXED) {
-      for (int i = tid; i < PAGE_TOKENS * CPR; i += NT) {
+      for (int i = tid; i < rows * CPR; i += NT) {
         const int row = i / CPR, c = (i - row * CPR) * 8;
         if (c < dk) cp_async16(kdst + row * ROW + c, ksrc + row * dk + c);
         if (c < dv) cp_async16(vdst + row * ROW + c, vsrc + row * dv + c);
       }
     } else {
-      for (int i = tid; i < PAGE_TOKENS * CPR; i += NT) {
+      for (int i = tid; i < rows * CPR; i += NT) {
         const int row = i / CPR, c = i - row * CPR;
         cp_async16(kdst + row * ROW + c * 8, ksrc + row * HD + c * 8);
         cp_async16(vdst + row * ROW + c * 8, vsrc + row * HD + c * 8);
