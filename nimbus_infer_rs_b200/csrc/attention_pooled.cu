@@ -43,7 +43,8 @@ qk_norm_rope_append_kernel(const float* src, int stride, int q_col, int k_col, i
   const int slot = row_slot[r];
   TQ* qo = q_out + (size_t)r * n_heads * d;
   if (slot < 0) {
-    for (int i = threadIdx.x; i < n_heads * d; i += QK_THREADS) qo[i] = nb_from_f32<TQ>(0.0f);
+    if (blockIdx.y == 0)
+      for (int i = threadIdx.x; i < n_heads * d; i += QK_THREADS) qo[i] = nb_from_f32<TQ>(0.0f);
     return;
   }
   const int pos = row_pos[r];
@@ -77,7 +78,8 @@ qk_norm_rope_append_kernel(const float* src, int stride, int q_col, int k_col, i
     inv_k = 1.0f / sqrtf(nb_block_sum(sk, red) / (float)(n_kv_heads * d) + eps);
   }
   __syncthreads();
-  for (int hh = warp; hh < n_heads + (write ? n_kv_heads : 0); hh += QK_THREADS / 32) {
+  for (int hh = blockIdx.y * (QK_THREADS / 32) + warp; hh < n_heads + (write ? n_kv_heads : 0);
+       hh += gridDim.y * (QK_THREADS / 32)) {
     const bool is_q = hh < n_heads;
     const int g = hh - n_heads;
     const float* x = row + (is_q ? q_col + hh * d : k_col + g * d);
@@ -323,8 +325,13 @@ NB_EXPORT int nb_qkv_norm_rope_append(const float* src, int stride, int q_col, i
              NB_ERR_BAD_ARG, "qkv_norm_rope_append: bad sizes heads=%d/%d d=%d/%d rot=%d", n_heads,
              n_kv_heads, d, dv, rot_dims);
   if (v_table == nullptr) { v_table = block_table; v_max_pages = max_pages; }
+  // few rows (a decode step): a row's heads are dealt out to several CTAs, as many as give each warp
+  // one head while the launch stays within two CTAs an SM (8 rows of 40 heads, one CTA a row:
+  // 11 us)
+  const int per_row = (n_heads + (write ? n_kv_heads : 0) + QK_THREADS / 32 - 1) / (QK_THREADS / 32);
+  const int ny = n_rows >= 2 * 148 ? 1 : (per_row < 2 * 148 / n_rows ? per_row : 2 * 148 / n_rows);
 #define NB_QK(TQ, TC)                                                                             \
-  NB_CUDA(nb_launch(qk_norm_rope_append_kernel<TQ, TC>, dim3(n_rows), dim3(QK_THREADS), 0, stream, \
+  NB_CUDA(nb_launch(qk_norm_rope_append_kernel<TQ, TC>, dim3(n_rows, ny), dim3(QK_THREADS), 0, stream, \
                     src, stride, q_col, k_col, v_col, q_gamma, k_gamma, eps, freq, rot_dims,      \
                     amplitude, row_slot, row_pos, (TQ*)q_out, (TC*)kc, (TC*)vc, block_table,      \
                     max_pages, v_table, v_max_pages, page, n_heads, n_kv_heads, d, dv, write, whole))

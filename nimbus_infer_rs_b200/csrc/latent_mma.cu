@@ -253,20 +253,44 @@ __global__ void latent_merge_kernel(const float* part_o, const float* part_ml, c
     for (int d = threadIdx.x; d < R; d += blockDim.x) dst[d] = __float2bfloat16_rn(0.0f);
     return;
   }
+  // Every warp has the runs' weights in its lanes (32 at a time) and asks for eight runs' sums side
+  // by side: with a thread walking over the runs and their maxima alone, each of up to 32 steps was
+  // a trip to L2 (14.7 us a step of eight sequences and 32 runs).
+  const int lane = threadIdx.x & 31;
   const float* ml = part_ml + pair * n_splits * 2;
-  float m = sink != nullptr ? sink[h] * LOG2E : -INFINITY;
-  for (int i = 0; i < n_splits; ++i)
-    if (ml[2 * i + 1] > 0.0f) m = fmaxf(m, ml[2 * i]);
-  float l = sink != nullptr ? exp2_fast(sink[h] * LOG2E - m) : 0.0f;
-  for (int i = 0; i < n_splits; ++i)
-    if (ml[2 * i + 1] > 0.0f) l += ml[2 * i + 1] * exp2_fast(ml[2 * i] - m);
+  const float s2 = sink != nullptr ? sink[h] * LOG2E : -INFINITY;
+  float m_i[2], l_i[2], m = s2;            // at most 64 runs (see the launcher)
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int i = q * 32 + lane;
+    m_i[q] = i < n_splits ? ml[2 * i] : 0.0f;
+    l_i[q] = i < n_splits ? ml[2 * i + 1] : 0.0f;
+    if (l_i[q] > 0.0f) m = fmaxf(m, m_i[q]);
+  }
+  m = nb_warp_max(m);
+  float w[2], l = 0.0f;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    w[q] = l_i[q] > 0.0f ? exp2_fast(m_i[q] - m) : 0.0f;
+    l = fmaf(w[q], l_i[q] > 0.0f ? l_i[q] : 0.0f, l);
+  }
+  l = nb_warp_sum(l) + (sink != nullptr ? exp2_fast(s2 - m) : 0.0f);
   const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-  for (int d = threadIdx.x; d < R; d += blockDim.x) {
+  for (int d0 = threadIdx.x - lane; d0 < R; d0 += blockDim.x) {
+    const int d = d0 + lane;
     float acc = 0.0f;
-    for (int i = 0; i < n_splits; ++i)
-      if (ml[2 * i + 1] > 0.0f)
-        acc = fmaf(part_o[(pair * n_splits + i) * R + d], exp2_fast(ml[2 * i] - m), acc);
-    dst[d] = __float2bfloat16_rn(acc * inv);
+    for (int i0 = 0; i0 < n_splits; i0 += 8) {
+      float v[8], f[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        f[j] = __shfl_sync(0xffffffffu, i0 < 32 ? w[0] : w[1], (i0 + j) & 31);
+        // (an empty run has left nothing in its place)
+        v[j] = f[j] > 0.0f && d < R ? part_o[(pair * n_splits + i0 + j) * R + d] : 0.0f;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc = fmaf(v[j], f[j], acc);
+    }
+    if (d < R) dst[d] = __float2bfloat16_rn(acc * inv);
   }
 }
 
@@ -340,7 +364,7 @@ NB_EXPORT int nb_attention_latent_mma(const void* q, const int* cu_rows, const i
   if (rc) return rc;
   NB_CHECK_LAUNCH("attention_latent_mma");
   if (n_splits > 1) {
-    NB_CUDA(nb_launch(latent_merge_kernel, dim3((unsigned)((size_t)n_rows * n_heads)), dim3(64), 0, stream,
+    NB_CUDA(nb_launch(latent_merge_kernel, dim3((unsigned)((size_t)n_rows * n_heads)), dim3(128), 0, stream,
                       (const float*)part_o, (const float*)part_ml, row_slot, sink, (bf16*)out, n_heads,
                       value_dim, n_splits));
     NB_CHECK_LAUNCH("latent_merge");
