@@ -51,7 +51,10 @@ __host__ __device__ constexpr int cta_threads(int bn, int epi) { return 96 + 32 
 // One CTA per SM walks over tiles; two accumulators in tensor memory let the epilogue of one
 // tile overlap the main loop of the next.  EPI 1 adds a staging area for the epilogue: 4 KB
 // (32 rows x 128 bytes, 128-byte swizzled) per epilogue warp for bf16 output, twice that for
-// fp32 output (two 32-column boxes per warp, which also receive the residual by TMA).
+// fp32 output up to 128 columns (two 32-column boxes per warp, which also receive the residual by
+// TMA).  Wider fp32 tiles have one box a warp, through which its two chunks of columns go one after the
+// other: what that adds to the epilogue (a store to be read, a second residual to be brought) runs beside
+// the next tile's products, and the 64 KB it saves are two stages of the ring.
 // PAIR 1: two CTAs of a cluster share 256 x BN tiles (`cta_group::2`): each brings its 128
 // rows of X and half of the tile's rows of W, so a stage holds BN / 2 rows of W.
 template <int BN, int EPI, int ESIZE, int PAIR>
@@ -60,7 +63,9 @@ struct SmemLayout {
   static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int EPI_WARPS = epi_warps(BN, EPI);
-  static constexpr int STG_PER_WARP = EPI ? (ESIZE == 4 ? 8192 : 4096) : 0;
+  // fp32 tiles wider than 128 columns: one 32-column box a warp, used twice a tile
+  static constexpr int BOXES = ESIZE == 4 && BN <= 128 ? 2 : 1;
+  static constexpr int STG_PER_WARP = EPI ? BOXES * 4096 : 0;
   static constexpr int STG_BYTES = EPI_WARPS * STG_PER_WARP;
   static constexpr int BUDGET = 222 * 1024;   // of the 227 KB a CTA may have
   static constexpr int STAGES_RAW = (BUDGET - STG_BYTES) / STAGE_BYTES;
@@ -165,13 +170,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   // (constants): a product of a decode step is a few microseconds long, and the trip to HBM
   // for its first weights would be a good part of that.
   int pre_kb = 0;   // K blocks whose weights are already on their way (the producer's)
-  if constexpr (!PAIR) {
-    if (tid == 0 && walker < num_tiles) {
-      pre_kb = num_kb < L::STAGES ? num_kb : L::STAGES;
-      const int n0 = (walker % tiles_n) * BN;
-      for (int kb = 0; kb < pre_kb; ++kb) {
+  if (tid == 0 && walker < num_tiles) {
+    pre_kb = num_kb < L::STAGES ? num_kb : L::STAGES;
+    const int n0 = (walker % tiles_n) * BN + (PAIR ? (int)rank * (BN / 2) : 0);
+    for (int kb = 0; kb < pre_kb; ++kb) {
+      const uint32_t w_dst = base + kb * L::STAGE_BYTES + L::A_BYTES;
+      if constexpr (PAIR) {
+        if (rank == 0) mbar_expect_tx(full_bar(kb), 2u * ((uint32_t)a_box_bytes + L::B_BYTES));
+        tma_load_2d_pair(w_dst, &map_w, kb * BK, n0, cluster_addr(full_bar(kb), 0));
+      } else {
         mbar_expect_tx(full_bar(kb), (uint32_t)a_box_bytes + L::B_BYTES);
-        tma_load_2d(base + kb * L::STAGE_BYTES + L::A_BYTES, &map_w, kb * BK, n0, full_bar(kb));
+        tma_load_2d(w_dst, &map_w, kb * BK, n0, full_bar(kb));
       }
     }
   }
@@ -234,7 +243,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   } else if (split_xw && (warp == 0 || warp == 2 + EW)) {
     const bool rows_of_x = warp == 0;
     if (lane == 0) {
-      if constexpr (!PAIR) pre_kb = walker < num_tiles ? (num_kb < L::STAGES ? num_kb : L::STAGES) : 0;
+      pre_kb = walker < num_tiles ? (num_kb < L::STAGES ? num_kb : L::STAGES) : 0;
       uint32_t it = 0;
       bool ok = true;
       for (int tile = walker; tile < num_tiles && ok; tile += n_walkers) {
@@ -251,9 +260,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             // both CTAs' bytes are counted on the leader's barrier, which the leader arms
             const uint32_t lead_bar = cluster_addr(full_bar(s), 0);
             if (rows_of_x) {
-              if (rank == 0) mbar_expect_tx(full_bar(s), 2u * ((uint32_t)a_box_bytes + L::B_BYTES));
+              if (rank == 0 && !early) mbar_expect_tx(full_bar(s), 2u * ((uint32_t)a_box_bytes + L::B_BYTES));
               tma_load_2d_pair(a_dst, &map_x, kb * BK, m0, lead_bar);
-            } else {
+            } else if (!early) {
               tma_load_2d_pair(a_dst + L::A_BYTES, &map_w, kb * BK, n0, lead_bar);
             }
             continue;
@@ -365,7 +374,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       if (lane == 0) {
         bulk_wait_read_all();   // the stores of the previous tile have read this warp's buffers
         if (F32 && residual != nullptr) {
-          for (int u = 0; u < nch; ++u) {
+          for (int u = 0; u < nch && u < L::BOXES; ++u) {
             mbar_expect_tx(res_bar(e, u), 4096u);
             tma_load_2d(stg + u * 4096u, &map_out, col0 + u * 32, row0, res_bar(e, u));
           }
@@ -419,7 +428,18 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         }
         nb_apply_act_fast_all(f, act);
         if constexpr (F32) {
-          const uint32_t buf = my_row + c * 4096u;
+          const uint32_t box = L::BOXES == 2 ? c * 4096u : 0u;
+          const uint32_t buf = my_row + box;
+          if (L::BOXES == 1 && c > 0) {      // the box is free once the first chunk's store has read it
+            if (lane == 0) {
+              bulk_wait_read_all();
+              if (residual != nullptr) {
+                mbar_expect_tx(res_bar(e, c), 4096u);
+                tma_load_2d(stg, &map_out, nb, row0, res_bar(e, c));
+              }
+            }
+            __syncwarp();
+          }
           if (residual != nullptr) {
             const bool got = __shfl_sync(0xffffffffu,
                                          (int)mbar_wait(res_bar(e, c), t & 1u, abort_flag), 0) != 0;
@@ -442,7 +462,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
           fence_async_smem();
           __syncwarp();
           if (lane == 0 && nb < N && row0 < M) {
-            tma_store_2d(&map_out, stg + c * 4096u, nb, row0);
+            tma_store_2d(&map_out, stg + box, nb, row0);
             bulk_commit();
           }
         } else {
@@ -666,20 +686,9 @@ int launch(const void* X, const void* W, const float* bias, const float* residua
   if constexpr (PAIR) {
     // clusters of two CTAs, one cluster per pair of SMs
     const int pairs = (int)(num_tiles < sms / 2 ? num_tiles : sms / 2);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * pairs);
-    cfg.blockDim = dim3(cta_threads(BN, EPI));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    NB_CUDA(cudaLaunchKernelEx(&cfg, kern, mx, mw, mo, bias, residual, (TOut*)out, M, N, K, act, tiles_n,
-                               (int)num_tiles, a_rows * BK * 2, error_word(), 1 << 1));
+    NB_CUDA(nb_launch_clusters(kern, dim3(2 * pairs), dim3(cta_threads(BN, EPI)), (size_t)smem, stream, 2, mx, mw,
+                               mo, bias, residual, (TOut*)out, M, N, K, act, tiles_n, (int)num_tiles,
+                               a_rows * BK * 2, error_word(), 1 << 1));
     return 0;
   }
   const int grid = (int)(num_tiles < sms ? num_tiles : sms);   // one CTA per SM walks the tiles
@@ -737,6 +746,7 @@ int pick_tile_width(int M, int N, bool f32_out, bool tma_epi) {
 // product of a wave or two of tiles is no faster in pairs, or slower (12.3 -> 13.4 us at
 // 2048 x 2304 x 768): the cluster's start-up and its barriers cost more than the lighter
 // loads save; pairs are taken from three waves of single-CTA tiles on.
+int g_force_bn = 0, g_force_pair = 0;
 int g_use_pairs = 1;   // 0 off, 1 where the cost model prefers them, 2 wherever a paired kernel exists
 
 // Width of 256-row tiles for pairs of CTAs, or 0 if single CTAs with `single_bn` are better.
@@ -785,6 +795,13 @@ NB_EXPORT int nb_gemm_tcgen05_supported(int x_dtype, int w_dtype, int M, int N, 
 NB_EXPORT int nb_gemm_tcgen05_tune(int dual, int lanes) {
   g_dual = dual != 0;
   g_lanes = lanes != 0;
+  return 0;
+}
+
+// Tuning and tests: a tile width and whether pairs of CTAs take it (0: choose).
+NB_EXPORT int nb_gemm_tcgen05_force(int width, int pair) {
+  g_force_bn = width;
+  g_force_pair = pair;
   return 0;
 }
 
@@ -838,15 +855,18 @@ NB_EXPORT int nb_gemm_tcgen05(const void* X, const void* W, const float* bias, c
   // itself; otherwise every thread stores its own row segment.
   const int esize = out_dtype == NB_F32 ? 4 : 2;
   const bool tma_epi = ((long long)N * esize) % 16 == 0 && (residual == nullptr || residual == out);
-  const int bn = pick_tile_width(M, N, out_dtype == NB_F32, tma_epi);
+  const bool force = g_force_bn && tma_epi && M > BM;
+  const int bn = force && !g_force_pair ? g_force_bn : pick_tile_width(M, N, out_dtype == NB_F32, tma_epi);
   int rc;
   // Pairs of CTAs on 256-row tiles bring less into each SM per flop (half of the weight tile
   // each); they are taken when that outweighs the coarser tiles (see pick_pair_width).
-  const int pair_bn = (tma_epi && g_use_pairs) ? pick_pair_width(M, N, out_dtype == NB_F32, bn) : 0;
+  const int pair_bn = force ? (g_force_pair ? g_force_bn : 0) : (tma_epi && g_use_pairs) ? pick_pair_width(M, N, out_dtype == NB_F32, bn) : 0;
   if (pair_bn) {
     rc = NB_ERR_BAD_ARG;
     if (out_dtype == NB_F32) {
-      if (pair_bn == 128) rc = launch<128, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, stream);
+      if (pair_bn == 256) rc = launch<256, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, stream);
+      else if (pair_bn == 192) rc = launch<192, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, stream);
+      else if (pair_bn == 128) rc = launch<128, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, stream);
       else if (pair_bn == 96) rc = launch<96, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, stream);
     } else if (out_dtype == NB_BF16) {
       if (pair_bn == 256) rc = launch<256, 1, bf16, 1>(X, W, bias, residual, out, M, N, K, act, stream);
