@@ -4,14 +4,21 @@
 // prompts; heads of 64 or 128, pages of 64 tokens.
 //
 // A CTA takes 64 consecutive query rows of one sequence and one head and walks over the
-// sequence's pages up to the last key its rows may see.  Per page: the page's keys (transposed)
-// and values go to shared memory; the 16 x 16 threads each compute a 4 x 4 block of the 64 x 64
-// scores from the transposed query and key tiles (two 16-byte reads feed 16 multiply-adds);
-// scale, causal limit and window; running maximum and sum per row (fp32, maximum subtracted,
-// src/ops.rs:6-18) through shuffles among the 16 threads that share a row; probabilities to
-// shared memory; then every thread adds its 4 rows x head/16 columns of P V.  Keys after a
-// row's own position, before its window or beyond the sequence get no weight, and the rows of
-// the last page that hold no key yet are never multiplied with anything.
+// sequence's pages up to the last key its rows may see.  What bounds it is the multiply-adds (2 x 1,024
+// tokens x 12 heads of 64: 45 us at 128 a clock and SM), so everything is laid out to keep shared memory
+// out of their way: a thread has 8 rows x 8 keys of the scores and 8 rows x 8 columns of the result (with
+// heads of 128 twice the threads and 4 keys each), so four 16-byte reads feed 64 packed
+// multiply-adds; queries, keys and probabilities lie transposed, their 16-byte pieces exchanged by a
+// few bits of the row so that neither the transposing stores nor the reads meet in a bank.  The next
+// page's keys are asked for while P V runs and go from registers to shared memory after it, its values
+// by cp.async beside the next scores.  Scale, causal limit and window; running maximum per row (fp32,
+// maximum subtracted, src/ops.rs:6-18) through shuffles among the threads that share a row, the sums per
+// thread until the end.  Keys after a row's own position, before its window or beyond the
+// sequence get no weight, and the rows of the last page that hold no key yet are never read.
+//
+// Tiles see as many pages as lie before them, from 1 to all.  CTAs are dealt out longest first, every
+// other turn over the SMs backwards, so that an SM's CTAs add up to about the same (2 x 1,024 tokens x
+// 12 heads: 22 pages an SM on average, 24 at most; in order of the tiles 36).
 //
 // Reference: src/model.rs:401-422 (scores = dot(q,k)*scale for keys 0..P+i, softmax, weighted
 // values); head h reads key/value head h / group (src/model.rs:390).
@@ -21,158 +28,253 @@ namespace {
 
 constexpr int TQ = 64;            // query rows per CTA
 constexpr int PAGE_TOKENS = 64;   // keys per page
-constexpr int LD = 68;            // floats between rows of a 64-wide shared tile (16-byte aligned)
-constexpr int THREADS = 256;
+constexpr int LD = 64;            // floats between rows of a transposed tile
 
-template <typename T>
-__device__ __forceinline__ float to_f32(T v);
-template <>
-__device__ __forceinline__ float to_f32<float>(float v) { return v; }
-template <>
-__device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpair(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma2(f32x2& c, f32x2 a, f32x2 b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ void mul2(f32x2& c, f32x2 a) {
+  asm("mul.rn.f32x2 %0, %0, %1;\n" : "+l"(c) : "l"(a));
+}
+
+// Four consecutive numbers, widened; one load where the caller has seen that they are aligned.
+__device__ __forceinline__ float4 load4(const float* p, bool vec) {
+  return vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+__device__ __forceinline__ float4 load4(const __nv_bfloat16* p, bool vec) {
+  if (!vec)
+    return make_float4(__bfloat162float(p[0]), __bfloat162float(p[1]), __bfloat162float(p[2]),
+                       __bfloat162float(p[3]));
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// Where piece `c` (four columns) of row `d` of a transposed query or key tile lies: eight rows of the
+// source times four pieces of it, which a warp turns over at once, then lie in 32 banks.
+__device__ __forceinline__ int piece_of(int d, int c) { return d * LD + ((c ^ (((d >> 2) & 3) << 1)) << 2); }
+// The same for row `j` (a key) of the probabilities: a thread writes the keys 4 x, 4 x + 1, ...
+__device__ __forceinline__ int prob_of(int j, int c) { return j * LD + ((c ^ ((j >> 2) & 7)) << 2); }
+
+enum : int { VEC_Q = 1, VEC_KV = 2, VEC_OUT = 4 };   // operands whose rows may be taken 4 numbers at a time
 
 template <typename T, int HD, typename TOut>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(HD, HD == 64 ? 3 : 1)
 attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
                              const int* cu_rows, const int* seq_slot,
                              const int* seq_pos0, NbPagedKV kv, int group,
-                             TOut* out, int out_stride, float scale, int window) {
-  constexpr int CPT = HD / 16;          // output columns per thread
-  constexpr int VLD = HD + 4;           // floats between rows of the value tile
+                             TOut* out, int out_stride, float scale, int window, int vec, int sms) {
+  constexpr int THREADS = HD;           // a thread has 8 rows and 8 columns of the result
+  constexpr int TX = HD / 8;            // threads that share a row
+  constexpr int KPT = PAGE_TOKENS / TX; // keys a thread: 8 or 4
+  constexpr int KP = KPT / 2, NL = 16;  // pairs of them; pieces of four numbers of a page's keys a thread
   extern __shared__ __align__(16) float sm[];
-  float* Qt = sm;                       // [HD][LD]: Qt[d][i] = q of row i, column d
-  float* Kt = Qt + HD * LD;             // [HD][LD]: Kt[d][j] = key j of the page, column d
-  float* Vs = Kt + HD * LD;             // [64][VLD]
-  float* Ps = Vs + PAGE_TOKENS * VLD;   // [64][LD]: probabilities of the page, row i, key j
+  float* Qt = sm;                       // [HD][LD]: column d of row i
+  float* Kt = Qt + HD * LD;             // [HD][LD]: column d of key j
+  float* Pt = Kt + HD * LD;             // [64][LD]: probability of key j in row i
+  float* Vs = Pt + PAGE_TOKENS * LD;    // [64][HD]
 
   nb_grid_dependency_wait();
   nb_launch_dependents();
-  const int tile = blockIdx.x, h = blockIdx.y, s = blockIdx.z;
+  // this CTA's place in the order of work (see the head of the file)
+  const unsigned long long b = blockIdx.x + (unsigned long long)gridDim.x * (blockIdx.y + (unsigned long long)gridDim.y * blockIdx.z);
+  const unsigned long long total = (unsigned long long)gridDim.x * gridDim.y * gridDim.z;
+  const unsigned long long first = b - b % sms;
+  const unsigned long long turn = total - first < (unsigned long long)sms ? total - first : (unsigned long long)sms;
+  const unsigned long long rank = (b / sms) & 1 ? first + (turn - 1 - (b - first)) : b;
+  const unsigned hs = gridDim.y * gridDim.z, rest = (unsigned)(rank % hs);
+  const int tile = (int)(gridDim.x - 1 - (unsigned)(rank / hs)), h = (int)(rest % gridDim.y), s = (int)(rest / gridDim.y);
   const int row0 = cu_rows[s], n_q = cu_rows[s + 1] - row0;
   const int q0 = tile * TQ;
   const int slot = seq_slot[s];
   if (q0 >= n_q || slot < 0) return;
   const int pos0 = seq_pos0[s];
   const int kvh = h / group;
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  const int tid = threadIdx.x, ty = tid / TX, tx = tid % TX;
   const int rows_here = min(TQ, n_q - q0);
   const int last_pos = pos0 + q0 + rows_here - 1;                    // newest key any row sees
   const int first_key = (window > 0) ? max(0, pos0 + q0 + 1 - window) : 0;
   const int p_begin = first_key / PAGE_TOKENS, p_end = last_pos / PAGE_TOKENS + 1;
   const int* table = kv.block_table + (size_t)slot * kv.max_pages;
 
-  // the query tile, transposed; rows beyond the sequence are zero
-  for (int idx = tid; idx < TQ * HD; idx += THREADS) {
-    const int i = idx / HD, d = idx - i * HD;
-    Qt[d * LD + i] = i < rows_here
-                         ? to_f32<T>(q[(size_t)(row0 + q0 + i) * q_stride + q_col + (size_t)h * HD + d])
-                         : 0.0f;
-  }
+  // Which pieces this thread turns over: a warp takes 8 source rows x 4 pieces at a time, so a row's 64
+  // consecutive bytes come with one instruction.  Piece n of NL: row turn_j + 8 * (..), piece turn_d + ..
+  const int wj = (tid & 31) >> 2, wd = tid & 3, w = tid >> 5;
+  auto turn_row = [&](int n) { return wj + 8 * (n & 7); };
+  auto turn_piece = [&](int n) { return wd + 4 * (w + (n >> 3) * (THREADS / 32)); };
+  auto put = [&](float* t, int n, const float4& v) {
+    const int j = turn_row(n), d = turn_piece(n) * 4;
+    float* at = t + piece_of(d, j >> 2) + (j & 3);      // the four rows d .. d + 3 share their exchange
+    at[0] = v.x; at[LD] = v.y; at[2 * LD] = v.z; at[3 * LD] = v.w;
+  };
+  const float4 zero4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float4 kn[NL];                        // a page's keys on their way
+  auto ask_keys = [&](int p) {
+    const T* src = (const T*)kv.k + ((size_t)table[p] * kv.n_kv_heads + kvh) * PAGE_TOKENS * HD;
+    const int keys_here = last_pos + 1 - p * PAGE_TOKENS;      // what lies beyond is an earlier owner's
+#pragma unroll
+    for (int n = 0; n < NL; ++n)
+      kn[n] = turn_row(n) < keys_here ? load4(src + turn_row(n) * HD + turn_piece(n) * 4, vec & VEC_KV) : zero4;
+  };
+  auto bring_values = [&](int p) {
+    const T* src = (const T*)kv.v + ((size_t)table[p] * kv.n_kv_heads + kvh) * PAGE_TOKENS * HD;
+    const int keys_here = last_pos + 1 - p * PAGE_TOKENS;
+#pragma unroll 4
+    for (int idx = tid; idx < PAGE_TOKENS * HD / 4; idx += THREADS) {
+      float* dst = Vs + idx * 4;
+      if (idx / (HD / 4) >= keys_here) *reinterpret_cast<float4*>(dst) = zero4;
+      else if (sizeof(T) == 4 && (vec & VEC_KV)) cp_async16(dst, src + idx * 4);
+      else *reinterpret_cast<float4*>(dst) = load4(src + idx * 4, vec & VEC_KV);
+    }
+    cp_async_commit();
+  };
 
-  float o[4][CPT];
+  ask_keys(p_begin);
+  // the query tile; rows beyond the sequence are zero
+#pragma unroll 4
+  for (int n = 0; n < NL; ++n) {
+    const int i = turn_row(n);
+    put(Qt, n, i < rows_here ? load4(q + (size_t)(row0 + q0 + i) * q_stride + q_col + (size_t)h * HD + turn_piece(n) * 4, vec & VEC_Q)
+                             : zero4);
+  }
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int n = 0; n < NL; ++n) put(Kt, n, kn[n]);
+  __syncthreads();
+  bring_values(p_begin);
+
+  f32x2 o[8][4];            // rows ty * 8 + i; columns tx * 4 + (0, 1), (2, 3) and HD / 2 further
 #pragma unroll
-    for (int c = 0; c < CPT; ++c) o[i][c] = 0.0f;
-  float m_run[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, l_run[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) o[i][c] = 0ull;
+  float m_run[8], l_run[8];  // the sum of this thread's keys only
+#pragma unroll
+  for (int i = 0; i < 8; ++i) { m_run[i] = -INFINITY; l_run[i] = 0.0f; }
 
   for (int p = p_begin; p < p_end; ++p) {
-    __syncthreads();   // the tiles of the page before are no longer read (and Qt is complete)
-    const int page_id = table[p];
-    const T* ksrc = (const T*)kv.k + ((size_t)page_id * kv.n_kv_heads + kvh) * PAGE_TOKENS * HD;
-    const T* vsrc = (const T*)kv.v + ((size_t)page_id * kv.n_kv_heads + kvh) * PAGE_TOKENS * HD;
-    const int keys_here = min(PAGE_TOKENS, last_pos + 1 - p * PAGE_TOKENS);   // rows that hold a key
-    for (int idx = tid; idx < PAGE_TOKENS * HD; idx += THREADS) {
-      const int j = idx / HD, d = idx - j * HD;
-      const bool live = j < keys_here;          // what lies beyond is an earlier owner's: never read
-      Kt[d * LD + j] = live ? to_f32<T>(ksrc[idx]) : 0.0f;
-      Vs[j * VLD + d] = live ? to_f32<T>(vsrc[idx]) : 0.0f;
-    }
-    __syncthreads();
-
-    // scores: rows ty*4 + ii, keys tx*4 + jj
-    float sc[4][4];
+    // scores: rows ty * 8 + i, keys tx * 4 + (0 .. 3) and, with 8 a thread, 32 further
+    f32x2 sc[8][KP];
 #pragma unroll
-    for (int ii = 0; ii < 4; ++ii)
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj) sc[ii][jj] = 0.0f;
-#pragma unroll 8
+      for (int c = 0; c < KP; ++c) sc[i][c] = 0ull;
+#pragma unroll 4
     for (int d = 0; d < HD; ++d) {
-      const float4 a = *reinterpret_cast<const float4*>(Qt + d * LD + ty * 4);
-      const float4 b = *reinterpret_cast<const float4*>(Kt + d * LD + tx * 4);
-      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+      const float4 a0 = *reinterpret_cast<const float4*>(Qt + piece_of(d, ty * 2));
+      const float4 a1 = *reinterpret_cast<const float4*>(Qt + piece_of(d, ty * 2 + 1));
+      f32x2 kk[KP];
 #pragma unroll
-      for (int ii = 0; ii < 4; ++ii)
+      for (int c = 0; c < KP / 2; ++c) {
+        const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(Kt + piece_of(d, tx + 8 * c));
+        kk[2 * c] = t.x; kk[2 * c + 1] = t.y;
+      }
+      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) sc[ii][jj] = fmaf(av[ii], bv[jj], sc[ii][jj]);
+      for (int i = 0; i < 8; ++i) {
+        const f32x2 a2 = pair_of(av[i], av[i]);
+#pragma unroll
+        for (int c = 0; c < KP; ++c) fma2(sc[i][c], a2, kk[c]);
+      }
     }
-    // scale, causal limit, window; the row's maximum and sum among the 16 threads of the row
+    // scale, causal limit, window; the row's maximum among the threads of the row
+    const bool all = (p + 1) * PAGE_TOKENS <= pos0 + q0 + 1 && window <= 0;   // every row sees every key
+    float pr[8][KPT];
 #pragma unroll
-    for (int ii = 0; ii < 4; ++ii) {
-      const int qp = pos0 + q0 + ty * 4 + ii;          // absolute position of the row's query
+    for (int i = 0; i < 8; ++i) {
+      const int qp = pos0 + q0 + ty * 8 + i;           // absolute position of the row's query
       float mx = -INFINITY;
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj) {
-        const int key = p * PAGE_TOKENS + tx * 4 + jj;
-        const bool ok = key <= qp && (window <= 0 || key > qp - window);
-        sc[ii][jj] = ok ? sc[ii][jj] * scale : -INFINITY;
-        mx = fmaxf(mx, sc[ii][jj]);
+      for (int c = 0; c < KPT; ++c) {
+        const int key = p * PAGE_TOKENS + tx * 4 + (c & 3) + (c >> 2) * 32;
+        const float2 v = unpair(sc[i][c >> 1]);
+        const bool ok = all || (key <= qp && (window <= 0 || key > qp - window));
+        pr[i][c] = ok ? ((c & 1) ? v.y : v.x) * scale : -INFINITY;
+        mx = fmaxf(mx, pr[i][c]);
       }
 #pragma unroll
-      for (int off = 8; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-      const float m_new = fmaxf(m_run[ii], mx);
+      for (int off = TX / 2; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+      const float m_new = fmaxf(m_run[i], mx);
       const float m_use = (m_new == -INFINITY) ? 0.0f : m_new;
-      const float resc = (m_run[ii] == -INFINITY) ? 0.0f : expf(m_run[ii] - m_use);
-      m_run[ii] = m_new;
+      const float resc = (m_run[i] == -INFINITY) ? 0.0f : expf(m_run[i] - m_use);
+      m_run[i] = m_new;
       float sum = 0.0f;
-      float pr[4];
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj) {
-        pr[jj] = (sc[ii][jj] == -INFINITY) ? 0.0f : expf(sc[ii][jj] - m_use);
-        sum += pr[jj];
+      for (int c = 0; c < KPT; ++c) {
+        pr[i][c] = (pr[i][c] == -INFINITY) ? 0.0f : expf(pr[i][c] - m_use);
+        sum += pr[i][c];
       }
+      l_run[i] = l_run[i] * resc + sum;
+      const f32x2 r2 = pair_of(resc, resc);
 #pragma unroll
-      for (int off = 8; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-      l_run[ii] = l_run[ii] * resc + sum;
-#pragma unroll
-      for (int c = 0; c < CPT; ++c) o[ii][c] *= resc;
-      *reinterpret_cast<float4*>(Ps + (ty * 4 + ii) * LD + tx * 4) = make_float4(pr[0], pr[1], pr[2], pr[3]);
+      for (int c = 0; c < 4; ++c) mul2(o[i][c], r2);
     }
-    __syncthreads();
+    // a warp reads only what its own threads wrote (its rows)
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < KPT; ++c) {
+      const int j = tx * 4 + (c & 3) + (c >> 2) * 32;
+      *reinterpret_cast<float4*>(Pt + prob_of(j, ty * 2)) = make_float4(pr[0][c], pr[1][c], pr[2][c], pr[3][c]);
+      *reinterpret_cast<float4*>(Pt + prob_of(j, ty * 2 + 1)) = make_float4(pr[4][c], pr[5][c], pr[6][c], pr[7][c]);
+    }
+    cp_async_wait<0>();
+    __syncthreads();       // the values are there; nobody reads the keys any more
+    const bool more = p + 1 < p_end;
+    if (more) ask_keys(p + 1);
 
-    // o[ii][c] += sum_j P[row][j] V[j][tx*CPT + c]
-#pragma unroll 2
-    for (int j = 0; j < PAGE_TOKENS; j += 4) {
-      float pv[4][4];
+    // o += P V
+#pragma unroll 4
+    for (int j = 0; j < PAGE_TOKENS; ++j) {
+      const float4 a0 = *reinterpret_cast<const float4*>(Pt + prob_of(j, ty * 2));
+      const float4 a1 = *reinterpret_cast<const float4*>(Pt + prob_of(j, ty * 2 + 1));
+      const ulonglong2 v0 = *reinterpret_cast<const ulonglong2*>(Vs + j * HD + tx * 4);
+      const ulonglong2 v1 = *reinterpret_cast<const ulonglong2*>(Vs + j * HD + HD / 2 + tx * 4);
+      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-      for (int ii = 0; ii < 4; ++ii) {
-        const float4 t4 = *reinterpret_cast<const float4*>(Ps + (ty * 4 + ii) * LD + j);
-        pv[ii][0] = t4.x; pv[ii][1] = t4.y; pv[ii][2] = t4.z; pv[ii][3] = t4.w;
-      }
-#pragma unroll
-      for (int jj = 0; jj < 4; ++jj) {
-        float vv[CPT];
-#pragma unroll
-        for (int c4 = 0; c4 < CPT / 4; ++c4) {
-          const float4 t4 = *reinterpret_cast<const float4*>(Vs + (j + jj) * VLD + tx * CPT + c4 * 4);
-          vv[c4 * 4] = t4.x; vv[c4 * 4 + 1] = t4.y; vv[c4 * 4 + 2] = t4.z; vv[c4 * 4 + 3] = t4.w;
-        }
-#pragma unroll
-        for (int ii = 0; ii < 4; ++ii)
-#pragma unroll
-          for (int c = 0; c < CPT; ++c) o[ii][c] = fmaf(pv[ii][jj], vv[c], o[ii][c]);
+      for (int i = 0; i < 8; ++i) {
+        const f32x2 a2 = pair_of(av[i], av[i]);
+        fma2(o[i][0], a2, v0.x);
+        fma2(o[i][1], a2, v0.y);
+        fma2(o[i][2], a2, v1.x);
+        fma2(o[i][3], a2, v1.y);
       }
     }
+    if (more) {
+#pragma unroll
+      for (int n = 0; n < NL; ++n) put(Kt, n, kn[n]);
+    }
+    __syncthreads();       // the next keys are there; nobody reads the values any more
+    if (more) bring_values(p + 1);
   }
 
 #pragma unroll
-  for (int ii = 0; ii < 4; ++ii) {
-    const int i = ty * 4 + ii;
-    if (i >= rows_here) continue;
-    const float inv = l_run[ii] > 0.0f ? 1.0f / l_run[ii] : 0.0f;
-    TOut* dst = out + (size_t)(row0 + q0 + i) * out_stride + (size_t)h * HD + tx * CPT;
+  for (int i = 0; i < 8; ++i) {
 #pragma unroll
-    for (int c = 0; c < CPT; ++c) dst[c] = nb_from_f32<TOut>(o[ii][c] * inv);
+    for (int off = TX / 2; off > 0; off >>= 1) l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], off);
+    if (ty * 8 + i >= rows_here) continue;
+    const float inv = l_run[i] > 0.0f ? 1.0f / l_run[i] : 0.0f;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const float2 x = unpair(o[i][2 * c]), y = unpair(o[i][2 * c + 1]);
+      TOut* dst = out + (size_t)(row0 + q0 + ty * 8 + i) * out_stride + (size_t)h * HD + c * (HD / 2) + tx * 4;
+      if (sizeof(TOut) == 4 && (vec & VEC_OUT)) {
+        *reinterpret_cast<float4*>(dst) = make_float4(x.x * inv, x.y * inv, y.x * inv, y.y * inv);
+      } else {
+        dst[0] = nb_from_f32<TOut>(x.x * inv); dst[1] = nb_from_f32<TOut>(x.y * inv);
+        dst[2] = nb_from_f32<TOut>(y.x * inv); dst[3] = nb_from_f32<TOut>(y.y * inv);
+      }
+    }
   }
 }
 
@@ -180,17 +282,21 @@ template <typename T, int HD, typename TOut>
 int launch(const void* q, int q_stride, int q_col, const int* cu_rows, const int* seq_slot,
            const int* seq_pos0, const NbPagedKV& kv, int n_heads, void* out, int out_stride,
            float scale, int window, int n_seqs, int max_q_len, cudaStream_t stream) {
-  const size_t smem = (size_t)(2 * HD * LD + PAGE_TOKENS * (HD + 4) + TQ * LD) * sizeof(float);
+  const size_t smem = (size_t)(2 * HD * LD + PAGE_TOKENS * (HD + LD)) * sizeof(float);
   auto kern = attention_prefill_f32_kernel<T, HD, TOut>;
   static bool configured = false;   // per instantiation
   if (!configured) {
     NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured = true;
   }
+  const bool vec_q = (uintptr_t)q % (4 * sizeof(T)) == 0 && q_stride % 4 == 0 && q_col % 4 == 0;
+  const bool vec_kv = (uintptr_t)kv.k % 16 == 0 && (uintptr_t)kv.v % 16 == 0;
+  const bool vec_out = (uintptr_t)out % 16 == 0 && out_stride % 4 == 0;
+  const int vec = (vec_q ? VEC_Q : 0) | (vec_kv ? VEC_KV : 0) | (vec_out ? VEC_OUT : 0);
   dim3 grid((max_q_len + TQ - 1) / TQ, n_heads, n_seqs);
-  NB_CUDA(nb_launch(kern, grid, dim3(THREADS), smem, stream, (const T*)q, q_stride, q_col, cu_rows,
+  NB_CUDA(nb_launch(kern, grid, dim3(HD), smem, stream, (const T*)q, q_stride, q_col, cu_rows,
                     seq_slot, seq_pos0, kv, n_heads / kv.n_kv_heads, (TOut*)out, out_stride, scale,
-                    window));
+                    window, vec, nb_device_sms()));
   return 0;
 }
 
