@@ -29,7 +29,14 @@ namespace {
 constexpr int THREADS = 128;
 constexpr int WARPS = 4;
 
-// G: query heads per key/value head served by one CTA (group <= G).
+// The kernel of a 32-bit cache.  G: query heads per key/value head served by one CTA (group <= G).
+//
+// A chain of dependent steps bounds it, not its bytes (8 sequences of some 250 tokens x 12 heads of 64
+// took 12.6 us, their keys and values 1.9), so the chain is kept short: where the step's rows are the only
+// thing the kernel in front writes (append > 0) the first pages are asked for ahead of the wait; a
+// warp takes the scores of up to 16 keys together, with one maximum and one rescaling for all
+// of them, instead of a running maximum every two keys; 2 to 8 splits meet in a cluster's shared
+// memory (`clustered`).
 template <typename T, int HD, int G, typename TOut>
 __global__ void __launch_bounds__(THREADS)
 attention_decode_kernel(const T* q, int q_stride, int q_col,
@@ -37,30 +44,31 @@ attention_decode_kernel(const T* q, int q_stride, int q_col,
                         NbPagedKV kv, int group, TOut* out, int out_stride,
                         float scale, float softcap, const float* sink, NbAttnOpts opt, int n_splits, float* part_acc,
                         float* part_ml, int* counters, int append,
-                        int k_col, int v_col) {
+                        int k_col, int v_col, bool clustered) {
   constexpr int EPL = Lane16<T>::N;           // elements per lane
   constexpr int LPR = HD / EPL;               // lanes per key row
-  constexpr int RPW = 32 / LPR;               // key rows per warp iteration
+  constexpr int RPW = 32 / LPR;               // key rows side by side in a warp
   constexpr int KEYS_PER_WARP = PAGE_TOKENS / WARPS;
   constexpr int ITERS = KEYS_PER_WARP / RPW;
+  constexpr int IB = ITERS * G <= 32 ? ITERS : 32 / G;   // turns whose scores are taken together
   constexpr int TILE = PAGE_TOKENS * HD;      // elements of one page of one head
   static_assert(LPR >= 1 && LPR <= 32 && (LPR & (LPR - 1)) == 0, "head size not supported");
-  static_assert(ITERS >= 1, "head size not supported");
+  static_assert(ITERS >= 1 && IB >= 1 && ITERS % IB == 0, "head size not supported");
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* tiles = reinterpret_cast<T*>(smem_raw);                       // [2 stages][K tile | V tile]
-  float* q_s = reinterpret_cast<float*>(smem_raw + (size_t)4 * TILE * sizeof(T));  // [G][HD]
-  float* w_acc = q_s + G * HD;                                     // [WARPS][G][HD]
+  float* w_acc = reinterpret_cast<float*>(smem_raw + (size_t)4 * TILE * sizeof(T));   // [WARPS][G][HD]
   float* w_ml = w_acc + WARPS * G * HD;                            // [WARPS][G][2]
+  float* c_part = w_ml + WARPS * G * 2;                            // clustered: [splits][group][HD + 2]
   __shared__ int s_last;
 
-  nb_grid_dependency_wait();
   const int split = blockIdx.x, kvh = blockIdx.y, r = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int sub = lane / LPR, part = lane % LPR;
   const int n_heads = kv.n_kv_heads * group;
   const int slot = row_slot[r];
   if (slot < 0) {   // padding row: zeros, written by split 0
+    nb_grid_dependency_wait();
     if (split == 0)
       for (int i = tid; i < group * HD; i += THREADS)
         out[(size_t)r * out_stride + (size_t)kvh * group * HD + i] = nb_from_f32<TOut>(0.0f);
@@ -81,14 +89,6 @@ attention_decode_kernel(const T* q, int q_stride, int q_col,
   const int p_end = head_split ? min((keep_first + PAGE_TOKENS - 1) / PAGE_TOKENS, first_page)
                                : min(first_page + n_pages, p_begin + per_split);
 
-  // queries of the group, fp32
-  for (int i = tid; i < G * HD; i += THREADS) {
-    const int gh = i / HD, c = i - gh * HD;
-    q_s[i] = (gh < group)
-                 ? nb_to_f32(q[(size_t)r * q_stride + q_col + (size_t)(kvh * group + gh) * HD + c])
-                 : 0.0f;
-  }
-
   const int* table = kv.block_table + (size_t)slot * kv.max_pages;
   auto issue = [&](int page_idx, int stage) {
     const int page_id = table[page_idx];
@@ -96,39 +96,42 @@ attention_decode_kernel(const T* q, int q_stride, int q_col,
     const T* vsrc = (const T*)kv.v + ((size_t)page_id * kv.n_kv_heads + kvh) * TILE;
     T* kdst = tiles + (size_t)stage * 2 * TILE;
     T* vdst = kdst + TILE;
-    constexpr int VECS = TILE / EPL;   // 16-byte pieces per tile
-    for (int i = tid; i < VECS; i += THREADS) {
+    // only the rows that hold keys: scores and values of the others are replaced, never used
+    const int vecs = min(PAGE_TOKENS, kv_len - page_idx * PAGE_TOKENS) * LPR;   // 16-byte pieces
+#pragma unroll 4
+    for (int i = tid; i < vecs; i += THREADS) {
       cp_async16(kdst + i * EPL, ksrc + i * EPL);
       cp_async16(vdst + i * EPL, vsrc + i * EPL);
     }
-    cp_async_commit();
   };
 
-  float m_run[G], l_run[G], acc[G][EPL];
+  // append > 0: the step's own key and value come with the query row, the rest of the pages was
+  // written by earlier steps; else the kernel in front may have written the cache
+  if (append <= 0) nb_grid_dependency_wait();
+  if (p_begin < p_end) issue(p_begin, 0);
+  cp_async_commit();
+  if (p_begin + 1 < p_end) issue(p_begin + 1, 1);
+  cp_async_commit();
+  nb_grid_dependency_wait();
+  // every CTA of a cluster says that it runs (see the tensor-core kernel)
+  if (clustered) asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
+
+  float m_run[G], l_run[G], acc[G][EPL], qreg[G][EPL];
 #pragma unroll
   for (int gh = 0; gh < G; ++gh) {
     m_run[gh] = -INFINITY;
     l_run[gh] = 0.0f;
 #pragma unroll
-    for (int e = 0; e < EPL; ++e) acc[gh][e] = 0.0f;
+    for (int e = 0; e < EPL; ++e) {
+      acc[gh][e] = 0.0f;
+      qreg[gh][e] = (gh < group) ? nb_to_f32(q[(size_t)r * q_stride + q_col + (size_t)(kvh * group + gh) * HD + part * EPL + e])
+                                 : 0.0f;
+    }
   }
-
-  if (p_begin < p_end) issue(p_begin, 0);
-  __syncthreads();   // q_s is complete
-  float qreg[G][EPL];
-#pragma unroll
-  for (int gh = 0; gh < G; ++gh)
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) qreg[gh][e] = q_s[gh * HD + part * EPL + e];
 
   for (int p = p_begin; p < p_end; ++p) {
     const int stage = (p - p_begin) & 1;
-    if (p + 1 < p_end) {
-      issue(p + 1, stage ^ 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
+    cp_async_wait<1>();
     __syncthreads();
     T* kt = tiles + (size_t)stage * 2 * TILE;
     T* vt = kt + TILE;
@@ -149,44 +152,77 @@ attention_decode_kernel(const T* q, int q_stride, int q_col,
       }
       __syncthreads();
     }
+#pragma unroll 1
+    for (int it0 = 0; it0 < ITERS; it0 += IB) {
+      const int row0 = warp * KEYS_PER_WARP + it0 * RPW + sub;   // this lane's first key within the page
+      const int j0 = p * PAGE_TOKENS + row0;
+      float sc[G][IB];
 #pragma unroll
-    for (int it = 0; it < ITERS; ++it) {
-      const int row = warp * KEYS_PER_WARP + it * RPW + sub;   // key within the page
-      const int j = p * PAGE_TOKENS + row;
-      const bool valid = (j >= j_begin || j < keep_first) && (j < kv_len);
-      float kf[EPL], vf[EPL];
-      Lane16<T>::load(kt + (size_t)row * HD + part * EPL, kf);
-      Lane16<T>::load(vt + (size_t)row * HD + part * EPL, vf);
-      if (!valid) {   // whatever an unused cache row holds must not reach the sum
+      for (int it = 0; it < IB; ++it) {
+        float kf[EPL];
+        Lane16<T>::load(kt + (size_t)(row0 + it * RPW) * HD + part * EPL, kf);
 #pragma unroll
-        for (int e = 0; e < EPL; ++e) vf[e] = 0.0f;
+        for (int gh = 0; gh < G; ++gh) {
+          float dot = 0.0f;
+#pragma unroll
+          for (int e = 0; e < EPL; ++e) dot = fmaf(qreg[gh][e], kf[e], dot);
+          sc[gh][it] = dot;
+        }
+      }
+#pragma unroll
+      for (int o = LPR / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int it = 0; it < IB; ++it)
+#pragma unroll
+          for (int gh = 0; gh < G; ++gh) sc[gh][it] += __shfl_xor_sync(0xffffffffu, sc[gh][it], o);
+      bool valid[IB];
+#pragma unroll
+      for (int it = 0; it < IB; ++it) {
+        const int j = j0 + it * RPW;
+        valid[it] = (j >= j_begin || j < keep_first) && j < kv_len;
       }
 #pragma unroll
       for (int gh = 0; gh < G; ++gh) {
-        float dot = 0.0f;
+        float mx = -INFINITY;
 #pragma unroll
-        for (int e = 0; e < EPL; ++e) dot = fmaf(qreg[gh][e], kf[e], dot);
-#pragma unroll
-        for (int o = LPR / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        float s = dot * scale;
-        if (softcap > 0.0f) s = softcap * tanhf(s / softcap);
-        if (!valid) s = -INFINITY;
-        float mx = s;
+        for (int it = 0; it < IB; ++it) {
+          float s = sc[gh][it] * scale;
+          if (softcap > 0.0f) s = softcap * tanhf(s / softcap);
+          sc[gh][it] = valid[it] ? s : -INFINITY;
+          mx = fmaxf(mx, sc[gh][it]);
+        }
 #pragma unroll
         for (int o = LPR; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         const float m_new = fmaxf(m_run[gh], mx);
-        if (m_new > -INFINITY) {   // warp-uniform
-          const float rescale = (m_run[gh] == -INFINITY) ? 0.0f : expf(m_run[gh] - m_new);
-          const float pr = valid ? expf(s - m_new) : 0.0f;
-          l_run[gh] = l_run[gh] * rescale + pr;
+        const float m_use = m_new == -INFINITY ? 0.0f : m_new;      // nothing to attend to yet
+        const float rescale = (m_run[gh] == -INFINITY) ? 0.0f : expf(m_run[gh] - m_use);
+        l_run[gh] *= rescale;
 #pragma unroll
-          for (int e = 0; e < EPL; ++e) acc[gh][e] = fmaf(pr, vf[e], acc[gh][e] * rescale);
-          m_run[gh] = m_new;
+        for (int e = 0; e < EPL; ++e) acc[gh][e] *= rescale;
+        m_run[gh] = m_new;
+#pragma unroll
+        for (int it = 0; it < IB; ++it) {
+          sc[gh][it] = valid[it] ? expf(sc[gh][it] - m_use) : 0.0f;
+          l_run[gh] += sc[gh][it];
         }
       }
+#pragma unroll
+      for (int it = 0; it < IB; ++it) {
+        float vf[EPL];
+        Lane16<T>::load(vt + (size_t)(row0 + it * RPW) * HD + part * EPL, vf);
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) vf[e] = valid[it] ? vf[e] : 0.0f;   // what an unused row holds must not reach the sum
+#pragma unroll
+        for (int gh = 0; gh < G; ++gh)
+#pragma unroll
+          for (int e = 0; e < EPL; ++e) acc[gh][e] = fmaf(sc[gh][it], vf[e], acc[gh][e]);
+      }
     }
-    __syncthreads();   // the stage is free for the copy after next
+    __syncthreads();   // the stage is free
+    if (p + 2 < p_end) issue(p + 2, stage);
+    cp_async_commit();
   }
+  cp_async_wait<0>();
 
   nb_launch_dependents();   // the pages are read: the next kernel may be set up
   // merge the key rows a warp handled side by side (lanes with equal `part`)
@@ -209,6 +245,12 @@ attention_decode_kernel(const T* q, int q_stride, int q_col,
     }
   }
   __syncthreads();
+  unsigned c_remote = 0;    // this split's place in split 0's shared memory
+  if (clustered) {
+    asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
+    const unsigned local = (unsigned)__cvta_generic_to_shared(c_part + (size_t)split * group * (HD + 2));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(c_remote) : "r"(local), "r"(0));
+  }
   // merge the warps -> partial result of this split
   for (int i = tid; i < group * HD; i += THREADS) {
     const int gh = i / HD, c = i - gh * HD;
@@ -230,6 +272,15 @@ attention_decode_kernel(const T* q, int q_stride, int q_col,
       out[(size_t)r * out_stride + (size_t)head * HD + c] = nb_from_f32<TOut>(l > 0.0f ? a / l : a);
       continue;
     }
+    if (clustered) {
+      const unsigned at = c_remote + (unsigned)(gh * (HD + 2)) * 4u;
+      asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(at + (unsigned)c * 4u), "f"(a) : "memory");
+      if (c == 0) {
+        asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(at + (unsigned)HD * 4u), "f"(M) : "memory");
+        asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(at + (unsigned)(HD + 1) * 4u), "f"(l) : "memory");
+      }
+      continue;
+    }
     const size_t pi = ((size_t)r * n_heads + head) * n_splits + split;
     part_acc[pi * HD + c] = a;
     if (c == 0) {
@@ -238,6 +289,31 @@ attention_decode_kernel(const T* q, int q_stride, int q_col,
     }
   }
   if (n_splits == 1) return;
+  if (clustered) {
+    // the stores above are visible to split 0 once every CTA has arrived (release) and split 0
+    // has waited (acquire); the other splits wait too, so that none leaves the cluster early
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    if (split != 0) return;
+    for (int i = tid; i < group * HD; i += THREADS) {
+      const int gh = i / HD, c = i - gh * HD, head = kvh * group + gh;
+      const float* row = c_part + (size_t)gh * (HD + 2);
+      const int step = group * (HD + 2);
+      float M = -INFINITY;
+      for (int s = 0; s < n_splits; ++s) M = fmaxf(M, row[s * step + HD]);
+      float a = 0.0f, l = 0.0f;
+      for (int s = 0; s < n_splits; ++s) {
+        const float ms = row[s * step + HD];
+        const float f = (ms == -INFINITY) ? 0.0f : expf(ms - M);
+        a += f * row[s * step + c];
+        l += f * row[s * step + HD + 1];
+      }
+      if (sink != nullptr) a *= nb_sink_fix(l, M, sink[head], false);
+      a *= opt.gate_of(r, head);
+      out[(size_t)r * out_stride + (size_t)head * HD + c] = nb_from_f32<TOut>(l > 0.0f ? a / l : a);
+    }
+    return;
+  }
   // the CTA that finishes last for this (row, key/value head) merges the splits
   __threadfence();
   __syncthreads();
@@ -299,16 +375,17 @@ template <typename T, int HD, int G, typename TOut>
 int launch(const void* q, int q_stride, int q_col, const int* row_slot, const int* row_pos,
            const NbPagedKV& kv, int group, void* out, int out_stride, float scale, float softcap, const float* sink, NbAttnOpts opt,
            int n_rows, int n_splits, float* part_acc, float* part_ml, int* counters, int append,
-           int k_col, int v_col, cudaStream_t stream) {
-  const size_t smem = (size_t)4 * PAGE_TOKENS * HD * sizeof(T) +
-                      (size_t)(G * HD + WARPS * G * HD + WARPS * G * 2) * sizeof(float);
+           int k_col, int v_col, bool clustered, cudaStream_t stream) {
+  const size_t own = (size_t)4 * PAGE_TOKENS * HD * sizeof(T) + (size_t)(WARPS * G * HD + WARPS * G * 2) * sizeof(float);
+  const size_t most = own + (size_t)MAX_CLUSTER * G * (HD + 2) * sizeof(float);
+  const size_t smem = own + (clustered ? (size_t)n_splits * group * (HD + 2) * sizeof(float) : 0);
   auto kern = attention_decode_kernel<T, HD, G, TOut>;
-  if (smem > 48 * 1024)
-    NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (most > 48 * 1024)
+    NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
   dim3 grid(n_splits, kv.n_kv_heads, n_rows);
-  NB_CUDA(nb_launch(kern, grid, dim3(THREADS), smem, stream, (const T*)q, q_stride, q_col, row_slot,
-                    row_pos, kv, group, (TOut*)out, out_stride, scale, softcap, sink, opt, n_splits, part_acc,
-                    part_ml, counters, append, k_col, v_col));
+  NB_CUDA(nb_launch_clusters(kern, grid, dim3(THREADS), smem, stream, clustered ? n_splits : 1, (const T*)q, q_stride,
+                             q_col, row_slot, row_pos, kv, group, (TOut*)out, out_stride, scale, softcap, sink, opt,
+                             n_splits, part_acc, part_ml, counters, append, k_col, v_col, clustered));
   return 0;
 }
 
@@ -316,9 +393,9 @@ template <typename T, int HD, typename TOut>
 int by_group(int group, const void* q, int q_stride, int q_col, const int* row_slot,
              const int* row_pos, const NbPagedKV& kv, void* out, int out_stride, float scale, float softcap,
              const float* sink, NbAttnOpts opt, int n_rows, int n_splits, float* pa, float* pm, int* cn, int ap,
-             int kc, int vc, cudaStream_t st) {
+             int kc, int vc, bool clustered, cudaStream_t st) {
 #define NB_G(G_) \
-  return launch<T, HD, G_, TOut>(q, q_stride, q_col, row_slot, row_pos, kv, group, out, out_stride, scale, softcap, sink, opt, n_rows, n_splits, pa, pm, cn, ap, kc, vc, st)
+  return launch<T, HD, G_, TOut>(q, q_stride, q_col, row_slot, row_pos, kv, group, out, out_stride, scale, softcap, sink, opt, n_rows, n_splits, pa, pm, cn, ap, kc, vc, clustered, st)
   if (group == 1) NB_G(1);
   if (group == 2) NB_G(2);
   if (group <= 4) NB_G(4);
@@ -330,9 +407,9 @@ template <typename T, typename TOut>
 int by_head_dim(int hd, int group, const void* q, int q_stride, int q_col, const int* row_slot,
                 const int* row_pos, const NbPagedKV& kv, void* out, int out_stride, float scale, float softcap,
                 const float* sink, NbAttnOpts opt, int n_rows, int n_splits, float* pa, float* pm, int* cn, int ap,
-                int kc, int vc, cudaStream_t st) {
+                int kc, int vc, bool clustered, cudaStream_t st) {
 #define NB_HD(HD_) \
-  return by_group<T, HD_, TOut>(group, q, q_stride, q_col, row_slot, row_pos, kv, out, out_stride, scale, softcap, sink, opt, n_rows, n_splits, pa, pm, cn, ap, kc, vc, st)
+  return by_group<T, HD_, TOut>(group, q, q_stride, q_col, row_slot, row_pos, kv, out, out_stride, scale, softcap, sink, opt, n_rows, n_splits, pa, pm, cn, ap, kc, vc, clustered, st)
   switch (hd) {
     case 16: NB_HD(16);
     case 32: NB_HD(32);
@@ -393,16 +470,16 @@ int attention_decode(const void* q, int dtype, int q_stride, int q_col, const in
   const int group = n_heads / n_kv_heads;
   typedef __nv_bfloat16 bf16;
   int rc;
-#define NB_ARGS head_dim, group, q, q_stride, q_col, row_slot, row_pos, kv, out, out_stride, scale, softcap, sink, opt, n_rows, n_splits, part_acc, part_ml, counters, append, k_col, v_col, stream
+#define NB_ARGS head_dim, group, q, q_stride, q_col, row_slot, row_pos, kv, out, out_stride, scale, softcap, sink, opt, n_rows, n_splits, part_acc, part_ml, counters, append, k_col, v_col, clustered, stream
+  // up to MAX_CLUSTER splits merge through the shared memory of a thread-block cluster, more
+  // through the scratch arrays and a counter
+  const bool clustered = clusters_allowed > 0 && n_splits >= 2 && n_splits <= MAX_CLUSTER;
   if (dtype == NB_F32) {
     rc = out_dtype == NB_F32 ? by_head_dim<float, float>(NB_ARGS) : by_head_dim<float, bf16>(NB_ARGS);
   } else {
     // bf16 cache: tensor cores (needs 16-byte aligned rows and 4-byte aligned query columns)
     NB_REQUIRE(q_stride % 8 == 0 && q_col % 2 == 0 && (uintptr_t)q % 16 == 0, NB_ERR_UNSUPPORTED,
                "attention_decode: query rows must be 16-byte aligned");
-    // up to MAX_CLUSTER splits merge through the shared memory of a thread-block cluster, more
-    // through the scratch arrays and a counter
-    const bool clustered = clusters_allowed > 0 && n_splits >= 2 && n_splits <= MAX_CLUSTER;
     rc = out_dtype == NB_F32
              ? mma_by_head_dim<float>(head_dim, q, q_stride, q_col, row_slot, row_pos, kv, group, out, out_stride, scale, softcap, sink, opt, n_rows, n_splits, part_acc, part_ml, counters, append, k_col, v_col, clustered, stream)
              : mma_by_head_dim<bf16>(head_dim, q, q_stride, q_col, row_slot, row_pos, kv, group, out, out_stride, scale, softcap, sink, opt, n_rows, n_splits, part_acc, part_ml, counters, append, k_col, v_col, clustered, stream);

@@ -29,7 +29,6 @@ PARAM_ACTIVATIONS = {"swish_clamp"}
 ROW_ACTIVATIONS = {"tanh": ACT_TANH, "xielu": ACT_XIELU}
 
 _DTYPE_CODE = {torch.float32: 0, torch.bfloat16: 1}
-DECODE_TARGET_CTAS = 4 * 148   # CTAs the split 32-bit decode attention aims to put on the GPU
 # CTAs the tensor-core prefill attention aims to put on the GPU by cutting the keys of a tile
 # into runs: one per SM.  (Two of its CTAs on an SM are bound by instruction issue, so cutting
 # further only adds the merge; measured on GPT-2 124M, 2 x 1024 tokens.)
@@ -61,6 +60,15 @@ def decode_splits(base_ctas: int, pages: int, page: int, head_dim: int, sms: int
     while 2 * s <= most and 2 * s * base_ctas <= sms and pages % (2 * s) == 0:
         s *= 2
     return s
+
+
+def decode_splits_f32(base_ctas: int, pages: int, page: int, head_dim: int, sms: int, cluster: int) -> int:
+    """Splits of a sequence's pages in the 32-bit decode attention: as many as put one launch on the
+    GPU at once (a CTA keeps two pages of keys and values, 64 KB with heads of 64), no more than merge
+    inside a cluster (`cluster`, 0: none do) unless a split would then walk over more than four pages."""
+    room = max(1, min(8, (228 * 1024) // (4 * page * head_dim * 4 + 4096))) * sms
+    s = max(1, min(pages, room // base_ctas))
+    return min(s, cluster) if 0 < cluster and pages <= 4 * cluster else s
 
 
 def latent_splits(ctas: int, pages: int, sms: int) -> int:
@@ -489,10 +497,10 @@ class CudaBackend:
     # -- cache and attention ----------------------------------------------------------
     def _decode_splits(self, base_ctas: int, pages: int, kv, dtype) -> int:
         """Into how many splits a decode launch cuts each sequence's pages (`base_ctas`: rows x
-        key-value heads).  The 32-bit kernel aims at a fixed number of CTAs; the tensor-core
-        kernel follows `decode_splits`."""
+        key-value heads): `decode_splits_f32` and, on the tensor cores, `decode_splits`."""
         if dtype != torch.bfloat16:
-            return max(1, min(pages, DECODE_TARGET_CTAS // base_ctas))
+            return decode_splits_f32(base_ctas, pages, kv.page, kv.head_dim, self._sms,
+                                     self._cluster_limit if self.decode_clusters else 0)
         return decode_splits(base_ctas, pages, kv.page, kv.head_dim, self._sms,
                              self._cluster_limit if self.decode_clusters else 16)
 
