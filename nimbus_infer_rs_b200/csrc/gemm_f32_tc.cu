@@ -57,16 +57,21 @@ namespace {
 
 typedef __nv_bfloat16 bf16;
 
-constexpr int BM = 128, BN = 128, BK = 64;
-constexpr int PIECE = BM * BK * 2;          // bytes of a 128 x 64 box
-constexpr int BLOCK_BYTES = 6 * PIECE;      // X's three pieces, W's three pieces
+constexpr int BM = 128, BK = 64;
 constexpr int STAGES = 2;                   // blocks of K in flight
-constexpr int SMALL = 4;                    // blocks of K whose small terms are added up in one place
-constexpr int EPI = 16;                     // warps of the epilogue
-constexpr int THREADS = 64 + 32 * EPI;
-constexpr int OLD = BN + 4;                 // floats between rows of the finished tile
-constexpr int SMEM = STAGES * BLOCK_BYTES + 1024 + 256;
-static_assert(BM * OLD * 4 <= STAGES * BLOCK_BYTES, "the finished tile goes where the ring was");
+constexpr int SMALL = 8;                    // blocks of K whose small terms are added up in one place
+
+template <int BN>                           // columns of a tile
+struct Tile {
+  static constexpr int XPIECE = BM * BK * 2, WPIECE = BN * BK * 2;        // bytes of the boxes
+  static constexpr int BLOCK_BYTES = 3 * (XPIECE + WPIECE);               // X's three pieces, W's three pieces
+  static constexpr int EPI = 4 * (BN / 32);                               // warps of the epilogue
+  static constexpr int THREADS = 64 + 32 * EPI;
+  static constexpr int OLD = BN + 4;                                      // floats between rows of the finished tile
+  static constexpr int SMEM = STAGES * BLOCK_BYTES + 1024 + 256;
+  static_assert(BN % 32 == 0 && BN <= 128, "large and small accumulators fill the tensor memory");
+  static_assert(BM * OLD * 4 <= STAGES * BLOCK_BYTES, "the finished tile goes where the ring was");
+};
 
 __device__ __forceinline__ void split3(float x, bf16& h, bf16& m, bf16& l) {
   h = __float2bfloat16_rn(x);
@@ -87,39 +92,52 @@ __device__ __forceinline__ void tc05_ld_32x32b_x16(uint32_t taddr, uint32_t (&v)
       : "memory");
 }
 
-// Rows 0 .. M-1 of X and 0 .. N-1 of W, a warp each, into pieces [3][rows][K]; scale[row] is what
+// Rows 0 .. M-1 of X and 0 .. N-1 of W, WPR warps each, into pieces [3][rows][K]; scale[row] is what
 // a result of the row is to be multiplied by, 0 for rows that cannot be split (their pieces are zeros).
-// K % 4 == 0.
+// K % 4 == 0.  Bound by its bytes and by how many of them are on their way: a row of up to HELD
+// pieces of four numbers a thread is read once, all of it asked for together, and kept.
+constexpr int HELD = 8;
+template <int WPR>
 __global__ void __launch_bounds__(256)
 split_kernel(const float* X, const float* __restrict__ W, bf16* xp, bf16* wp, float* x_scale,
-             float* w_scale,             int M, int N, int K) {
+             float* w_scale, int M, int N, int K) {
+  constexpr int TPR = 32 * WPR, ROWS = 8 / WPR;
+  __shared__ float s_top[8];
   nb_grid_dependency_wait();
   nb_launch_dependents();
-  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (row >= M + N) return;
-  const bool is_w = row >= M;
+  const int warp = threadIdx.x >> 5, row = blockIdx.x * ROWS + warp / WPR, t = threadIdx.x % TPR;
+  const bool live = row < M + N, is_w = row >= M;
   const int r = is_w ? row - M : row, rows = is_w ? N : M;
   const float4* src = reinterpret_cast<const float4*>((is_w ? W : X) + (size_t)r * K);
   bf16* dst = (is_w ? wp : xp) + (size_t)r * K;
+  const int n = live ? K / 4 : 0;
+  float4 f[HELD];
+  // the largest magnitude of the row; infinity where one of its numbers is not finite
   float top = 0.0f;
-  bool finite = true;
-  for (int k = lane; k < K / 4; k += 32) {
-    const float4 f = src[k];
-    const float v[4] = {f.x, f.y, f.z, f.w};
+  auto see = [&](const float4& q) {
+    const float v[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      finite = finite && (__float_as_uint(v[e]) & 0x7f800000u) != 0x7f800000u;
-      top = fmaxf(top, fabsf(v[e]));
-    }
-  }
-  finite = __all_sync(0xffffffffu, finite);
+    for (int e = 0; e < 4; ++e)
+      top = fmaxf(top, (__float_as_uint(v[e]) & 0x7f800000u) != 0x7f800000u ? fabsf(v[e]) : INFINITY);
+  };
+#pragma unroll
+  for (int i = 0; i < HELD; ++i)
+    f[i] = t + i * TPR < n ? src[t + i * TPR] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+  for (int i = 0; i < HELD; ++i) see(f[i]);
+  for (int k = t + HELD * TPR; k < n; k += TPR) see(src[k]);
   top = nb_warp_max(top);
-  const bool whole = finite && top <= 0x1p50f;
+  if constexpr (WPR > 1) {
+    if ((threadIdx.x & 31) == 0) s_top[warp] = top;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < WPR; ++i) top = fmaxf(top, s_top[warp / WPR * WPR + i]);
+  }
+  const bool whole = top <= 0x1p50f;
   const int up = whole && top > 0.0f && top < 0x1p-30f ? -ilogbf(top) : 0;
-  if (lane == 0) (is_w ? w_scale : x_scale)[r] = whole ? ldexpf(1.0f, -up) : 0.0f;
-  for (int k = lane; k < K / 4; k += 32) {
-    const float4 f = src[k];
-    float v[4] = {f.x, f.y, f.z, f.w};
+  if (live && t == 0) (is_w ? w_scale : x_scale)[r] = whole ? ldexpf(1.0f, -up) : 0.0f;
+  auto put = [&](int k, const float4& q) {
+    float v[4] = {q.x, q.y, q.z, q.w};
     if (up != 0 || !whole) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) v[e] = whole ? ldexpf(v[e], up) : 0.0f;
@@ -130,15 +148,21 @@ split_kernel(const float* X, const float* __restrict__ W, bf16* xp, bf16* wp, fl
 #pragma unroll
     for (int i = 0; i < 3; ++i)
       *reinterpret_cast<uint2*>(dst + (size_t)i * rows * K + k * 4) = *reinterpret_cast<const uint2*>(p[i]);
-  }
+  };
+#pragma unroll
+  for (int i = 0; i < HELD; ++i)
+    if (t + i * TPR < n) put(t + i * TPR, f[i]);
+  for (int k = t + HELD * TPR; k < n; k += TPR) put(k, src[k]);
 }
 
-template <typename TOut>
-__global__ void __launch_bounds__(THREADS, 1)
+template <int BN, typename TOut>
+__global__ void __launch_bounds__(Tile<BN>::THREADS, 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                    const float* X, const float* __restrict__ W, const float* x_scale, const float* w_scale,
                    const float* __restrict__ bias, const float* residual, TOut* out, int ld, int M, int N,
                    int K, int act, int tiles_n, int run, int* err_word) {
+  constexpr int XPIECE = Tile<BN>::XPIECE, WPIECE = Tile<BN>::WPIECE, BLOCK_BYTES = Tile<BN>::BLOCK_BYTES;
+  constexpr int EPI = Tile<BN>::EPI, OLD = Tile<BN>::OLD;
   extern __shared__ unsigned char smem_dyn[];
   const uint32_t raw = smem_u32(smem_dyn);
   const uint32_t base = (raw + 1023u) & ~1023u;          // swizzle atoms are 1024 bytes
@@ -146,10 +170,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   const uint32_t bars = base + STAGES * BLOCK_BYTES;
   auto full = [&](int s, int p) { return bars + 8u * (s * 3 + p); };       // one a piece
   auto empty = [&](int s) { return bars + 8u * (3 * STAGES + s); };
-  // accumulators 0 and 1: large terms, 2 and 3: small terms
+  // accumulators 0 and 1: large terms, 2: small terms, in two halves
   auto acc_full = [&](int b) { return bars + 8u * (4 * STAGES + b); };
-  auto acc_empty = [&](int b) { return bars + 8u * (4 * STAGES + 4 + b); };
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_dyn + (bars - raw) + 8 * (4 * STAGES + 8));
+  auto acc_empty = [&](int b) { return bars + 8u * (4 * STAGES + 3 + b); };
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_dyn + (bars - raw) + 8 * (4 * STAGES + 6));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = (int)(blockIdx.x / tiles_n) * BM, n0 = (int)(blockIdx.x % tiles_n) * BN;
@@ -160,7 +184,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       for (int p = 0; p < 3; ++p) mbar_init(full(s, p), 1);
       mbar_init(empty(s), 1);
     }
-    for (int b = 0; b < 4; ++b) {
+    for (int b = 0; b < 3; ++b) {
       mbar_init(acc_full(b), 1);
       mbar_init(acc_empty(b), EPI);
     }
@@ -188,65 +212,57 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         if (!mbar_wait(empty(s), (((uint32_t)(kb / STAGES)) & 1u) ^ 1u, abort_flag)) break;
         const uint32_t st = base + (uint32_t)(s * BLOCK_BYTES);
         for (int p = 0; p < 3; ++p) {        // a box beyond its piece's rows brings rows nobody stores
-          mbar_expect_tx(full(s, p), 2u * PIECE);
-          tma_load_2d(st + (uint32_t)(p * PIECE), &map_x, kb * BK, p * M + m0, full(s, p));
-          tma_load_2d(st + (uint32_t)((3 + p) * PIECE), &map_w, kb * BK, p * N + n0, full(s, p));
+          mbar_expect_tx(full(s, p), (uint32_t)(XPIECE + WPIECE));
+          tma_load_2d(st + (uint32_t)(p * XPIECE), &map_x, kb * BK, p * M + m0, full(s, p));
+          tma_load_2d(st + (uint32_t)(3 * XPIECE + p * WPIECE), &map_w, kb * BK, p * N + n0, full(s, p));
         }
       }
     }
     __syncwarp();
   } else if (warp == 1) {
     if (lane == 0) {
-      constexpr uint32_t idesc = instr_desc_bf16(BM, BN);
+      constexpr uint32_t one = instr_desc_bf16(BM, BN), two = instr_desc_bf16(BM, 2 * BN);
       bool ok = true;
       for (int kb = 0; kb < blocks; ++kb) {
-        const int s = kb % STAGES, g = kb / SMALL, small = 2 + (g & 1);
+        const int s = kb % STAGES, g = kb / SMALL;
         const bool first = kb % SMALL == 0, last = kb % SMALL == SMALL - 1 || kb + 1 == blocks;
         const uint32_t phase = (uint32_t)(kb / STAGES) & 1u;
         const uint32_t st = base + (uint32_t)(s * BLOCK_BYTES);
-        // 16 of K, from `k` of the block on: X's piece px times W's piece pw
-        auto product = [&](int px, int pw, int k, int b, bool fresh) {
-          const uint64_t da = smem_desc_sw128(st + (uint32_t)(px * PIECE));
-          const uint64_t db = smem_desc_sw128(st + (uint32_t)((3 + pw) * PIECE));
-          tc05_mma_bf16(tmem + (uint32_t)b * 128u, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc,
+        // 16 of K, from `k` of the block on: X's piece px times W's piece pw, or times that and the next
+        // one, which follows it in shared memory as 2 BN rows of one operand: the results lie side by side
+        auto product = [&](uint32_t idesc, int px, int pw, int k, int col, bool fresh) {
+          const uint64_t da = smem_desc_sw128(st + (uint32_t)(px * XPIECE));
+          const uint64_t db = smem_desc_sw128(st + (uint32_t)(3 * XPIECE + pw * WPIECE));
+          tc05_mma_bf16(tmem + (uint32_t)col, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc,
                         fresh ? 0u : 1u);
         };
-        auto large = [&](int b) {            // the large terms of half a block, for the epilogue to take out
-          product(0, 0, 2 * b, b, true);
-          product(0, 0, 2 * b + 1, b, false);
+        // the large terms, half a block at a time, for the epilogue to take out
+        ok = mbar_wait(full(s, 0), phase, abort_flag);
+        for (int b = 0; b < 2 && ok; ++b) {
+          ok = mbar_wait(acc_empty(b), ((uint32_t)kb & 1u) ^ 1u, abort_flag);
+          if (!ok) break;
+          tc05_fence_after();
+          product(one, 0, 0, 2 * b, b * 128, true);
+          product(one, 0, 0, 2 * b + 1, b * 128, false);
           tc05_commit(acc_full(b));
-        };
-        ok = mbar_wait(full(s, 0), phase, abort_flag) &&
-             mbar_wait(acc_empty(0), ((uint32_t)kb & 1u) ^ 1u, abort_flag);
-        if (!ok) break;
-        tc05_fence_after();
-        large(0);
-        if (first) ok = mbar_wait(acc_empty(small), ((uint32_t)(g >> 1) & 1u) ^ 1u, abort_flag);
+        }
+        if (first && ok) ok = mbar_wait(acc_empty(2), ((uint32_t)g & 1u) ^ 1u, abort_flag);
         ok = ok && mbar_wait(full(s, 1), phase, abort_flag);
         if (!ok) break;
         tc05_fence_after();
 #pragma unroll
-        for (int k = 0; k < BK / 16; ++k) {
-          product(0, 1, k, small, first && k == 0);
-          product(1, 0, k, small, false);
-          product(1, 1, k, small, false);
-        }
-        ok = mbar_wait(acc_empty(1), ((uint32_t)kb & 1u) ^ 1u, abort_flag);
-        if (!ok) break;
-        tc05_fence_after();
-        large(1);
+        for (int k = 0; k < BK / 16; ++k) product(two, 1, 0, k, 256, first && k == 0);      // mh' | mm'
         ok = mbar_wait(full(s, 2), phase, abort_flag);
         if (!ok) break;
         tc05_fence_after();
 #pragma unroll
         for (int k = 0; k < BK / 16; ++k) {
-          product(0, 2, k, small, false);
-          product(2, 0, k, small, false);
-          product(1, 2, k, small, false);
-          product(2, 1, k, small, false);
+          product(two, 0, 1, k, 256, false);         // hm' | hl'
+          product(two, 2, 0, k, 256, false);         // lh' | lm'
+          product(one, 1, 2, k, 256, false);         // ml'
         }
         tc05_commit(empty(s));
-        if (last) tc05_commit(acc_full(small));
+        if (last) tc05_commit(acc_full(2));
       }
     }
     __syncwarp();
@@ -260,13 +276,15 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     auto take_out = [&](int b, uint32_t parity) {
       if (!__all_sync(0xffffffffu, mbar_wait(acc_full(b), parity, abort_flag))) return false;
       tc05_fence_after();
+      for (int half = 0; half < (b == 2 ? 2 : 1); ++half) {
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        uint32_t v[16];
-        tc05_ld_32x32b_x16(lanes + (uint32_t)(b * 128 + q * 16), v);
-        tc05_wait_ld();
+        for (int q = 0; q < 2; ++q) {
+          uint32_t v[16];
+          tc05_ld_32x32b_x16(lanes + (uint32_t)(b * 128 + half * BN + q * 16), v);
+          tc05_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 16; ++j) u[q * 16 + j] += __uint_as_float(v[j]);
+          for (int j = 0; j < 16; ++j) u[q * 16 + j] += __uint_as_float(v[j]);
+        }
       }
       tc05_fence_before();
       __syncwarp();
@@ -277,7 +295,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     for (int kb = 0, left = run; kb < blocks && ok; ++kb) {
       const int g = kb / SMALL;
       ok = take_out(0, (uint32_t)kb & 1u) && take_out(1, (uint32_t)kb & 1u);
-      if (ok && (kb % SMALL == SMALL - 1 || kb + 1 == blocks)) ok = take_out(2 + (g & 1), (uint32_t)(g >> 1) & 1u);
+      if (ok && (kb % SMALL == SMALL - 1 || kb + 1 == blocks)) ok = take_out(2, (uint32_t)g & 1u);
       if (--left == 0 || kb + 1 == blocks) {
         left = run;
 #pragma unroll
@@ -299,9 +317,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   __syncthreads();
   const bool aborted = *abort_flag != 0;
   if (!aborted && warp >= 2) {
-    // a warp a row at a time: four columns a lane
+    // a warp a row at a time: four columns a lane (of a narrower tile the first lanes only)
     const bool vec = ld % 4 == 0 && (uintptr_t)out % (4 * sizeof(TOut)) == 0 && (uintptr_t)residual % 16 == 0;
-    const int n = n0 + lane * 4;
+    const int n = lane * 4 < BN ? n0 + lane * 4 : N;
     float b4[4], ws[4];
     unsigned odd_w = 0;               // the lanes with a column that could not be split
 #pragma unroll
@@ -315,7 +333,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     for (int i = warp - 2; i < BM; i += EPI) {
       const int m = m0 + i;
       if (m >= M) break;
-      const float4 t = *reinterpret_cast<const float4*>(tile_s + (size_t)i * OLD + lane * 4);
+      const float4 t = *reinterpret_cast<const float4*>(tile_s + (size_t)i * OLD + (lane * 4 < BN ? lane * 4 : 0));
       const float xs = x_scale[m];
       float y[4] = {t.x * xs * ws[0], t.y * xs * ws[1], t.z * xs * ws[2], t.w * xs * ws[3]}, r[4] = {0.0f, 0.0f, 0.0f, 0.0f};
       // what could not be split, four columns at a time with the warp's lanes along K (1024x768x768 us:
@@ -410,6 +428,7 @@ long long align256(long long n) { return (n + 255) & ~255LL; }
 constexpr long long PIECES_MAX = 96LL << 20;
 struct Cut { int rows, cols; };
 Cut cut_of(int M, int N, int K) {
+  constexpr int BN = 128;
   const long long sms = nb_device_sms(), tm = (M + BM - 1) / BM, tn = (N + BN - 1) / BN;
   const long long most = PIECES_MAX / (6LL * K * BM) > 1 ? PIECES_MAX / (6LL * K * BM) : 1;
   const long long parts = (tm + most - 1) / most, rows = (tm + parts - 1) / parts;
@@ -427,6 +446,42 @@ Cut cut_of(int M, int N, int K) {
   return cut;
 }
 
+template <int BN, typename TOut>
+int launch_tiles(const float* X, const float* W, const bf16* xp, const bf16* wp, const float* x_scale, const float* w_scale,
+                 const float* bias, const float* residual, TOut* out, int ld, int M, int N, int K, int act,
+                 cudaStream_t stream) {
+  auto kern = gemm_f32_tc_kernel<BN, TOut>;
+  static bool configured = false;   // per instantiation
+  if (!configured) {
+    NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<BN>::SMEM));
+    configured = true;
+  }
+  CUtensorMap mx, mw;
+  int rc = make_map(&mx, xp, 3LL * M, K, BM, BK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2);
+  if (rc) return rc;
+  rc = make_map(&mw, wp, 3LL * N, K, BN, BK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2);
+  if (rc) return rc;
+  int run = 1;                      // blocks of a run: as many as there are runs
+  while (run * run < (K + BK - 1) / BK) ++run;
+  int* w = nb_error_words();
+  const int tiles_n = (N + BN - 1) / BN;
+  NB_CUDA(nb_launch(kern, dim3((unsigned)(tiles_n * ((M + BM - 1) / BM))), dim3(Tile<BN>::THREADS),
+                    (size_t)Tile<BN>::SMEM, stream, mx, mw, X, W, x_scale, w_scale, bias, residual, out, ld, M, N, K,
+                    act, tiles_n, run, w ? w + NB_ERRW_GEMM_F32_TC : nullptr));
+  return 0;
+}
+
+// Columns of a tile: the width with the least waves of tiles x time of a block of K in it.
+int g_force_bn = 0;
+double block_us(int bn) { return bn == 96 ? 1.15 : 1.4; }
+double waves(long long M, long long N, int bn) {
+  return ceil((double)((M + BM - 1) / BM) * (double)((N + bn - 1) / bn) / nb_device_sms());
+}
+int tile_width(int M, int N) {
+  if (g_force_bn) return g_force_bn;
+  return waves(M, N, 96) * block_us(96) < waves(M, N, 128) * block_us(128) ? 96 : 128;
+}
+
 template <typename TOut>
 int launch(const float* X, const float* W, const float* bias, const float* residual, void* out, int M,
            int N, int K, int act, unsigned char* scratch, cudaStream_t stream) {
@@ -435,36 +490,27 @@ int launch(const float* X, const float* W, const float* bias, const float* resid
   bf16* wp = (bf16*)(scratch + align256(6LL * cut.rows * K));
   float* x_scale = (float*)(scratch + align256(6LL * cut.rows * K) + align256(6LL * cut.cols * K));
   float* w_scale = x_scale + cut.rows;
-  auto kern = gemm_f32_tc_kernel<TOut>;
-  static bool configured = false;   // per instantiation
-  if (!configured) {
-    NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-    configured = true;
-  }
-  int run = 1;                      // blocks of a run: as many as there are runs
-  while (run * run < (K + BK - 1) / BK) ++run;
-  int* w = nb_error_words();
   for (int n0 = 0; n0 < N; n0 += cut.cols) {
     const int nc = N - n0 < cut.cols ? N - n0 : cut.cols;
     for (int m0 = 0; m0 < M; m0 += cut.rows) {
       const int mc = M - m0 < cut.rows ? M - m0 : cut.rows;
-      CUtensorMap mx, mw;
-      int rc = make_map(&mx, xp, 3LL * mc, K, BM, BK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2);
-      if (rc) return rc;
-      rc = make_map(&mw, wp, 3LL * nc, K, BN, BK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2);
-      if (rc) return rc;
       const float* Xc = X + (size_t)m0 * K;
       const float* Wc = W + (size_t)n0 * K;
       const size_t o = (size_t)m0 * N + n0;
       // (pieces that the launch before made are there still)
       const int xs = n0 == 0 || cut.rows < M ? mc : 0, ws = m0 == 0 ? nc : 0;
-      NB_CUDA(nb_launch(split_kernel, dim3((unsigned)((xs + ws + 7) / 8)), dim3(256), 0, stream, Xc, Wc, xp, wp,
-                        x_scale, w_scale, xs, ws, K));
-      const int tiles_n = (nc + BN - 1) / BN;
-      NB_CUDA(nb_launch(kern, dim3((unsigned)(tiles_n * ((mc + BM - 1) / BM))), dim3(THREADS), (size_t)SMEM, stream,
-                        mx, mw, Xc, Wc, x_scale, w_scale, bias == nullptr ? nullptr : bias + n0,
-                        residual == nullptr ? nullptr : residual + o, (TOut*)out + o, N, mc, nc, K, act, tiles_n,
-                        run, w ? w + NB_ERRW_GEMM_F32_TC : nullptr));
+      if (K <= 4 * 32 * HELD)         // a warp holds the row
+        NB_CUDA(nb_launch(split_kernel<1>, dim3((unsigned)((xs + ws + 7) / 8)), dim3(256), 0, stream, Xc, Wc, xp, wp,
+                          x_scale, w_scale, xs, ws, K));
+      else
+        NB_CUDA(nb_launch(split_kernel<4>, dim3((unsigned)((xs + ws + 1) / 2)), dim3(256), 0, stream, Xc, Wc, xp, wp,
+                          x_scale, w_scale, xs, ws, K));
+      const float* bc = bias == nullptr ? nullptr : bias + n0;
+      const float* rc = residual == nullptr ? nullptr : residual + o;
+      const int e = tile_width(mc, nc) == 96
+                        ? launch_tiles<96>(Xc, Wc, xp, wp, x_scale, w_scale, bc, rc, (TOut*)out + o, N, mc, nc, K, act, stream)
+                        : launch_tiles<128>(Xc, Wc, xp, wp, x_scale, w_scale, bc, rc, (TOut*)out + o, N, mc, nc, K, act, stream);
+      if (e) return e;
     }
   }
   return 0;
@@ -491,8 +537,8 @@ NB_EXPORT int nb_gemm_f32_tc_supported(int M, int N, int K) {
 NB_EXPORT int nb_gemm_f32_tc_preferred(int M, int N, int K) {
   if (!nb_gemm_f32_tc_supported(M, N, K) || M < 65 || K < 128) return 0;
   const double sms = nb_device_sms(), blocks = (K + BK - 1) / BK;
-  const double tiles = (double)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  const double here = ceil(tiles / sms) * (7.0 + blocks * 1.65) + ((double)M + N) * K * 10.0 / 4e6;
+  const int bn = tile_width(M, N);
+  const double here = waves(M, N, bn) * (7.0 + blocks * block_us(bn)) + ((double)M + N) * K * 10.0 / 4e6;
   const int cut = nb_gemm_f32_cut(M, N, K);
   const double small = (double)((M + 63) / 64) * ((N + 63) / 64) / sms;            // 64 x 64 tiles an SM
   if (cut == 0) return here < 4.0 + 0.045 * K * (small > 0.87 ? 1.15 * small : 1.0) ? 1 : 0;
@@ -512,6 +558,13 @@ NB_EXPORT void nb_gemm_f32_tc_cut(int M, int N, int K, int* out2) {
   const Cut cut = cut_of(M, N, K);
   out2[0] = cut.rows;
   out2[1] = cut.cols;
+}
+
+// Tuning and tests: columns of a tile (96, 128; 0 = choose).
+NB_EXPORT int nb_gemm_f32_tc_force(int columns) {
+  NB_REQUIRE(columns == 0 || columns == 96 || columns == 128, NB_ERR_BAD_ARG, "gemm_f32_tc: no tile of %d columns", columns);
+  g_force_bn = columns;
+  return 0;
 }
 
 NB_EXPORT int nb_gemm_f32_tc_set_wait_budget(long long cycles) { return set_wait_budget(cycles); }
