@@ -14,17 +14,17 @@
 //   * K is cut among the CTAs of a thread-block cluster (1 to 8), chosen so that the launch
 //     fills the GPU once: each CTA walks over its run of 64-column blocks of K into its own
 //     accumulator;
-//   * the sums meet by a reduce-scatter through distributed shared memory: the rows of X are
-//     dealt out to the CTAs of the cluster (in fours), every CTA sends each other CTA that
-//     CTA's rows of its accumulator with `st.async` (16 bytes a store, counted on a barrier in
-//     the receiver's shared memory, so no cluster barrier stands between sending and adding
-//     up), and each adds up what it got in rank order (the result does not depend on timing),
-//     applies bias, activation and residual and stores its rows: 32 lanes write 32
-//     consecutive columns of a row.
-// Warp 0: one thread issues the TMA loads (128 x 64 boxes of W, rows x 64 boxes of X, 128-byte
-// swizzled) into a ring of stages; the weights of the first stages are asked for before the
-// wait on the kernel in front (they are constants).  Warp 1 owns the tensor memory and issues
-// the MMAs.  Warps 2 to 5 are the epilogue, one per quarter of the lanes.
+//   * the sums meet through distributed shared memory: every CTA turns its accumulator over into
+//     its own shared memory (over the ring, which is free by then) as rows of X x 128 columns; behind a
+//     cluster barrier each CTA takes its share of the rows from all of them, 512 consecutive bytes a
+//     warp, adds in rank order (the result does not depend on timing), applies bias,
+//     activation and residual and stores 16 bytes a thread.  (Sent out instead with `st.async`, 16
+//     bytes a store, the exchange went at 8 bytes a clock and SM: SLOW_FIGURES)
+// Warp 0 issues the TMA loads (128 x 64 boxes of W, rows x 64 boxes of X, 128-byte
+// swizzled) into a ring of stages of 104 KB at most, so that a CTA of the next launch fits beside it; the
+// weights of the first stages are asked for before the wait on the kernel in front (they are
+// constants).  Warp 1 owns the tensor memory and issues the MMAs.  Warps 2 to 9 are the epilogue, two per
+// quarter of the lanes.
 //
 // Every wait on an mbarrier is bounded by a clock budget; a wait that runs out raises the
 // kernel's error word, all roles leave their loops, every thread still passes the cluster's
@@ -46,8 +46,10 @@ constexpr int MAX_ROWS = 128;
 constexpr int MAX_STAGES = 8;
 constexpr int MAX_SPLIT = 8;         // portable cluster size
 constexpr int W_BYTES = BW * BK * 2;                 // 16 KB
-constexpr int THREADS = 64 + 4 * 32;
-constexpr int SMEM_BUDGET = 200 * 1024;
+constexpr int EPI_WARPS = 8;
+constexpr int THREADS = 64 + EPI_WARPS * 32;
+constexpr int SMEM_BUDGET = 104 * 1024;
+constexpr int AHEAD = 2;             // pieces of the residual a thread asks for ahead
 
 struct RowsShape {
   int nb;            // rows of X rounded up to 16: the MMA's N
@@ -57,62 +59,35 @@ struct RowsShape {
   int stage_bytes;   // W box + X box
   int x_bytes;       // X box
   int chunk;         // rows of X a CTA finishes (a multiple of 4)
-  int cpad;          // floats between two weight rows in the receive buffer (cpad / 4 is odd)
+  int body;          // bytes of the ring, and of the sums that take its place
   int tmem_cols;     // power of two >= nb, >= 32
   int smem;          // dynamic shared memory
 };
 
-// Four rows of the residual at column n (zero where there is none).
-__device__ __forceinline__ void load_residual4(float (&r)[4], const float* residual, int m0, int m_end,
-                                               int n, int N) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-    r[j] = (residual && m0 + j < m_end) ? residual[(size_t)(m0 + j) * N + n] : 0.0f;
-}
-
-__device__ __forceinline__ void st_async_v4(uint32_t remote, uint32_t remote_bar, const uint32_t* v) {
-  asm volatile(
-      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1,%2,%3,%4}, [%5];\n" ::"r"(remote),
-      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(remote_bar)
-      : "memory");
-}
-
-// One row of the result: bias, activation, residual, store.
-template <typename TOut>
-__device__ __forceinline__ void finish_rows4(const float (&a)[4], const float (&r)[4], int m0, int m_end,
-                                             int n, int N, float b, int act, TOut* out) {
-  float f[4] = {a[0] + b, a[1] + b, a[2] + b, a[3] + b};
-  nb_apply_act_fast_all(f, act);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    if (m0 + j >= m_end) break;
-    const float y = f[j] + r[j];
-    if constexpr (sizeof(TOut) == 4) reinterpret_cast<float*>(out)[(size_t)(m0 + j) * N + n] = y;
-    else reinterpret_cast<bf16*>(out)[(size_t)(m0 + j) * N + n] = __float2bfloat16_rn(y);
-  }
+__device__ __forceinline__ float4 ld_cluster4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];\n"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
 }
 
 template <typename TOut>
 __global__ void __launch_bounds__(THREADS)
 gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                     const float* __restrict__ bias, const float* residual, TOut* out, int M, int N,
-                    int K, int act, RowsShape sh, int* err_word) {
+                    int K, int act, RowsShape sh, bool vec, int* err_word) {
   extern __shared__ unsigned char smem_dyn[];
   const uint32_t raw = smem_u32(smem_dyn);
   const uint32_t base = (raw + 1023u) & ~1023u;          // swizzle atoms want 1024-byte alignment
   unsigned char* gen = smem_dyn + (base - raw);
-  // [ring of stages] [what the other CTAs send: [rank][128 weight rows][cpad]] [barriers]
-  // [tmem slot, abort]
-  const uint32_t ring_bytes = (uint32_t)(sh.stages * sh.stage_bytes);
-  const uint32_t recv = base + ring_bytes;
-  const uint32_t recv_bytes = sh.split > 1 ? (uint32_t)(sh.split * BW * sh.cpad * 4) : 0u;
-  const uint32_t bars = recv + recv_bytes;
+  // [ring of stages, then sums: [row of X][128 weight rows]] [barriers] [tmem slot, abort]
+  const uint32_t bars = base + (uint32_t)sh.body;
   auto full_bar = [&](int s) { return bars + 8u * s; };
   auto empty_bar = [&](int s) { return bars + 8u * (MAX_STAGES + s); };
   const uint32_t acc_full = bars + 8u * (2 * MAX_STAGES);
-  const uint32_t recv_bar = bars + 8u * (2 * MAX_STAGES + 1);
-  uint32_t* tmem_slot =
-      reinterpret_cast<uint32_t*>(gen + ring_bytes + recv_bytes + (2 * MAX_STAGES + 2) * 8);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + sh.body + (2 * MAX_STAGES + 2) * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -131,7 +106,6 @@ gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       mbar_init(empty_bar(s), 1);
     }
     mbar_init(acc_full, 1);
-    mbar_init(recv_bar, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -159,17 +133,23 @@ gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     }
   }
   nb_grid_dependency_wait();
-  // Rows of X this CTA finishes, and the bytes the other CTAs will send for them.
-  const int m_lo = (int)rank * sh.chunk;
-  const int my_rows = max(0, min(sh.nb, m_lo + sh.chunk) - m_lo);
-  if (tid == 0 && sh.split > 1)
-    mbar_expect_tx(recv_bar, (uint32_t)((sh.split - 1) * BW * my_rows * 4));
-  // Every CTA of the cluster says that it runs and that its barrier is armed; the matching
-  // wait stands in front of the first store into another CTA's shared memory, by when the
-  // others have long arrived.  (The arrive stands behind the wait on the predecessor: see
-  // the decode attention.)
-  __syncwarp();
-  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+  // the rows this CTA finishes; a thread of the epilogue takes four columns, the same in every row
+  const int m_lo = (int)rank * sh.chunk, m_hi = min(M, m_lo + sh.chunk);
+  const int row_first = m_lo + (warp - 2), n = n0 + lane * 4;
+  float4 ahead[AHEAD];
+  float b4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  if (warp >= 2) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (bias != nullptr && n + j < N) b4[j] = __ldg(bias + n + j);
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) {
+      const int m = row_first + i * EPI_WARPS;
+      ahead[i] = (vec && residual != nullptr && m < m_hi && n < N)
+                     ? *reinterpret_cast<const float4*>(residual + (size_t)m * N + n)
+                     : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+  }
 
   if (warp == 0) {
     // A TMA tile load costs its issuing thread about 190 clocks whatever the size of its box:
@@ -178,7 +158,8 @@ gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     // its own earlier wait for it: it can never be two rounds of the ring ahead of the MMAs
     // (where the parity of an older phase of the stage's barrier would pass for the awaited one).
     pre_kb = __shfl_sync(0xffffffffu, pre_kb, 0);
-    const int producers = sh.stages % 4 == 0 ? 4 : (sh.stages % 3 == 0 ? 3 : (sh.stages % 2 == 0 ? 2 : 1));
+    const int producers = n_kb <= sh.stages ? 4      // no stage is filled twice
+                          : sh.stages % 4 == 0 ? 4 : (sh.stages % 3 == 0 ? 3 : (sh.stages % 2 == 0 ? 2 : 1));
     if (lane < producers) {   // --------------------------------------------- TMA producers
       for (int i = lane; i < n_kb; i += producers) {
         const int s = i % sh.stages;
@@ -219,114 +200,79 @@ gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     }
   }
 
-  // ---- epilogue warps: this CTA's sums are complete
-  const int quarter = warp & 3;                 // the 32 tensor-memory lanes this warp may read
-  const int n_local = quarter * 32 + lane;      // weight row of the tile = column of the output
-  const int n = n0 + n_local;
-  const int m_end = min(M, sh.nb);
-  // the bias of this thread's column (a constant), fetched while the products run
-  const float b = (warp >= 2 && bias && n < N) ? __ldg(bias + n) : 0.0f;
-  bool ready = true;
-  if (warp >= 2)
-    ready = __shfl_sync(0xffffffffu, (int)mbar_wait(acc_full, 0u, abort_flag), 0) != 0;
-  // the lanes of the producer's and the issuer's warps come together first: the barrier wants
-  // whole warps
-  __syncwarp();
-  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-
-  if (warp >= 2 && ready) {
+  // ---- epilogue warps: this CTA's sums are complete (and the ring free)
+  float* sums = reinterpret_cast<float*>(gen);
+  if (warp >= 2 && __shfl_sync(0xffffffffu, (int)mbar_wait(acc_full, 0u, abort_flag), 0) != 0) {
     tc05_fence_after();
-    // columns of the accumulator = rows of X, in fours; four that belong to CTA d go to
-    // [this rank][n_local][their place in d's rows] of d's buffer, the own ones stay here
-    const uint32_t slot = recv + (uint32_t)(((int)rank * BW + n_local) * sh.cpad) * 4u;
-    for (int c0 = 0; c0 < sh.nb; c0 += 32) {
+    const int quarter = warp & 3;                 // the 32 tensor-memory lanes this warp may read
+    float* column = sums + quarter * 32 + lane;   // its weight row's sums, one a row of X
+    for (int c0 = (warp - 2) / 4 * 32; c0 < sh.nb; c0 += 64) {
       uint32_t v[32];
-      if (n_kb > 0) {
-        tc05_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, v);
-        tc05_wait_ld();
-      } else {
+      tc05_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, v);
+      tc05_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = 0u;
-      }
-      if (sh.split == 1) {   // nothing to exchange: finish the rows right away
-        if (n < N) {
-          // all of the chunk's residual before its first store: it may be `out` itself, and a
-          // load behind a store would wait for it
-          float res[8][4];
-#pragma unroll
-          for (int g4 = 0; g4 < 8; ++g4) load_residual4(res[g4], residual, c0 + 4 * g4, m_end, n, N);
-#pragma unroll
-          for (int g4 = 0; g4 < 8; ++g4) {
-            if (c0 + 4 * g4 >= m_end) break;
-            const float a[4] = {__uint_as_float(v[4 * g4]), __uint_as_float(v[4 * g4 + 1]),
-                                __uint_as_float(v[4 * g4 + 2]), __uint_as_float(v[4 * g4 + 3])};
-            finish_rows4<TOut>(a, res[g4], c0 + 4 * g4, m_end, n, N, b, act, out);
-          }
-        }
-        continue;
-      }
-#pragma unroll
-      for (int g4 = 0; g4 < 8; ++g4) {
-        const int m = c0 + 4 * g4;
-        if (m >= sh.nb) break;
-        const int dest = m / sh.chunk;
-        const uint32_t at = slot + (uint32_t)(m - dest * sh.chunk) * 4u;
-        if (dest == (int)rank) {
-          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(at), "r"(v[4 * g4]), "r"(v[4 * g4 + 1]),
-                       "r"(v[4 * g4 + 2]), "r"(v[4 * g4 + 3])
-                       : "memory");
-        } else {
-          st_async_v4(cluster_addr(at, (uint32_t)dest), cluster_addr(recv_bar, (uint32_t)dest), &v[4 * g4]);
-        }
-      }
+      for (int j = 0; j < 32; ++j)
+        if (c0 + j < sh.nb) column[(c0 + j) * BW] = __uint_as_float(v[j]);
     }
     tc05_fence_before();
   }
-  // Second phase of the cluster's barrier: this thread has sent what it had to send (the wait
-  // is the last thing the kernel does: no CTA leaves while another may still send to it).
   __syncwarp();
-  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-  if (warp >= 2 && ready) {
-    if (sh.split > 1) {
-      // the residual of this CTA's first rows is fetched while the others' sums are on their way
-      constexpr int PRE = 4;
-      float res[PRE][4];
+  if (sh.split > 1)
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  else
+    __syncthreads();
+  if (warp >= 2 && *abort_flag == 0) {
+    int i = 0;
+#pragma unroll 2
+    for (int m = row_first; m < m_hi; m += EPI_WARPS, ++i) {
+      const uint32_t at = base + (uint32_t)((m * BW + lane * 4) * 4);
+      float y[4] = {0.0f, 0.0f, 0.0f, 0.0f}, r[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      float4 part[MAX_SPLIT];
 #pragma unroll
-      for (int g4 = 0; g4 < PRE; ++g4) {
+      for (int q = 0; q < MAX_SPLIT; ++q)           // all asked for before the first is used
+        if (q < sh.split) part[q] = ld_cluster4(cluster_addr(at, (uint32_t)q));
 #pragma unroll
-        for (int j = 0; j < 4; ++j) res[g4][j] = 0.0f;
-        if (n < N && 4 * g4 < my_rows) load_residual4(res[g4], residual, m_lo + 4 * g4, m_end, n, N);
+      for (int q = 0; q < MAX_SPLIT; ++q) {
+        if (q >= sh.split) break;
+        y[0] += part[q].x; y[1] += part[q].y; y[2] += part[q].z; y[3] += part[q].w;
       }
-      // what the others sent for this CTA's rows has arrived when the barrier has its bytes
-      const bool got = __shfl_sync(0xffffffffu, (int)mbar_wait(recv_bar, 0u, abort_flag), 0) != 0;
-      if (got && n < N) {
-        for (int off0 = 0; off0 < my_rows; off0 += 4 * PRE) {
-          if (off0 > 0) {   // further rows: their residual now, all of it before the next stores
+      if (n >= N) continue;
+      const size_t o = (size_t)m * N + n;
+      if (residual != nullptr) {
+        if (vec) {
+          const float4 q = i == 0 ? ahead[0] : i == 1 ? ahead[1] : *reinterpret_cast<const float4*>(residual + o);
+          r[0] = q.x; r[1] = q.y; r[2] = q.z; r[3] = q.w;
+        } else {
 #pragma unroll
-            for (int g4 = 0; g4 < PRE; ++g4)
-              if (off0 + 4 * g4 < my_rows) load_residual4(res[g4], residual, m_lo + off0 + 4 * g4, m_end, n, N);
-          }
-#pragma unroll
-          for (int g4 = 0; g4 < PRE; ++g4) {
-            const int off = off0 + 4 * g4;
-            if (off >= my_rows || m_lo + off >= m_end) break;
-            float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            for (int s = 0; s < sh.split; ++s) {   // in rank order
-              float4 x;
-              asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];\n"
-                           : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
-                           : "r"(recv + (uint32_t)((s * BW + n_local) * sh.cpad + off) * 4u));
-              a[0] += x.x; a[1] += x.y; a[2] += x.z; a[3] += x.w;
-            }
-            finish_rows4<TOut>(a, res[g4], m_lo + off, m_end, n, N, b, act, out);
-          }
+          for (int j = 0; j < 4; ++j)
+            if (n + j < N) r[j] = residual[o + j];
         }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) y[j] += b4[j];
+      nb_apply_act_fast_all(y, act);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) y[j] += r[j];
+      if (vec) {
+        if constexpr (sizeof(TOut) == 4) {
+          *reinterpret_cast<float4*>(out + o) = make_float4(y[0], y[1], y[2], y[3]);
+        } else {
+          uint2 u;
+          __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
+          h[0] = __floats2bfloat162_rn(y[0], y[1]);
+          h[1] = __floats2bfloat162_rn(y[2], y[3]);
+          *reinterpret_cast<uint2*>(out + o) = u;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (n + j < N) out[o + j] = nb_from_f32<TOut>(y[j]);
       }
     }
   }
-
   __syncwarp();
-  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  if (sh.split > 1)       // nobody leaves while another reads its shared memory
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
   tc05_fence_before();
   __syncthreads();
   if (*abort_flag) {
@@ -377,7 +323,7 @@ bool plan_rows(int M, int N, int K, RowsShape* out) {
     const int kb_per = (num_kb + split - 1) / split;
     if (split > 1 && (split - 1) * kb_per >= num_kb) continue;   // a CTA without a K block
     const long long mma = (long long)kb_per * (BK / UMMA_K) * 85;
-    const long long load = (long long)kb_per * s.stage_bytes / 64;
+    const long long load = (long long)kb_per * s.stage_bytes / 55;
     const long long cost = (mma > load ? mma : load) + (split > 1 ? 600 : 0) + 40LL * split;
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = split; }
   }
@@ -385,12 +331,13 @@ bool plan_rows(int M, int N, int K, RowsShape* out) {
   s.split = best;
   s.kb_per = (num_kb + best - 1) / best;
   s.chunk = ((s.nb + best - 1) / best + 3) / 4 * 4;
-  s.cpad = (s.chunk / 4) % 2 == 1 ? s.chunk : s.chunk + 4;   // an odd number of 16-byte units: no bank conflicts
-  const int recv = best > 1 ? best * BW * s.cpad * 4 : 0;
   int stages = s.kb_per < MAX_STAGES ? s.kb_per : MAX_STAGES;
-  while (stages > 1 && stages * s.stage_bytes + recv > SMEM_BUDGET) --stages;
+  while (stages > 1 && stages * s.stage_bytes > SMEM_BUDGET) --stages;
+  if (stages < s.kb_per && (stages == 5 || stages == 7)) --stages;     // four or three lanes bring them in
   s.stages = stages;
-  s.smem = stages * s.stage_bytes + recv + (2 * MAX_STAGES + 2) * 8 + 16 + 1024;
+  const int sums = s.nb * BW * 4;
+  s.body = stages * s.stage_bytes > sums ? stages * s.stage_bytes : sums;
+  s.smem = s.body + (2 * MAX_STAGES + 2) * 8 + 16 + 1024;
   if (s.smem > 227 * 1024) return false;
   *out = s;
   return true;
@@ -411,8 +358,9 @@ int launch_rows(const void* X, const void* W, const float* bias, const float* re
     configured = true;
   }
   const int tiles_n = (N + BW - 1) / BW;
+  const bool vec = N % 4 == 0 && (uintptr_t)out % (4 * sizeof(TOut)) == 0 && (uintptr_t)residual % 16 == 0;
   NB_CUDA(nb_launch_clusters(kern, dim3(tiles_n * sh.split), dim3(THREADS), (size_t)sh.smem, stream,
-                             sh.split, mx, mw, bias, residual, (TOut*)out, M, N, K, act, sh,
+                             sh.split, mx, mw, bias, residual, (TOut*)out, M, N, K, act, sh, vec,
                              error_word()));
   return 0;
 }
