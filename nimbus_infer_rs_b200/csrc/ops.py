@@ -1502,11 +1502,29 @@ class CudaBackend:
 
     def advance_decode(self, tokens, next_tokens, row_pos, row_slot):
         """tokens <- next_tokens, row_pos += 1 for live rows (between two decode steps)."""
+        self.hand_over_decode(tokens, next_tokens, row_pos, row_slot, None)
+
+    def hand_over_decode(self, tokens, next_tokens, row_pos, row_slot, host):
+        """:meth:`advance_decode`, with pinned host memory that takes ``next_tokens`` as well."""
         for t, n in ((tokens, "tokens"), (next_tokens, "next"), (row_pos, "row_pos"),
                      (row_slot, "row_slot")):
             _check(t, n, torch.int32, 1)
+        if host is not None and not (host.is_pinned() and host.dtype == torch.int32 and host.is_contiguous()
+                                     and host.numel() >= tokens.numel()):
+            raise KernelError("hand_over_decode: the host's tokens go to pinned int32 memory")
         self._call("nb_advance_decode", _ptr(tokens), _ptr(next_tokens), _ptr(row_pos),
-                   _ptr(row_slot), (tokens.numel()), self._stream())
+                   _ptr(row_slot), _ptr(host), (tokens.numel()), self._stream())
+
+    def take_tokens(self, tokens, ring, count):
+        """``tokens`` <- the next entry of ``ring`` (pinned int32 ``[turns, 1 + n]``; ``count``, an int on
+        the device, says which and moves on), unless the entry's first number is 0."""
+        _check(tokens, "tokens", torch.int32, 1)
+        _check(count, "count", torch.int32, 1)
+        if not (ring.is_pinned() and ring.dtype == torch.int32 and ring.is_contiguous() and ring.dim() == 2
+                and ring.shape[1] == tokens.numel() + 1):
+            raise KernelError("take_tokens: the ring is pinned int32 memory, an entry 1 + n numbers")
+        self._call("nb_take_tokens", _ptr(tokens), _ptr(ring), _ptr(count), ring.shape[0], tokens.numel(),
+                   self._stream())
 
     # -- sampling ---------------------------------------------------------------------
     def argmax(self, logits, out):

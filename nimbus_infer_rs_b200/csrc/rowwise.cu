@@ -1149,15 +1149,18 @@ NB_EXPORT int nb_kv_append(const void* src, int dtype, int src_stride, int k_col
 
 // ---------------------------------------------------------------------------------
 // Between two decode steps on the device: the sampled token becomes the next input and the
-// position of every live row moves on by one.  Rows with a negative slot are padding.
+// position of every live row moves on by one.  Rows with a negative slot are padding.  `host` (or
+// null): pinned host memory that takes the sampled tokens as well, so that reading them is a wait for
+// the stream and no copy behind it.
 // ---------------------------------------------------------------------------------
 __global__ void advance_decode_kernel(int* tokens, const int* next,
                                       int* row_pos, const int* row_slot,
-                                      int n) {
+                                      int* host, int n) {
   nb_grid_dependency_wait();
   nb_launch_dependents();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
+  if (host != nullptr) host[i] = next[i];
   if (row_slot[i] >= 0) {
     tokens[i] = next[i];
     row_pos[i] += 1;
@@ -1167,10 +1170,37 @@ __global__ void advance_decode_kernel(int* tokens, const int* next,
 }
 
 NB_EXPORT int nb_advance_decode(int* tokens, const int* next, int* row_pos, const int* row_slot,
-                                int n, cudaStream_t stream) {
+                                int* host, int n, cudaStream_t stream) {
   if (n == 0) return 0;
   NB_CUDA(nb_launch(advance_decode_kernel, dim3((n + 127) / 128), dim3(128), 0, stream, tokens, next,
-                    row_pos, row_slot, n));
+                    row_pos, row_slot, host, n));
   NB_CHECK_LAUNCH("advance_decode");
+  return 0;
+}
+
+// The tokens of a decode step from the host: `ring` is pinned host memory, `turns` entries of 1 + n
+// numbers, taken in turn (`count`, on the device, says which is next and is moved on); an entry whose
+// first number is 0 leaves the tokens as they lie on the device.  A kernel and not a copy, so that it can
+// be recorded with the step it belongs to while the host is turns ahead.
+__global__ void __launch_bounds__(256)
+take_tokens_kernel(int* tokens, const volatile int* ring, int* count, int turns, int n) {
+  nb_grid_dependency_wait();
+  nb_launch_dependents();
+  const int c = *count;
+  const volatile int* entry = ring + (size_t)(c % turns) * (n + 1);
+  const int given = entry[0];
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const int t = entry[1 + i];          // asked for beside `given`, not behind it
+    if (given != 0) tokens[i] = t;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) *count = c + 1 == turns ? 0 : c + 1;
+}
+
+NB_EXPORT int nb_take_tokens(int* tokens, const int* ring, int* count, int turns, int n, cudaStream_t stream) {
+  if (n == 0) return 0;
+  NB_REQUIRE(turns >= 1, NB_ERR_BAD_ARG, "take_tokens: a ring has entries");
+  NB_CUDA(nb_launch(take_tokens_kernel, dim3(1), dim3(256), 0, stream, tokens, ring, count, turns, n));
+  NB_CHECK_LAUNCH("take_tokens");
   return 0;
 }
