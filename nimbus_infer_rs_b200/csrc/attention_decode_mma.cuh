@@ -47,7 +47,7 @@ __device__ __forceinline__ uint32_t pack2_bf16(float lo, float hi) {
 }
 
 // MMA_STAGES: pages (keys and values) in flight per CTA; NW: warps.  Four warps share a page
-// (16 keys each).  A page costs a warp about 1,400 clocks of dependent steps (loads from
+// (16 keys each), two have 32 keys each.  A page costs a warp about 1,400 clocks of dependent steps (loads from
 // shared memory, two rounds of tensor-core instructions with the softmax between them), so
 // when the CTAs of a launch fit on the GPU with four pages each, eight warps take two pages
 // at a time; a large batch has four warps and two pages per CTA, for more CTAs per SM.
@@ -68,8 +68,9 @@ attention_decode_mma_kernel(const __nv_bfloat16* q, int q_stride, int q_col,
   constexpr int KS = HD / 16;          // k-steps of the score product = row tiles of the value product
   constexpr int GH = 8;                // query heads an MMA column block holds
   constexpr int NT = NW * 32;          // threads
-  constexpr int PPI = NW / 4;          // pages per turn of the loop
-  static_assert((NW == 4 || NW == 8) && MMA_STAGES % PPI == 0, "four or eight warps");
+  constexpr int PPI = NW > 4 ? NW / 4 : 1;   // pages per turn of the loop
+  constexpr int QPW = NW < 4 ? 4 / NW : 1;   // quarters of a page a warp takes
+  static_assert((NW == 1 || NW == 2 || NW == 4 || NW == 8) && MMA_STAGES % PPI == 0, "one to eight warps");
   const int dk = MIXED ? kv.head_dim : HD, dv = MIXED ? kv.value_dim : HD;
   const int KTILE = PAGE_TOKENS * dk, VTILE = PAGE_TOKENS * dv;    // elements of one page of one head
   constexpr int STILE = PAGE_TOKENS * ROW;
@@ -97,7 +98,7 @@ attention_decode_mma_kernel(const __nv_bfloat16* q, int q_stride, int q_col,
   const int split = blockIdx.x, kvh = blockIdx.y, r = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int wq = warp & 3, po = warp >> 2;   // quarter of a page, page of a turn
+  const int wq = NW < 4 ? warp * QPW : warp & 3, po = NW < 4 ? 0 : warp >> 2;   // (first) quarter of a page, page of a turn
   const int n_heads = kv.n_kv_heads * group;
   const int slot = row_slot[r];
   if (slot < 0) {   // padding row: zeros, written by split 0
@@ -118,7 +119,13 @@ attention_decode_mma_kernel(const __nv_bfloat16* q, int q_stride, int q_col,
   // with kept first tokens the last split is theirs: the pages before the window's first that
   // hold some of them (none when the window still reaches back to them)
   const int run_splits = opt.keeps() ? n_splits - 1 : n_splits;
-  const int per_split = (n_pages + run_splits - 1) / run_splits;
+  const int per_split = max((n_pages + run_splits - 1) / run_splits, PPI);
+  // a short sequence is one split's: that one finishes it, and the cluster does not meet
+  const bool alone = n_splits == 1 || (clustered && !opt.keeps() && n_pages <= per_split);
+  if (alone && split > 0) {
+    nb_grid_dependency_wait();
+    return;
+  }
   const bool head_split = opt.keeps() && split == n_splits - 1;
   const int p_begin = head_split ? 0 : first_page + split * per_split;
   const int p_end = head_split ? min((keep_first + PAGE_TOKENS - 1) / PAGE_TOKENS, first_page)
@@ -174,7 +181,8 @@ attention_decode_mma_kernel(const __nv_bfloat16* q, int q_stride, int q_col,
   nb_grid_dependency_wait();
   // Every CTA of a cluster says that it runs (a padding row's CTAs have all left above); the
   // matching wait stands in front of the first store into another CTA's shared memory.
-  if constexpr (clustered) asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
+  if constexpr (clustered)
+    if (!alone) asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
 
   // Q^T as the B operand of the score product: column g of the block is query head g of the
   // group (zero beyond the group); this thread holds rows 2t, 2t+1 and 2t+8, 2t+9 of each k-step
@@ -254,40 +262,51 @@ attention_decode_mma_kernel(const __nv_bfloat16* q, int q_stride, int q_col,
     const int p = p0 + po;                            // this warp's page
     bf16* kt = tiles + (size_t)(stage + po) * 2 * STILE;
     bf16* vt = kt + STILE;
-    const int key0 = p * PAGE_TOKENS + wq * 16;       // first key of this warp's 16
-    if (p < p_end && key0 < kv_len && (key0 + 16 > j_begin || key0 < keep_first)) {   // warp-uniform: something to attend to
-      // the k-steps of the score product in accumulators of their own, added up afterwards:
-      // a tensor-core instruction takes long to hand its result to the next one
-      float sck[KS < 4 ? KS : 4][4];
+    const int key0 = p * PAGE_TOKENS + wq * 16;       // first key of this warp's 16 (or 32, 64)
+    if (p < p_end && key0 < kv_len && (key0 + QPW * 16 > j_begin || key0 < keep_first)) {   // warp-uniform: something to attend to
+      float sc[QPW][4];
 #pragma unroll
-      for (int i = 0; i < (KS < 4 ? KS : 4); ++i)
+      for (int qd = 0; qd < QPW; ++qd) {
+        // the k-steps of the score product in accumulators of their own, added up afterwards:
+        // a tensor-core instruction takes long to hand its result to the next one
+        constexpr int NA = QPW > 1 ? (KS < 2 ? KS : 2) : (KS < 4 ? KS : 4);
+        float sck[NA][4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) sck[i][j] = 0.0f;
+        for (int i = 0; i < NA; ++i)
 #pragma unroll
-      for (int ks = 0; ks < KS; ++ks) {
-        if (MIXED && ks * 16 >= dk) break;
-        uint32_t ka[4];
-        ldsm_x4(ka, kt + (wq * 16 + (lane & 15)) * ROW + ks * 16 + (lane >> 4) * 8);
-        mma_16816(sck[ks & 3], ka, qb[ks][0], qb[ks][1]);
+          for (int j = 0; j < 4; ++j) sck[i][j] = 0.0f;
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks) {
+          if (MIXED && ks * 16 >= dk) break;
+          uint32_t ka[4];
+          ldsm_x4(ka, kt + ((wq + qd) * 16 + (lane & 15)) * ROW + ks * 16 + (lane >> 4) * 8);
+          mma_16816(sck[ks % NA], ka, qb[ks][0], qb[ks][1]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float a = sck[0][j];
+#pragma unroll
+          for (int i = 1; i < NA; ++i) a += sck[i][j];
+          sc[qd][j] = a;
+        }
       }
-      float sc[4];
+      float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float a = sck[0][j];
+      for (int qd = 0; qd < QPW; ++qd) {
+        const int ja = key0 + qd * 16 + g, jb = ja + 8;
+        const bool va = (ja >= j_begin || ja < keep_first) && ja < kv_len,
+                   vb = (jb >= j_begin || jb < keep_first) && jb < kv_len;
+        if (softcap > 0.0f) {   // uniform: capped scores carry their scale already
 #pragma unroll
-        for (int i = 1; i < (KS < 4 ? KS : 4); ++i) a += sck[i][j];
-        sc[j] = a;
+          for (int j = 0; j < 4; ++j) sc[qd][j] = nb_softcap(sc[qd][j], cap_in, softcap);
+        }
+        sc[qd][0] = va ? sc[qd][0] * sl2 : -INFINITY;
+        sc[qd][1] = va ? sc[qd][1] * sl2 : -INFINITY;
+        sc[qd][2] = vb ? sc[qd][2] * sl2 : -INFINITY;
+        sc[qd][3] = vb ? sc[qd][3] * sl2 : -INFINITY;
+        mx0 = fmaxf(mx0, fmaxf(sc[qd][0], sc[qd][2]));
+        mx1 = fmaxf(mx1, fmaxf(sc[qd][1], sc[qd][3]));
       }
-      const int ja = key0 + g, jb = ja + 8;
-      const bool va = (ja >= j_begin || ja < keep_first) && ja < kv_len,
-                 vb = (jb >= j_begin || jb < keep_first) && jb < kv_len;
-      if (softcap > 0.0f) {   // uniform: capped scores carry their scale already
-#pragma unroll
-        for (int j = 0; j < 4; ++j) sc[j] = nb_softcap(sc[j], cap_in, softcap);
-      }
-      const float s0 = va ? sc[0] * sl2 : -INFINITY, s1 = va ? sc[1] * sl2 : -INFINITY;
-      const float s2 = vb ? sc[2] * sl2 : -INFINITY, s3 = vb ? sc[3] * sl2 : -INFINITY;
-      float mx0 = fmaxf(s0, s2), mx1 = fmaxf(s1, s3);
 #pragma unroll
       for (int off = 4; off < 32; off <<= 1) {
         mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, off));
@@ -298,31 +317,36 @@ attention_decode_mma_kernel(const __nv_bfloat16* q, int q_stride, int q_col,
       const float r1 = (m_run[1] == -INFINITY) ? 0.0f : nb_exp2(m_run[1] - mn1);
       m_run[0] = mn0;
       m_run[1] = mn1;
-      const float p0 = nb_exp2(s0 - mn0), p1 = nb_exp2(s1 - mn1);
-      const float p2 = nb_exp2(s2 - mn0), p3 = nb_exp2(s3 - mn1);
-      l_run[0] = l_run[0] * r0 + p0 + p2;
-      l_run[1] = l_run[1] * r1 + p1 + p3;
+      l_run[0] *= r0;
+      l_run[1] *= r1;
 #pragma unroll
       for (int i = 0; i < KS; ++i) {
         o[i][0] *= r0; o[i][1] *= r1; o[i][2] *= r0; o[i][3] *= r1;
       }
-      // P as the B operand of the value product: this thread needs keys 2t, 2t+1 (and +8) of
-      // head g; they sit in lanes (g' = 2t, t' = g/2) and (g' = 2t+1, t' = g/2)
-      const uint32_t pe = pack2_bf16(p0, p2);   // head 2t:   keys g, g+8
-      const uint32_t po = pack2_bf16(p1, p3);   // head 2t+1: keys g, g+8
-      const int src1 = (2 * t) * 4 + (g >> 1), src2 = src1 + 4;
-      const uint32_t e1 = __shfl_sync(0xffffffffu, pe, src1), o1 = __shfl_sync(0xffffffffu, po, src1);
-      const uint32_t e2 = __shfl_sync(0xffffffffu, pe, src2), o2 = __shfl_sync(0xffffffffu, po, src2);
-      const uint32_t x1 = (g & 1) ? o1 : e1, x2 = (g & 1) ? o2 : e2;
-      const uint32_t pb0 = __byte_perm(x1, x2, 0x5410);   // keys 2t, 2t+1
-      const uint32_t pb1 = __byte_perm(x1, x2, 0x7632);   // keys 2t+8, 2t+9
 #pragma unroll
-      for (int i = 0; i < KS; ++i) {
-        if (MIXED && i * 16 >= dv) break;
-        uint32_t va4[4];
-        ldsm_x4_trans(va4, vt + (wq * 16 + (lane & 7) + (lane >> 4) * 8) * ROW + i * 16 +
-                               ((lane >> 3) & 1) * 8);
-        mma_16816(o[i], va4, pb0, pb1);
+      for (int qd = 0; qd < QPW; ++qd) {
+        const float p0 = nb_exp2(sc[qd][0] - mn0), p1 = nb_exp2(sc[qd][1] - mn1);
+        const float p2 = nb_exp2(sc[qd][2] - mn0), p3 = nb_exp2(sc[qd][3] - mn1);
+        l_run[0] += p0 + p2;
+        l_run[1] += p1 + p3;
+        // P as the B operand of the value product: this thread needs keys 2t, 2t+1 (and +8) of
+        // head g; they sit in lanes (g' = 2t, t' = g/2) and (g' = 2t+1, t' = g/2)
+        const uint32_t pe = pack2_bf16(p0, p2);   // head 2t:   keys g, g+8
+        const uint32_t po = pack2_bf16(p1, p3);   // head 2t+1: keys g, g+8
+        const int src1 = (2 * t) * 4 + (g >> 1), src2 = src1 + 4;
+        const uint32_t e1 = __shfl_sync(0xffffffffu, pe, src1), o1 = __shfl_sync(0xffffffffu, po, src1);
+        const uint32_t e2 = __shfl_sync(0xffffffffu, pe, src2), o2 = __shfl_sync(0xffffffffu, po, src2);
+        const uint32_t x1 = (g & 1) ? o1 : e1, x2 = (g & 1) ? o2 : e2;
+        const uint32_t pb0 = __byte_perm(x1, x2, 0x5410);   // keys 2t, 2t+1
+        const uint32_t pb1 = __byte_perm(x1, x2, 0x7632);   // keys 2t+8, 2t+9
+#pragma unroll
+        for (int i = 0; i < KS; ++i) {
+          if (MIXED && i * 16 >= dv) break;
+          uint32_t va4[4];
+          ldsm_x4_trans(va4, vt + ((wq + qd) * 16 + (lane & 7) + (lane >> 4) * 8) * ROW + i * 16 +
+                                 ((lane >> 3) & 1) * 8);
+          mma_16816(o[i], va4, pb0, pb1);
+        }
       }
     }
     __syncthreads();   // the stages are free: the pages after the ones in flight go there
@@ -388,7 +412,7 @@ attention_decode_mma_kernel(const __nv_bfloat16* q, int q_stride, int q_col,
     }
   };
   unsigned c_remote = 0;    // this split's place in split 0's shared memory
-  if constexpr (clustered) {
+  if (clustered && !alone) {
     asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
     const unsigned local = (unsigned)__cvta_generic_to_shared(c_part + (size_t)split * group * (HD + 2));
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(c_remote) : "r"(local), "r"(0));
@@ -408,7 +432,7 @@ attention_decode_mma_kernel(const __nv_bfloat16* q, int q_stride, int q_col,
       l += f * w_ml[(w * GH + gh) * 2 + 1];
     }
     const int head = kvh * group + gh;
-    if (n_splits == 1) {
+    if (alone) {
       if (sink != nullptr) a *= nb_sink_fix(l, M, sink[head], true);
       a *= opt.gate_of(r, head);
       emit(gh, c, l > 0.0f ? a / l : a);
@@ -430,7 +454,7 @@ attention_decode_mma_kernel(const __nv_bfloat16* q, int q_stride, int q_col,
       part_ml[pi * 2 + 1] = l;
     }
   }
-  if (n_splits == 1) {
+  if (alone) {
     finish_maps();
     return;
   }
@@ -565,13 +589,25 @@ int launch_mma(const void* q, int q_stride, int q_col, const int* row_slot, cons
   const long long ctas = (long long)n_splits * kv.n_kv_heads * n_rows;
   long long per_sm = (long long)((228 * 1024) / (smem4 + 1024));
   if (per_sm > 8) per_sm = 8;   // 2,048 threads an SM
-  if (ctas <= per_sm * sms)
-    return launch_mma_s<HD, TOut, 4, 8, MAPS, MIXED>(q, q_stride, q_col, row_slot, row_pos, kv, group, out, out_stride,
-                                        scale, softcap, sink, opt, n_rows, n_splits, part_acc, part_ml, counters,
-                                        append, k_col, v_col, clustered, stream);
-  return launch_mma_s<HD, TOut, 2, 4, MAPS, MIXED>(q, q_stride, q_col, row_slot, row_pos, kv, group, out, out_stride,
-                                      scale, softcap, sink, opt, n_rows, n_splits, part_acc, part_ml, counters, append,
-                                      k_col, v_col, clustered, stream);
+#define NB_GO(STAGES_, WARPS_)                                                                                    \
+  return launch_mma_s<HD, TOut, STAGES_, WARPS_, MAPS, MIXED>(q, q_stride, q_col, row_slot, row_pos, kv, group, out, \
+                                                              out_stride, scale, softcap, sink, opt, n_rows, n_splits, \
+                                                              part_acc, part_ml, counters, append, k_col, v_col, clustered, stream)
+  if constexpr (HD == 64 && !MAPS && !MIXED) {
+    // Heads of 64: four warps and two pages where splits share a sequence or the CTAs are few (us, one
+    // sequence of 900 tokens x 12 heads in eight splits 3.5, with eight warps and four pages 3.9; 4 x 450 tokens
+    // 4.7 and 5.2); whole sequences in so many CTAs that latencies overlap among them by
+    // two warps with 32 keys each and, where that puts all of them on the GPU, one page (64
+    // sequences of 97 to 152 tokens x 25 heads 13.1, with two pages 16.0, with four warps 16.2; x 12 heads
+    // 9.5, 9.0 and 9.3; of 500 to 1,000 tokens x 25 heads 54.1, 53.4 and 52.9).
+    if (n_splits > 1 || ctas <= 4LL * sms) NB_GO(2, 4);
+    if (ctas <= 6LL * sms) NB_GO(2, 2);
+    NB_GO(1, 2);
+  } else {
+    if (ctas <= per_sm * sms) NB_GO(4, 8);
+    NB_GO(2, 4);
+  }
+#undef NB_GO
 }
 
 }  // namespace

@@ -276,15 +276,20 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     auto take_out = [&](int b, uint32_t parity) {
       if (!__all_sync(0xffffffffu, mbar_wait(acc_full(b), parity, abort_flag))) return false;
       tc05_fence_after();
-      for (int half = 0; half < (b == 2 ? 2 : 1); ++half) {
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          uint32_t v[16];
-          tc05_ld_32x32b_x16(lanes + (uint32_t)(b * 128 + half * BN + q * 16), v);
+      for (int q = 0; q < 2; ++q) {
+        uint32_t v[16];
+        tc05_ld_32x32b_x16(lanes + (uint32_t)(b * 128 + q * 16), v);
+        if (b == 2) {      // the two halves are added up first: that rounds 2^-8 of the result
+          uint32_t w[16];
+          tc05_ld_32x32b_x16(lanes + (uint32_t)(b * 128 + BN + q * 16), w);
           tc05_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 16; ++j) u[q * 16 + j] += __uint_as_float(v[j]);
+          for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
         }
+        tc05_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) u[q * 16 + j] += __uint_as_float(v[j]);
       }
       tc05_fence_before();
       __syncwarp();

@@ -48,7 +48,7 @@ constexpr int MAX_SPLIT = 8;         // portable cluster size
 constexpr int W_BYTES = BW * BK * 2;                 // 16 KB
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 64 + EPI_WARPS * 32;
-constexpr int SMEM_BUDGET = 104 * 1024;
+constexpr int SMEM_BUDGET = 200 * 1024;
 constexpr int AHEAD = 2;             // pieces of the residual a thread asks for ahead
 
 struct RowsShape {

@@ -792,80 +792,47 @@ int launch(const void* X, const void* W, const float* bias, const float* residua
 }
 
 // Tile width.  A single row tile (at most 128 rows) is a weight stream: many narrow tiles
-// with a deep ring.  Otherwise every tile re-reads its 128 rows of X and its BN rows of W from
-// L2, so wide tiles win for large products; for products of a few hundred tiles what counts
-// is how many waves the 148 SMs need and how long a wave is, so the width is the one with
-// the least waves x (width + a tile's fixed cost, about 48 columns' worth of time).  The
-// fp32 TMA epilogue has room for 128 columns at most and alone takes 96; the direct-store
-// epilogue takes 64, 128 and 256.
-int pick_tile_width(int M, int N, bool f32_out, bool tma_epi) {
-  const long long tiles_m = (M + BM - 1) / BM;
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-      sms = 148;
-  }
-  // A single row tile: narrow tiles, so that many CTAs share the stream of weights -- unless
-  // there are more of them than SMs (the output head): an MMA costs its issuing thread the
-  // same up to 128 columns, so a CTA that walks over several tiles does so twice as fast with
-  // tiles of 128.
-  if (tiles_m == 1) return (N + 63) / 64 > sms ? 128 : 64;
-  const int cand_f32_tma[] = {128, 96, 64}, cand_bf16_tma[] = {256, 192, 128, 64}, cand_direct[] = {256, 128, 64};
-  const int* cand = !tma_epi ? cand_direct : (f32_out ? cand_f32_tma : cand_bf16_tma);
-  const int n_cand = !tma_epi ? 3 : (f32_out ? 3 : 4);
-  int best = cand[n_cand - 1];
-  long long best_cost = -1;
-  for (int i = 0; i < n_cand; ++i) {
-    const int bn = cand[i];
-    if (bn > 64 && N < bn) continue;                       // wider than the output: wasted columns
-    const long long tiles = tiles_m * ((N + bn - 1) / bn);
-    const long long cost = ((tiles + sms - 1) / sms) * (bn + 48);
-    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = bn; }   // ties: the wider
-  }
-  return best;
-}
+// with a deep ring; of more tiles than SMs (the output head) 128 wide, since an MMA costs its
+// issuing thread the same up to 128 columns.
+int pick_stream_width(int N) { return (N + 63) / 64 > nb_device_sms() ? 128 : 64; }
 
-// What a large product is bound by is the 64 bytes per clock an SM can take in: a 128 x 256
-// tile brings 48 KB per K block for 512 clocks of MMAs.  In a pair each CTA brings half of the
-// weight tile (32 KB), which measures 1.36 against 1.20 PFLOP/s at 8192 x 6400 x 1600.  A
-// product of a wave or two of tiles is no faster in pairs, or slower (12.3 -> 13.4 us at
-// 2048 x 2304 x 768): the cluster's start-up and its barriers cost more than the lighter
-// loads save; pairs are taken from three waves of single-CTA tiles on.
+// Wider tiles re-read less of X and W from L2, and pairs of CTAs bring half of the weight tile each
+// (what bounds a large product is the 64 bytes per clock an SM can take in: 48 KB a block of K
+// for a 128 x 256 tile, 32 KB in a pair); but what counts for products of a few hundred tiles is how many
+// waves the SMs, or pairs of them, need and how long a wave is.  So every shape has a line
+// of its own, us = start + waves x (wave + blocks of K x block), fitted to 13 products of 15 heights from
+// 160 to 12,000 rows each, with cold weights and fp32 results added in place or bf16 with GELU: off by 4
+// to 7 % on average, and the shape chosen by them 0.1 % slower than the fastest one.  Measured (us; what
+// was taken before, with pairs up to 128 columns for fp32 from three waves on, without their early
+// start): 4128x1024x4096 34.5 (46.7), 6765x768x3072 38.4 (49.6), 7232x1600x6400 130 (200), 7232x1600x1600 43.8
+// (55.7), 2048x1600x6400 39.6 (63.4), 12000x2048x2048 95.7 (127), 6765x2304x768 29.0 (31.1), 4128x3072x768 23.6
+// (26.4).
+struct TileCost { int bn, pair; float start, wave, block; };
+constexpr TileCost COST_F32[] = {{64, 0, 2.07f, 1.30f, 0.253f}, {96, 0, 2.61f, 1.40f, 0.289f}, {128, 0, 2.37f, 1.85f, 0.298f},
+                                 {96, 1, 4.73f, 0.57f, 0.285f}, {128, 1, 4.97f, 1.12f, 0.285f}, {192, 1, 4.74f, 2.59f, 0.293f},
+                                 {256, 1, 2.33f, 4.56f, 0.367f}};
+constexpr TileCost COST_B16[] = {{64, 0, 3.39f, 0.38f, 0.294f}, {128, 0, 3.63f, 1.33f, 0.306f}, {192, 0, 3.78f, 1.60f, 0.345f},
+                                 {256, 0, 4.56f, 1.22f, 0.477f}, {128, 1, 5.40f, 0.70f, 0.307f}, {192, 1, 5.39f, 1.25f, 0.317f},
+                                 {256, 1, 5.72f, 1.15f, 0.395f}};
+// Direct stores (rows that TMA cannot store) take single CTAs of 64, 128 and 256 columns, by fewest waves
+// x (width + a tile's fixed cost, about 48 columns' worth of time).
+constexpr TileCost COST_DIRECT[] = {{256, 0, 0.0f, 304.0f, 0.0f}, {128, 0, 0.0f, 176.0f, 0.0f}, {64, 0, 0.0f, 112.0f, 0.0f}};
+
+int g_use_pairs = 1;   // pairs of CTAs: 0 off, 1 where they are faster, 2 wherever a paired kernel exists
 int g_force_bn = 0, g_force_pair = 0;
-int g_use_pairs = 1;   // 0 off, 1 where the cost model prefers them, 2 wherever a paired kernel exists
 
-// Width of 256-row tiles for pairs of CTAs, or 0 if single CTAs with `single_bn` are better.
-// Cost of a shape: waves over the SMs (or pairs of SMs) x what a CTA brings in per K block
-// (its rows of X, its rows of W) plus a tile's fixed cost, all in rows of 128 bytes.
-int pick_pair_width(int M, int N, bool f32_out, int single_bn) {
-  if (M <= BM) return 0;
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-      sms = 148;
-  }
-  const long long fixed = 64;
-  const long long tiles1 = (long long)((M + BM - 1) / BM) * ((N + single_bn - 1) / single_bn);
-  // measured: pairs pay from three waves of single-CTA tiles on, for narrow outputs (fewer
-  // than 1024 columns) from six
-  if (g_use_pairs < 2 && (tiles1 < 3ll * sms || (N < 1024 && tiles1 < 6ll * sms))) return 0;
-  long long best_cost = g_use_pairs >= 2 ? (1ll << 60)
-                                         : ((tiles1 + sms - 1) / sms) * (BM + single_bn + fixed);
-  int best = 0;
-  const int cand_f32[] = {128, 96}, cand_bf16[] = {256, 192, 128};
-  const int* cand = f32_out ? cand_f32 : cand_bf16;
-  const int n_cand = f32_out ? 2 : 3;
-  const int pairs = sms / 2;
-  for (int i = 0; i < n_cand; ++i) {
-    const int bn = cand[i];
-    if (N < bn && i + 1 < n_cand) continue;               // wider than the output: try a narrower one
-    const long long tiles2 = (long long)((M + 2 * BM - 1) / (2 * BM)) * ((N + bn - 1) / bn);
-    const long long cost = ((tiles2 + pairs - 1) / pairs) * (BM + bn / 2 + fixed);
-    if (cost < best_cost) { best_cost = cost; best = bn; }
+template <int COUNT>
+TileCost pick_tile(const TileCost (&cost)[COUNT], int M, int N, int K, int pairs) {
+  const long long sms = nb_device_sms(), blocks = (K + BK - 1) / BK;
+  TileCost best = {};
+  float best_us = 0.0f;
+  for (const TileCost& c : cost) {
+    if (c.pair ? pairs == 0 || M <= BM : pairs == 2 && M > BM) continue;
+    if (c.bn > N && c.bn > 64 && !(c.pair && c.bn == 96) && !(pairs == 2 && c.bn == 128)) continue;   // wider than the output
+    const long long rows = c.pair ? 2 * BM : BM, walkers = c.pair ? sms / 2 : sms;
+    const long long tiles = ((M + rows - 1) / rows) * ((N + c.bn - 1) / c.bn);
+    const float us = c.start + (float)((tiles + walkers - 1) / walkers) * (c.wave + (float)blocks * c.block);
+    if (best.bn == 0 || us < best_us) { best = c; best_us = us; }
   }
   return best;
 }
@@ -942,16 +909,19 @@ NB_EXPORT int nb_gemm_tcgen05(const void* X, const void* W, const float* bias, c
   // itself; otherwise every thread stores its own row segment.
   const int esize = out_dtype == NB_F32 ? 4 : 2;
   const bool tma_epi = ((long long)N * esize) % 16 == 0 && (residual == nullptr || residual == out);
-  const bool force = g_force_bn && tma_epi && M > BM;
-  const int bn = force && !g_force_pair ? g_force_bn : pick_tile_width(M, N, out_dtype == NB_F32, tma_epi);
+  TileCost tile = {M <= BM ? pick_stream_width(N) : 0, 0};
+  if (M > BM) {
+    if (!tma_epi) tile = pick_tile(COST_DIRECT, M, N, K, 0);
+    else if (g_force_bn) tile = {g_force_bn, g_force_pair};
+    else if (out_dtype == NB_F32) tile = pick_tile(COST_F32, M, N, K, g_use_pairs);
+    else tile = pick_tile(COST_B16, M, N, K, g_use_pairs);
+  }
+  const int bn = tile.bn, pair_bn = tile.pair ? tile.bn : 0;
   int rc;
-  // Pairs of CTAs on 256-row tiles bring less into each SM per flop (half of the weight tile
-  // each); they are taken when that outweighs the coarser tiles (see pick_pair_width).
-  const int pair_bn = force ? (g_force_pair ? g_force_bn : 0) : (tma_epi && g_use_pairs) ? pick_pair_width(M, N, out_dtype == NB_F32, bn) : 0;
   if (pair_bn) {
     rc = NB_ERR_BAD_ARG;
     if (out_dtype == NB_F32) {
-      if (force && g_force_pair == 2 && K > BK && pair_bn <= 192) {
+      if (tile.pair == 2 && K > BK && pair_bn <= 192) {
         if (pair_bn == 192) rc = launch<192, 1, float, 2>(X, W, bias, residual, out, M, N, K, act, stream);
         else if (pair_bn == 128) rc = launch<128, 1, float, 2>(X, W, bias, residual, out, M, N, K, act, stream);
         else if (pair_bn == 96) rc = launch<96, 1, float, 2>(X, W, bias, residual, out, M, N, K, act, stream);

@@ -62,13 +62,32 @@ def decode_splits(base_ctas: int, pages: int, page: int, head_dim: int, sms: int
     return s
 
 
+def decode_splits_64(base_ctas: int, pages: int, sms: int, most: int) -> int:
+    """The same for heads of 64 (four warps and two pages a CTA, six CTAs an SM): the most splits that
+    deal the pages out evenly and leave the launch at four CTAs an SM, or two splits where that
+    fills it to six (us; 12 heads, 16 pages: one sequence in 8 splits 3.5, in 4 4.0; 4 sequences 4.7 and
+    5.0; 8 in 4 8.1, in 8 over 8.9; 24 in 2 10.8, whole 12.3; 32 in 2 11.5, whole 13.2; 25 heads: 16 in 2
+    8.4, whole 9.8; 24 in 2 19.3, whole 18.7)."""
+    for s in (8, 4, 2):
+        if s <= most and pages % s == 0 and s * base_ctas <= (4 if s > 2 else 6) * sms:
+            return s
+    return 1
+
+
 def decode_splits_f32(base_ctas: int, pages: int, page: int, head_dim: int, sms: int, cluster: int) -> int:
     """Splits of a sequence's pages in the 32-bit decode attention: as many as put one launch on the
-    GPU at once (a CTA keeps two pages of keys and values, 64 KB with heads of 64), no more than merge
-    inside a cluster (`cluster`, 0: none do) unless a split would then walk over more than four pages."""
+    GPU at once (a CTA keeps two pages of keys and values, 64 KB with heads of 64).  What merges inside
+    a cluster (up to `cluster` splits, 0: none do) deals the pages out evenly, and is preferred unless
+    a split would then walk over more than four pages (us; 12 heads of 64, 16 pages: one sequence in 8
+    splits 5.0, in 16 7.1; 5 sequences in 4 7.8, in 7 8.9; 8 in 4 12.3, in 3 13.9; 24 in 2, a third more than
+    fit, 20.5, whole 23.4; 32 in 2 24.1, whole 23.7)."""
     room = max(1, min(8, (228 * 1024) // (4 * page * head_dim * 4 + 4096))) * sms
-    s = max(1, min(pages, room // base_ctas))
-    return min(s, cluster) if 0 < cluster and pages <= 4 * cluster else s
+    if 0 < cluster and pages <= 4 * cluster:
+        for s in (8, 4, 2):
+            if s <= cluster and pages % s == 0 and s * base_ctas <= (room if s > 2 else room * 4 // 3):
+                return s
+        return 1
+    return max(1, min(pages, room // base_ctas))
 
 
 def latent_splits(ctas: int, pages: int, sms: int) -> int:
@@ -504,10 +523,13 @@ class CudaBackend:
     # -- cache and attention ----------------------------------------------------------
     def _decode_splits(self, base_ctas: int, pages: int, kv, dtype) -> int:
         """Into how many splits a decode launch cuts each sequence's pages (`base_ctas`: rows x
-        key-value heads): `decode_splits_f32` and, on the tensor cores, `decode_splits`."""
+        key-value heads): `decode_splits_f32` and, on the tensor cores, `decode_splits_64` or
+        `decode_splits`."""
         if dtype != torch.bfloat16:
             return decode_splits_f32(base_ctas, pages, kv.page, kv.head_dim, self._sms,
                                      self._cluster_limit if self.decode_clusters else 0)
+        if kv.head_dim == 64 and self.decode_clusters:
+            return decode_splits_64(base_ctas, pages, self._sms, self._cluster_limit)
         return decode_splits(base_ctas, pages, kv.page, kv.head_dim, self._sms,
                              self._cluster_limit if self.decode_clusters else 16)
 
