@@ -83,7 +83,7 @@ struct SmemLayout {
 };
 
 template <int BN, int EPI, typename TOut, int PAIR>
-__global__ void __launch_bounds__(cta_threads(BN, EPI))
+__global__ void __launch_bounds__(cta_threads(BN, EPI), 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ CUtensorMap map_out, const float* __restrict__ bias,
                     const float* residual, TOut* out, int M, int N, int K, int act, int tiles_n,
