@@ -29,6 +29,7 @@ namespace {
 constexpr int TQ = 64;            // query rows per CTA
 constexpr int PAGE_TOKENS = 64;   // keys per page
 constexpr int LD = 64;            // floats between rows of a transposed tile
+constexpr int THREADS = 128;
 
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
@@ -71,15 +72,15 @@ __device__ __forceinline__ int prob_of(int j, int c) { return j * LD + ((c ^ ((j
 enum : int { VEC_Q = 1, VEC_KV = 2, VEC_OUT = 4 };   // operands whose rows may be taken 4 numbers at a time
 
 template <typename T, int HD, typename TOut>
-__global__ void __launch_bounds__(HD, HD == 64 ? 3 : 1)
+__global__ void __launch_bounds__(THREADS, HD == 64 ? 3 : 1)
 attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
                              const int* cu_rows, const int* seq_slot,
                              const int* seq_pos0, NbPagedKV kv, int group,
                              TOut* out, int out_stride, float scale, int window, int vec, int sms) {
-  constexpr int THREADS = HD;           // a thread has 8 rows and 8 columns of the result
-  constexpr int TX = HD / 8;            // threads that share a row
-  constexpr int KPT = PAGE_TOKENS / TX; // keys a thread: 8 or 4
-  constexpr int KP = KPT / 2, NL = 16;  // pairs of them; pieces of four numbers of a page's keys a thread
+  constexpr int TX = 16;                // threads that share a row
+  constexpr int KPT = PAGE_TOKENS / TX, KP = KPT / 2;      // keys a thread, pairs of them
+  constexpr int CH = HD / TX / 4;       // pieces of four columns of the result a thread, HD / CH apart
+  constexpr int NL = PAGE_TOKENS * HD / 4 / THREADS;       // pieces of four numbers of a page's keys a thread
   extern __shared__ __align__(16) float sm[];
   float* Qt = sm;                       // [HD][LD]: column d of row i
   float* Kt = Qt + HD * LD;             // [HD][LD]: column d of key j
@@ -154,17 +155,17 @@ attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
   __syncthreads();
   bring_values(p_begin);
 
-  f32x2 o[8][4];            // rows ty * 8 + i; columns tx * 4 + (0, 1), (2, 3) and HD / 2 further
+  f32x2 o[8][2 * CH];       // rows ty * 8 + i; columns tx * 4 + (0, 1), (2, 3), and HD / 2 further
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) o[i][c] = 0ull;
+    for (int c = 0; c < 2 * CH; ++c) o[i][c] = 0ull;
   float m_run[8], l_run[8];  // the sum of this thread's keys only
 #pragma unroll
   for (int i = 0; i < 8; ++i) { m_run[i] = -INFINITY; l_run[i] = 0.0f; }
 
   for (int p = p_begin; p < p_end; ++p) {
-    // scores: rows ty * 8 + i, keys tx * 4 + (0 .. 3) and, with 8 a thread, 32 further
+    // scores: rows ty * 8 + i, keys tx * 4 + (0 .. 3)
     f32x2 sc[8][KP];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
@@ -175,11 +176,8 @@ attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
       const float4 a0 = *reinterpret_cast<const float4*>(Qt + piece_of(d, ty * 2));
       const float4 a1 = *reinterpret_cast<const float4*>(Qt + piece_of(d, ty * 2 + 1));
       f32x2 kk[KP];
-#pragma unroll
-      for (int c = 0; c < KP / 2; ++c) {
-        const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(Kt + piece_of(d, tx + 8 * c));
-        kk[2 * c] = t.x; kk[2 * c + 1] = t.y;
-      }
+      const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(Kt + piece_of(d, tx));
+      kk[0] = t.x; kk[1] = t.y;
       const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -197,7 +195,7 @@ attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
       float mx = -INFINITY;
 #pragma unroll
       for (int c = 0; c < KPT; ++c) {
-        const int key = p * PAGE_TOKENS + tx * 4 + (c & 3) + (c >> 2) * 32;
+        const int key = p * PAGE_TOKENS + tx * 4 + c;
         const float2 v = unpair(sc[i][c >> 1]);
         const bool ok = all || (key <= qp && (window <= 0 || key > qp - window));
         pr[i][c] = ok ? ((c & 1) ? v.y : v.x) * scale : -INFINITY;
@@ -218,13 +216,13 @@ attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
       l_run[i] = l_run[i] * resc + sum;
       const f32x2 r2 = pair_of(resc, resc);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) mul2(o[i][c], r2);
+      for (int c = 0; c < 2 * CH; ++c) mul2(o[i][c], r2);
     }
     // a warp reads only what its own threads wrote (its rows)
     __syncwarp();
 #pragma unroll
     for (int c = 0; c < KPT; ++c) {
-      const int j = tx * 4 + (c & 3) + (c >> 2) * 32;
+      const int j = tx * 4 + c;
       *reinterpret_cast<float4*>(Pt + prob_of(j, ty * 2)) = make_float4(pr[0][c], pr[1][c], pr[2][c], pr[3][c]);
       *reinterpret_cast<float4*>(Pt + prob_of(j, ty * 2 + 1)) = make_float4(pr[4][c], pr[5][c], pr[6][c], pr[7][c]);
     }
@@ -238,16 +236,18 @@ attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
     for (int j = 0; j < PAGE_TOKENS; ++j) {
       const float4 a0 = *reinterpret_cast<const float4*>(Pt + prob_of(j, ty * 2));
       const float4 a1 = *reinterpret_cast<const float4*>(Pt + prob_of(j, ty * 2 + 1));
-      const ulonglong2 v0 = *reinterpret_cast<const ulonglong2*>(Vs + j * HD + tx * 4);
-      const ulonglong2 v1 = *reinterpret_cast<const ulonglong2*>(Vs + j * HD + HD / 2 + tx * 4);
+      f32x2 vv[2 * CH];
+#pragma unroll
+      for (int c = 0; c < CH; ++c) {
+        const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(Vs + j * HD + c * (HD / 2) + tx * 4);
+        vv[2 * c] = t.x; vv[2 * c + 1] = t.y;
+      }
       const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const f32x2 a2 = pair_of(av[i], av[i]);
-        fma2(o[i][0], a2, v0.x);
-        fma2(o[i][1], a2, v0.y);
-        fma2(o[i][2], a2, v1.x);
-        fma2(o[i][3], a2, v1.y);
+#pragma unroll
+        for (int c = 0; c < 2 * CH; ++c) fma2(o[i][c], a2, vv[c]);
       }
     }
     if (more) {
@@ -265,7 +265,7 @@ attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
     if (ty * 8 + i >= rows_here) continue;
     const float inv = l_run[i] > 0.0f ? 1.0f / l_run[i] : 0.0f;
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
+    for (int c = 0; c < CH; ++c) {
       const float2 x = unpair(o[i][2 * c]), y = unpair(o[i][2 * c + 1]);
       TOut* dst = out + (size_t)(row0 + q0 + ty * 8 + i) * out_stride + (size_t)h * HD + c * (HD / 2) + tx * 4;
       if (sizeof(TOut) == 4 && (vec & VEC_OUT)) {
@@ -294,7 +294,7 @@ int launch(const void* q, int q_stride, int q_col, const int* cu_rows, const int
   const bool vec_out = (uintptr_t)out % 16 == 0 && out_stride % 4 == 0;
   const int vec = (vec_q ? VEC_Q : 0) | (vec_kv ? VEC_KV : 0) | (vec_out ? VEC_OUT : 0);
   dim3 grid((max_q_len + TQ - 1) / TQ, n_heads, n_seqs);
-  NB_CUDA(nb_launch(kern, grid, dim3(HD), smem, stream, (const T*)q, q_stride, q_col, cu_rows,
+  NB_CUDA(nb_launch(kern, grid, dim3(THREADS), smem, stream, (const T*)q, q_stride, q_col, cu_rows,
                     seq_slot, seq_pos0, kv, n_heads / kv.n_kv_heads, (TOut*)out, out_stride, scale,
                     window, vec, nb_device_sms()));
   return 0;
