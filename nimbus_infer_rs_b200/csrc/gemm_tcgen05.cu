@@ -57,9 +57,6 @@ __host__ __device__ constexpr int cta_threads(int bn, int epi) { return 96 + 32 
 // the next tile's products, and the 64 KB it saves are two stages of the ring.
 // PAIR 1: two CTAs of a cluster share 256 x BN tiles (`cta_group::2`): each brings its 128
 // rows of X and half of the tile's rows of W, so a stage holds BN / 2 rows of W.
-// PAIR 2: two such pairs, a cluster of four, share one tile and take half of K each; CTAs of the same rows
-// exchange 32-column chunks of their sums through shared memory (where the ring was) and each finishes
-// every other chunk.  For products of so few tiles that half of the SMs would idle.
 template <int BN, int EPI, int ESIZE, int PAIR>
 struct SmemLayout {
   static constexpr int A_BYTES = BM * BK * 2;
@@ -95,7 +92,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   static_assert(BN % 32 == 0 && BN >= 32 && BN <= 256, "tile width");
   static_assert(EPI == 1 || BN == 64 || BN == 128 || BN == 256, "direct-store epilogue: 64/128/256");
   static_assert(BN % 64 == 0 || (EPI == 1 && sizeof(TOut) == 4), "odd widths: fp32 TMA epilogue only");
-  static_assert(PAIR < 2 || (sizeof(TOut) == 4 && L::TILES_BYTES >= EW * 4096), "cut tiles: fp32 results, sums where the ring was");
   extern __shared__ unsigned char smem_dyn[];
   // 1024-byte alignment (swizzle atoms), computed on the shared-window address
   const uint32_t raw = smem_u32(smem_dyn);
@@ -113,20 +109,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  constexpr bool CUT = PAIR == 2;
+  const int num_kb = (K + BK - 1) / BK;
   // Paired CTAs: rank 0 is the leader.  It alone issues the MMAs (which read both CTAs'
   // shared memory and write both CTAs' tensor memory); the TMA loads of both CTAs count on the
   // leader's full barriers; commits go to the barriers of both; the epilogue warps of both tell
   // the leader's accumulator-empty barriers.
-  uint32_t crank = 0;
-  if constexpr (PAIR) asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(crank));
-  const uint32_t rank = crank & 1u, lead = crank & 2u;          // place in the pair, its leader's rank
-  const int half = (int)(crank >> 1);                           // CUT: which half of K
-  const int walker = (int)(blockIdx.x >> PAIR);                 // who walks over tiles
-  const int n_walkers = (int)(gridDim.x >> PAIR);
-  const int all_kb = (K + BK - 1) / BK;
-  const int kb0 = CUT ? half * ((all_kb + 1) / 2) : 0;          // this CTA's blocks of K
-  const int num_kb = CUT ? (half ? all_kb - kb0 : (all_kb + 1) / 2) : all_kb;
+  uint32_t rank = 0;
+  if constexpr (PAIR) asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
+  const int walker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;    // who walks over tiles
+  const int n_walkers = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
   const int m_off = PAIR ? (int)rank * BM : 0;                   // this CTA's rows in a tile
   constexpr int TILE_M = PAIR ? 2 * BM : BM;
 
@@ -186,7 +177,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       const uint32_t w_dst = base + kb * L::STAGE_BYTES + L::A_BYTES;
       if constexpr (PAIR) {
         if (rank == 0) mbar_expect_tx(full_bar(kb), 2u * ((uint32_t)a_box_bytes + L::B_BYTES));
-        tma_load_2d_pair(w_dst, &map_w, (kb0 + kb) * BK, n0, cluster_addr(full_bar(kb), lead));
+        tma_load_2d_pair(w_dst, &map_w, kb * BK, n0, cluster_addr(full_bar(kb), 0));
       } else {
         mbar_expect_tx(full_bar(kb), (uint32_t)a_box_bytes + L::B_BYTES);
         tma_load_2d(w_dst, &map_w, kb * BK, n0, full_bar(kb));
@@ -267,12 +258,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
           const uint32_t a_dst = base + s * L::STAGE_BYTES;
           if constexpr (PAIR) {
             // both CTAs' bytes are counted on the leader's barrier, which the leader arms
-            const uint32_t lead_bar = cluster_addr(full_bar(s), lead);
+            const uint32_t lead_bar = cluster_addr(full_bar(s), 0);
             if (rows_of_x) {
               if (rank == 0 && !early) mbar_expect_tx(full_bar(s), 2u * ((uint32_t)a_box_bytes + L::B_BYTES));
-              tma_load_2d_pair(a_dst, &map_x, (kb0 + kb) * BK, m0, lead_bar);
+              tma_load_2d_pair(a_dst, &map_x, kb * BK, m0, lead_bar);
             } else if (!early) {
-              tma_load_2d_pair(a_dst + L::A_BYTES, &map_w, (kb0 + kb) * BK, n0, lead_bar);
+              tma_load_2d_pair(a_dst + L::A_BYTES, &map_w, kb * BK, n0, lead_bar);
             }
             continue;
           }
@@ -349,10 +340,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                             (kb > 0 || k > 0) ? 1u : 0u);
           }
           // the stage is free (in both CTAs) once these MMAs have read it
-          if constexpr (PAIR) tc05_commit_pair(empty_bar(s), lead); else tc05_commit(empty_bar(s));
+          if constexpr (PAIR) tc05_commit_pair(empty_bar(s)); else tc05_commit(empty_bar(s));
         }
         // complete once all MMAs issued so far are done
-        if (ok) { if constexpr (PAIR) tc05_commit_pair(acc_full(ab), lead); else tc05_commit(acc_full(ab)); }
+        if (ok) { if constexpr (PAIR) tc05_commit_pair(acc_full(ab)); else tc05_commit(acc_full(ab)); }
       }
     }
   } else if constexpr (EPI == 1) {   // ---------- epilogue through shared memory and TMA stores
@@ -371,36 +362,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     const uint32_t my_row = stg + (uint32_t)lane * 128u;
     const uint32_t swz = (uint32_t)(lane & 7);
     uint32_t t = 0;
-    const uint32_t lead_empty0 = PAIR ? cluster_addr(acc_empty(0), lead) : 0u;
+    const uint32_t lead_empty0 = PAIR ? cluster_addr(acc_empty(0), 0) : 0u;
     if (dual) {   // the second issuing thread, before its warp turns to the epilogue
       if (e == 0 && lane == 0) dual_walk(1);
       __syncwarp();
     }
-    if constexpr (CUT) {
-      // The chunk that this CTA finishes waits for the other pair's sums (below); the other one goes there.
-      const int mine = half, theirs = 1 - half;
-      const int row0 = (walker / tiles_n) * TILE_M + m_off + quarter * 32, col = (walker % tiles_n) * BN + unit * 64;
-      if (lane == 0 && residual != nullptr && mine < nch) {
-        mbar_expect_tx(res_bar(e, 0), 4096u);
-        tma_load_2d(stg, &map_out, col + mine * 32, row0, res_bar(e, 0));
-      }
-      __syncwarp();
-      if (__shfl_sync(0xffffffffu, (int)mbar_wait(acc_full(0), 0u, abort_flag), 0) != 0 && theirs < nch) {
-        tc05_fence_after();
-        uint32_t v[32];
-        tc05_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(unit * 64 + theirs * 32), v);
-        tc05_wait_ld();
-        const uint32_t row = base + (uint32_t)e * 4096u + (uint32_t)lane * 128u;      // the MMAs are done with the ring
-#pragma unroll
-        for (int q4 = 0; q4 < 8; ++q4)
-          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(row + (((uint32_t)q4 ^ swz) << 4)), "r"(v[4 * q4]),
-                       "r"(v[4 * q4 + 1]), "r"(v[4 * q4 + 2]), "r"(v[4 * q4 + 3])
-                       : "memory");
-        tc05_fence_before();
-      }
-      __syncwarp();
-    }
-    for (int tile = CUT ? num_tiles : walker; tile < num_tiles; tile += n_walkers, ++t) {
+    for (int tile = walker; tile < num_tiles; tile += n_walkers, ++t) {
       const int m0 = (tile / tiles_n) * TILE_M + m_off, n0 = (tile % tiles_n) * BN;
       const int row0 = m0 + quarter * 32, col0 = n0 + unit * 64;
       const uint32_t ab = t & 1u, aphase = (t >> 1) & 1u;
@@ -527,7 +494,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         }
       }
     }
-    if (!CUT && lane == 0) bulk_wait_all();   // stores must have left shared memory before it goes away
+    if (lane == 0) bulk_wait_all();   // stores must have left shared memory before it goes away
   } else {             // ------------------------------------------------------ epilogue, direct stores
     const int quarter = warp & 3;   // the 32 tensor-memory lanes this warp may read
     const int half = (warp - 2) >> 2;   // which share of the tile's columns it takes
@@ -622,60 +589,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   
   }
 
-  if constexpr (CUT) {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-    const int e = warp - 2, quarter = warp & 3, unit = e >> 2, c = half;
-    if (e >= 0 && e < EW && unit * 64 + c * 32 < BN && *abort_flag == 0) {
-      const int row0 = (walker / tiles_n) * TILE_M + m_off + quarter * 32;
-      const int nb = (walker % tiles_n) * BN + unit * 64 + c * 32;
-      const uint32_t stg = stg_base + (uint32_t)e * L::STG_PER_WARP, swz = (uint32_t)(lane & 7);
-      const uint32_t buf = stg + (uint32_t)lane * 128u;
-      const uint32_t other = cluster_addr(base + (uint32_t)e * 4096u + (uint32_t)lane * 128u, crank ^ 2u);
-      const float bias_l = bias && nb + lane < N ? __ldg(bias + nb + lane) : 0.0f;
-      float4 o4[8];
-#pragma unroll
-      for (int q4 = 0; q4 < 8; ++q4)
-        asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];\n"
-                     : "=f"(o4[q4].x), "=f"(o4[q4].y), "=f"(o4[q4].z), "=f"(o4[q4].w)
-                     : "r"(other + (((uint32_t)q4 ^ swz) << 4))
-                     : "memory");
-      uint32_t v[32];
-      tc05_fence_after();
-      tc05_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(unit * 64 + c * 32), v);
-      tc05_wait_ld();
-      float f[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const float4 q = o4[j >> 2];
-        f[j] = __uint_as_float(v[j]) + ((j & 3) == 0 ? q.x : (j & 3) == 1 ? q.y : (j & 3) == 2 ? q.z : q.w);
-        f[j] += __shfl_sync(0xffffffffu, bias_l, j);
-      }
-      nb_apply_act_fast_all(f, act);
-      bool ok = true;
-      if (residual != nullptr) ok = __shfl_sync(0xffffffffu, (int)mbar_wait(res_bar(e, 0), 0u, abort_flag), 0) != 0;
-      if (ok) {
-#pragma unroll
-        for (int q4 = 0; q4 < 8; ++q4) {
-          const uint32_t at = buf + (((uint32_t)q4 ^ swz) << 4);
-          float4 r4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          if (residual != nullptr)
-            asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];\n" : "=f"(r4.x), "=f"(r4.y), "=f"(r4.z), "=f"(r4.w) : "r"(at));
-          asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};\n" ::"r"(at), "f"(f[4 * q4] + r4.x), "f"(f[4 * q4 + 1] + r4.y),
-                       "f"(f[4 * q4 + 2] + r4.z), "f"(f[4 * q4 + 3] + r4.w)
-                       : "memory");
-        }
-        fence_async_smem();
-        __syncwarp();
-        if (lane == 0 && nb < N && row0 < M) {
-          tma_store_2d(&map_out, stg, nb, row0);
-          bulk_commit();
-          bulk_wait_all();
-        }
-      }
-      __syncwarp();
-    }
-  }
   tc05_fence_before();
   __syncthreads();
   if (*abort_flag) {
@@ -771,9 +684,9 @@ int launch(const void* X, const void* W, const float* bias, const float* residua
     NB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   }
   if constexpr (PAIR) {
-    // clusters of two CTAs, one cluster per pair of SMs; of four, one per tile
-    const int walkers = PAIR == 2 || num_tiles < sms / 2 ? (int)num_tiles : sms / 2;
-    NB_CUDA(nb_launch_clusters(kern, dim3(walkers << PAIR), dim3(cta_threads(BN, EPI)), (size_t)smem, stream, 1 << PAIR, mx, mw,
+    // clusters of two CTAs, one cluster per pair of SMs
+    const int pairs = (int)(num_tiles < sms / 2 ? num_tiles : sms / 2);
+    NB_CUDA(nb_launch_clusters(kern, dim3(2 * pairs), dim3(cta_threads(BN, EPI)), (size_t)smem, stream, 2, mx, mw,
                                mo, bias, residual, (TOut*)out, M, N, K, act, tiles_n, (int)num_tiles,
                                a_rows * BK * 2, error_word(), 1 << 1));
     return 0;
@@ -921,11 +834,7 @@ NB_EXPORT int nb_gemm_tcgen05(const void* X, const void* W, const float* bias, c
   if (pair_bn) {
     rc = NB_ERR_BAD_ARG;
     if (out_dtype == NB_F32) {
-      if (tile.pair == 2 && K > BK && pair_bn <= 192) {
-        if (pair_bn == 192) rc = launch<192, 1, float, 2>(X, W, bias, residual, out, M, N, K, act, stream);
-        else if (pair_bn == 128) rc = launch<128, 1, float, 2>(X, W, bias, residual, out, M, N, K, act, stream);
-        else if (pair_bn == 96) rc = launch<96, 1, float, 2>(X, W, bias, residual, out, M, N, K, act, stream);
-      } else if (pair_bn == 256) rc = launch<256, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, stream);
+      if (pair_bn == 256) rc = launch<256, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, stream);
       else if (pair_bn == 192) rc = launch<192, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, stream);
       else if (pair_bn == 128) rc = launch<128, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, stream);
       else if (pair_bn == 96) rc = launch<96, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, stream);

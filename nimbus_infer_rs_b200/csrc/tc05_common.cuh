@@ -90,12 +90,12 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
       "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(leader_bar)
       : "memory");
 }
-// One arrival on the barrier at this offset in both CTAs of the pair (ranks `lead` and `lead` + 1 of the
-// cluster), once the MMAs issued so far are done.
-__device__ __forceinline__ void tc05_commit_pair(uint32_t bar, uint32_t lead = 0) {
+// One arrival on the barrier at this offset in both CTAs of the pair, once the MMAs issued so
+// far are done.
+__device__ __forceinline__ void tc05_commit_pair(uint32_t bar) {
   asm volatile(
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(bar),
-      "h"((unsigned short)(3u << lead))
+      "h"((unsigned short)3)
       : "memory");
 }
 // D (256 rows: 128 in each CTA's tensor memory) += A (each CTA's 128 rows) * B (each CTA's half
