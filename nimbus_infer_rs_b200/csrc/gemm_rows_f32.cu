@@ -104,6 +104,7 @@ gemm_rows_f32_kernel(const float* X, RowNorm norm, const float* __restrict__ W, 
     bt = norm.beta != nullptr && tid < quads ? __ldg(reinterpret_cast<const float4*>(norm.beta) + tid) : zero;
   }
   nb_grid_dependency_wait();
+  nb_launch_dependents();
   [[maybe_unused]] float4 xn[NORM ? ROWS : 1];         // the normed rows, zero beyond M and K
   if constexpr (NORM) {
     __shared__ __align__(16) float sums[2][8][ROWS];
@@ -160,7 +161,6 @@ gemm_rows_f32_kernel(const float* X, RowNorm norm, const float* __restrict__ W, 
       }
       if (m0 + ROWS >= M) {
         if (grp + (int)gridDim.x < n_groups) load_weights(grp + gridDim.x);
-        else nb_launch_dependents();     // this CTA's weights are all in
       }
       deal_out(acc, lane);
       __syncthreads();                   // the sums before these have been read

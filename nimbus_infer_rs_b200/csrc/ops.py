@@ -1537,16 +1537,12 @@ class CudaBackend:
         self._call("nb_advance_decode", _ptr(tokens), _ptr(next_tokens), _ptr(row_pos),
                    _ptr(row_slot), _ptr(host), (tokens.numel()), self._stream())
 
-    def take_tokens(self, tokens, ring, count):
-        """``tokens`` <- the next entry of ``ring`` (pinned int32 ``[turns, 1 + n]``; ``count``, an int on
-        the device, says which and moves on), unless the entry's first number is 0."""
+    def set_tokens(self, tokens, given):
+        """``tokens`` (int32, on the device) <- ``given``, a CPU tensor of as many int32 numbers."""
         _check(tokens, "tokens", torch.int32, 1)
-        _check(count, "count", torch.int32, 1)
-        if not (ring.is_pinned() and ring.dtype == torch.int32 and ring.is_contiguous() and ring.dim() == 2
-                and ring.shape[1] == tokens.numel() + 1):
-            raise KernelError("take_tokens: the ring is pinned int32 memory, an entry 1 + n numbers")
-        self._call("nb_take_tokens", _ptr(tokens), _ptr(ring), _ptr(count), ring.shape[0], tokens.numel(),
-                   self._stream())
+        if given.is_cuda or given.dtype != torch.int32 or given.shape != tokens.shape or not given.is_contiguous():
+            raise KernelError("set_tokens: expected as many int32 numbers on the host as there are tokens")
+        self._call("nb_set_tokens", _ptr(tokens), _ptr(given), tokens.numel(), self._stream())
 
     # -- sampling ---------------------------------------------------------------------
     def argmax(self, logits, out):

@@ -1178,29 +1178,26 @@ NB_EXPORT int nb_advance_decode(int* tokens, const int* next, int* row_pos, cons
   return 0;
 }
 
-// The tokens of a decode step from the host: `ring` is pinned host memory, `turns` entries of 1 + n
-// numbers, taken in turn (`count`, on the device, says which is next and is moved on); an entry whose
-// first number is 0 leaves the tokens as they lie on the device.  A kernel and not a copy, so that it can
-// be recorded with the step it belongs to while the host is turns ahead.
-__global__ void __launch_bounds__(256)
-take_tokens_kernel(int* tokens, const volatile int* ring, int* count, int turns, int n) {
+// The tokens of a decode step from the host, as the parameters of a launch: no copy, and nothing that the
+// host has to keep until the step has run.
+constexpr int TOKENS_A_LAUNCH = 960;
+struct TokenParams { int t[TOKENS_A_LAUNCH]; };
+__global__ void __launch_bounds__(128)
+set_tokens_kernel(int* tokens, const __grid_constant__ TokenParams given, int n) {
   nb_grid_dependency_wait();
   nb_launch_dependents();
-  const int c = *count;
-  const volatile int* entry = ring + (size_t)(c % turns) * (n + 1);
-  const int given = entry[0];
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int t = entry[1 + i];          // asked for beside `given`, not behind it
-    if (given != 0) tokens[i] = t;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) *count = c + 1 == turns ? 0 : c + 1;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) tokens[i] = given.t[i];
 }
 
-NB_EXPORT int nb_take_tokens(int* tokens, const int* ring, int* count, int turns, int n, cudaStream_t stream) {
-  if (n == 0) return 0;
-  NB_REQUIRE(turns >= 1, NB_ERR_BAD_ARG, "take_tokens: a ring has entries");
-  NB_CUDA(nb_launch(take_tokens_kernel, dim3(1), dim3(256), 0, stream, tokens, ring, count, turns, n));
-  NB_CHECK_LAUNCH("take_tokens");
+// `given` is host memory, read before the call returns.
+NB_EXPORT int nb_set_tokens(int* tokens, const int* given, int n, cudaStream_t stream) {
+  NB_REQUIRE(n >= 0 && (n == 0 || given != nullptr), NB_ERR_BAD_ARG, "set_tokens: bad arguments");
+  for (int at = 0; at < n; at += TOKENS_A_LAUNCH) {
+    const int here = n - at < TOKENS_A_LAUNCH ? n - at : TOKENS_A_LAUNCH;
+    TokenParams p;
+    for (int i = 0; i < here; ++i) p.t[i] = given[at + i];
+    NB_CUDA(nb_launch(set_tokens_kernel, dim3(1), dim3(128), 0, stream, tokens + at, p, here));
+  }
+  NB_CHECK_LAUNCH("set_tokens");
   return 0;
 }

@@ -22,46 +22,19 @@ from .batch import BatchLayout
 from .context import StepContext
 
 
-class _TokenRing:
-    """The tokens that go between the host and the steps of a session, in pinned memory that the steps'
-    own kernels read and write: recorded with a step, they cost the host a store where a copy
-    costs it a call (one sequence of GPT-2 124M, us a step: 309 with copies, MEASURED with this).
+class _Selected:
+    """Pinned memory that the last kernel of a step leaves the selected tokens in: reading them is a
+    wait for the stream and no copy behind it."""
 
-    An entry holds what one step is given and is written again only when that step is done: the
-    host may be ``TURNS`` steps ahead of the device."""
-    TURNS = 4
-
-    def __init__(self, n: int, device):
-        self.entries = torch.zeros((self.TURNS, 1 + n), dtype=torch.int32, pin_memory=True)
-        self.selected = torch.zeros(n, dtype=torch.int32, pin_memory=True)
-        self.entries_np, self.selected_np = self.entries.numpy(), self.selected.numpy()
-        self.count = torch.zeros(1, dtype=torch.int32, device=device)
-        self.done = [torch.cuda.Event() for _ in range(self.TURNS)]
-        self.turn = 0
-
-    def put(self, tokens) -> None:
-        """What the next step runs (``None``: what lies on the device)."""
-        self.done[self.turn].synchronize()        # returns at once if never recorded or done
-        entry = self.entries_np[self.turn]
-        if tokens is not None:
-            entry[1:] = tokens
-        entry[0] = tokens is not None
-
-    def given(self) -> None:
-        """The step that takes the entry has been launched."""
-        self.done[self.turn].record()
-        self.turn = (self.turn + 1) % self.TURNS
-
-    def restart(self) -> None:
-        """The step was not launched whole: the device's place in the ring is the host's again."""
-        self.count.fill_(self.turn)
-        self.done[self.turn].record()
+    def __init__(self, n: int):
+        self.tokens = torch.zeros(n, dtype=torch.int32, pin_memory=True)
+        self.numpy = self.tokens.numpy()
+        self.written = torch.cuda.Event()
 
     def __del__(self):
-        # the allocator of pinned memory knows of copies, not of kernels: no step may be at work on it
+        # the allocator of pinned memory knows of copies, not of kernels: no step may still write it
         try:
-            for event in self.done:
-                event.synchronize()
+            self.written.synchronize()
         except Exception:      # the process is ending, or the device has failed
             pass
 
@@ -98,7 +71,7 @@ class DecodeSession:
             self._buf.copy_(torch.from_numpy(host), non_blocking=False)
             self._graph, self._graph_launches, self.logits = kept["graph"], kept["launches"], kept["logits"]
             self.hist, self.hist_len = kept["history"]
-            self._ring = kept["ring"]
+            self._selected = kept["selected"]
             self._steps = 1 if self._graph is not None else 0
         else:
             self._buf = torch.from_numpy(host).to(dev)
@@ -111,7 +84,7 @@ class DecodeSession:
             self._graph_launches = 0
             self._steps = 0
             self.hist = self.hist_len = None
-            self._ring = _TokenRing(n, dev) if dev.type == "cuda" else None
+            self._selected = _Selected(n) if dev.type == "cuda" else None
             if self.params.repetition_penalty != 1.0:
                 # what each sequence has generated, for the penalty: the token a row runs is
                 # appended on the device at the start of every step
@@ -154,9 +127,6 @@ class DecodeSession:
     def _device_step(self) -> None:
         eng = self.engine
         ctx = StepContext(eng.rt, eng.ops, self._layout(), eng.model.position, eng.cache)
-        ring = self._ring
-        if ring is not None:
-            eng.ops.take_tokens(self.tokens, ring.entries, ring.count)
         if self.hist is not None:
             eng.ops.history_append(self.hist, self.hist_len, self.tokens, self.row_slot)
         self.logits = eng.model.forward(ctx)
@@ -174,8 +144,9 @@ class DecodeSession:
         else:
             eng.ops.sample_temperature(self.logits, float(self.params.temperature), self.u,
                                        self.next_tokens)
-        if ring is not None:
-            eng.ops.hand_over_decode(self.tokens, self.next_tokens, self.row_pos, self.row_slot, ring.selected)
+        if self._selected is not None:
+            eng.ops.hand_over_decode(self.tokens, self.next_tokens, self.row_pos, self.row_slot,
+                                     self._selected.tokens)
         else:
             eng.ops.advance_decode(self.tokens, self.next_tokens, self.row_pos, self.row_slot)
 
@@ -195,8 +166,14 @@ class DecodeSession:
             # the kernel may have handed a row back (a mark instead of a token on the device)
             raise ValueError("with top-k or top-p a step takes its tokens from the host: pass "
                              "what read_tokens() returned")
-        if self._ring is None and tokens is not None:
-            self.tokens.copy_(torch.tensor(tokens, dtype=torch.int32))
+        if tokens is not None:
+            given = np.empty(self.n, dtype=np.int32)
+            given[:] = tokens
+            given = torch.from_numpy(given)
+            if self._selected is None:
+                self.tokens.copy_(given)
+            else:      # a launch that carries them, ahead of the step's
+                eng.ops.set_tokens(self.tokens, given)
         if any(cache.lens[s] % PAGE == 0 or cache.lens[s] + 1 > cache.max_seq_len for s, _ in grow):
             cache.reserve(grow)            # a new page somewhere, or an error to raise
         if not self.params.greedy:
@@ -204,24 +181,16 @@ class DecodeSession:
                   for i, alive in enumerate(self.live)]
             self.u.copy_(torch.tensor(us, dtype=torch.float64), non_blocking=False)
             self.last_u = us
-        ring = self._ring
-        if ring is not None:
-            ring.put(tokens)               # behind everything that may refuse the step
-        try:
-            if not self.use_graph or self._steps == 0:
-                self._device_step()        # the first step runs plainly and warms the kernels
-            else:
-                if self._graph is None:
-                    self._capture()        # records the step; nothing runs yet
-                launches = eng.ops.launches
-                self._graph.replay()
-                eng.ops.launches = launches + self._graph_launches
-        except Exception:
-            if ring is not None:
-                ring.restart()
-            raise
-        if ring is not None:
-            ring.given()
+        if not self.use_graph or self._steps == 0:
+            self._device_step()            # the first step runs plainly and warms the kernels
+        else:
+            if self._graph is None:
+                self._capture()            # records the step; nothing runs yet
+            launches = eng.ops.launches
+            self._graph.replay()
+            eng.ops.launches = launches + self._graph_launches
+        if self._selected is not None:
+            self._selected.written.record()
         self._steps += 1
         self._sampled = True
         for s, _ in grow:
@@ -247,7 +216,7 @@ class DecodeSession:
         else:
             torch.cuda.current_stream().synchronize()
             self.engine.ops.raise_device_errors()     # a kernel of the step gave up a wait
-            tokens = self._ring.selected_np.tolist()
+            tokens = self._selected.numpy.tolist()
         if any(t < 0 for t, alive in zip(tokens, self.live) if alive):
             tokens = self._settle_on_host(tokens)
         return tokens
@@ -283,7 +252,7 @@ class DecodeSession:
             self.engine.decode_states[self._key] = {
                 "buffers": (self._buf, self.next_tokens, self.want_rows, self.cu_rows, self.u),
                 "graph": self._graph, "launches": self._graph_launches, "logits": self.logits,
-                "history": (self.hist, self.hist_len), "ring": self._ring,
+                "history": (self.hist, self.hist_len), "selected": self._selected,
                 # scratch buffers of the kernel library that the graph points into
                 "scratch": self.engine.ops.scratch_refs() if hasattr(self.engine.ops, "scratch_refs") else None}
             while len(self.engine.decode_states) > 8:

@@ -119,8 +119,11 @@ def test_32_bit_prompt_attention_at_the_edges_of_its_tiles(ops, dtype, H, Hk, hd
 
 
 def test_a_session_that_runs_ahead_of_the_device(tmp_path):
-    """Tokens from the host for more steps than the ring has turns, nothing read in between, steps
-    without tokens among them, and a step that is refused: the logits of plain steps."""
+    """Tokens from the host for many steps with nothing read in between, steps without tokens among
+    them, and a step that is refused: the logits of plain steps.  More tokens than one launch carries."""
+    ops, many = ops_mod.backend(), torch.zeros(1923, dtype=torch.int32, device=DEV)
+    ops.set_tokens(many, torch.arange(7, 1930, dtype=torch.int32))
+    assert many.tolist() == list(range(7, 1930))
     from nimbus_infer_rs_b200 import Engine
     from nimbus_infer_rs_b200.engine.decode import DecodeSession
     from tiny_configs import make_model
