@@ -4,21 +4,24 @@
 // prompts; heads of 64 or 128, pages of 64 tokens.
 //
 // A CTA takes 64 consecutive query rows of one sequence and one head and walks over the
-// sequence's pages up to the last key its rows may see.  What bounds it is the multiply-adds (2 x 1,024
-// tokens x 12 heads of 64: 45 us at 128 a clock and SM), so everything is laid out to keep shared memory
-// out of their way: a thread has 8 rows x 8 keys of the scores and 8 rows x 8 columns of the result (with
-// heads of 128 twice the threads and 4 keys each), so four 16-byte reads feed 64 packed
-// multiply-adds; queries, keys and probabilities lie transposed, their 16-byte pieces exchanged by a
-// few bits of the row so that neither the transposing stores nor the reads meet in a bank.  The next
-// page's keys are asked for while P V runs and go from registers to shared memory after it, its values
-// by cp.async beside the next scores.  Scale, causal limit and window; running maximum per row (fp32,
-// maximum subtracted, src/ops.rs:6-18) through shuffles among the threads that share a row, the sums per
-// thread until the end.  Keys after a row's own position, before its window or beyond the
-// sequence get no weight, and the rows of the last page that hold no key yet are never read.
+// sequence's pages up to the last key its rows may see, or over half of them (below).  The multiply-adds
+// are the floor (2 x 1,024 tokens x 12 heads of 64: 45 us at 128 a clock and SM); what bounds it is a warp's
+// chain of instructions, so as few of them as possible surround the multiply-adds: a thread has 8 rows
+// x 4 keys of the scores and 8 rows x 4 columns of the result (8 columns with heads of 128) as packed pairs of
+// rows, so three 16-byte reads and four doubled numbers feed 16 packed multiply-adds; queries, keys and
+// probabilities lie transposed, their 16-byte pieces exchanged by a few bits of the row so that neither
+// the transposing stores nor the reads meet in a bank.  The next page's keys are asked for while P V
+// runs and go from registers to shared memory after it, its values by cp.async beside the next scores.
+// Scale, causal limit and window; running maximum per row (fp32, maximum subtracted,
+// src/ops.rs:6-18) through shuffles among the threads that share a row, the sums per thread until
+// the end.  Keys after a row's own position, before its window or beyond the sequence get no weight, and
+// the rows of the last page that hold no key yet are never read.
 //
-// Tiles see as many pages as lie before them, from 1 to all.  CTAs are dealt out longest first, every
-// other turn over the SMs backwards, so that an SM's CTAs add up to about the same (2 x 1,024 tokens x
-// 12 heads: 22 pages an SM on average, 24 at most; in order of the tiles 36).
+// Tiles see as many pages as lie before them, from 1 to all, and a tile of 16 pages alone took as long as
+// all others together (192 us; an SM's pages are 22 on average).  So, where a chunk has several tiles,
+// the pages of a tile are halved between the two CTAs of a cluster, the second of which hands its maxima, sums
+// and weighted values to the first through shared memory; and the CTAs are dealt out longest first,
+// every other turn over the SMs backwards, so that an SM's CTAs add up to about the same.
 //
 // Reference: src/model.rs:401-422 (scores = dot(q,k)*scale for keys 0..P+i, softmax, weighted
 // values); head h reads key/value head h / group (src/model.rs:390).
@@ -76,9 +79,9 @@ __global__ void __launch_bounds__(THREADS, HD == 64 ? 3 : 1)
 attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
                              const int* cu_rows, const int* seq_slot,
                              const int* seq_pos0, NbPagedKV kv, int group,
-                             TOut* out, int out_stride, float scale, int window, int vec, int sms) {
+                             TOut* out, int out_stride, float scale, int window, int vec, int sms, int cut) {
   constexpr int TX = 16;                // threads that share a row
-  constexpr int KPT = PAGE_TOKENS / TX, KP = KPT / 2;      // keys a thread, pairs of them
+  constexpr int KPT = PAGE_TOKENS / TX; // keys a thread
   constexpr int CH = HD / TX / 4;       // pieces of four columns of the result a thread, HD / CH apart
   constexpr int NL = PAGE_TOKENS * HD / 4 / THREADS;       // pieces of four numbers of a page's keys a thread
   extern __shared__ __align__(16) float sm[];
@@ -89,14 +92,15 @@ attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
 
   nb_grid_dependency_wait();
   nb_launch_dependents();
-  // this CTA's place in the order of work (see the head of the file)
-  const unsigned long long b = blockIdx.x + (unsigned long long)gridDim.x * (blockIdx.y + (unsigned long long)gridDim.y * blockIdx.z);
-  const unsigned long long total = (unsigned long long)gridDim.x * gridDim.y * gridDim.z;
-  const unsigned long long first = b - b % sms;
-  const unsigned long long turn = total - first < (unsigned long long)sms ? total - first : (unsigned long long)sms;
-  const unsigned long long rank = (b / sms) & 1 ? first + (turn - 1 - (b - first)) : b;
+  // this CTA's place in the order of work (see the head of the file); `cut`: CTAs that share a tile
+  const unsigned half = blockIdx.x % cut, tiles = gridDim.x / cut, per_turn = (unsigned)sms / cut;
+  const unsigned long long b = blockIdx.x / cut + (unsigned long long)tiles * (blockIdx.y + (unsigned long long)gridDim.y * blockIdx.z);
+  const unsigned long long total = (unsigned long long)tiles * gridDim.y * gridDim.z;
+  const unsigned long long first = b - b % per_turn;
+  const unsigned long long turn = total - first < per_turn ? total - first : per_turn;
+  const unsigned long long rank = (b / per_turn) & 1 ? first + (turn - 1 - (b - first)) : b;
   const unsigned hs = gridDim.y * gridDim.z, rest = (unsigned)(rank % hs);
-  const int tile = (int)(gridDim.x - 1 - (unsigned)(rank / hs)), h = (int)(rest % gridDim.y), s = (int)(rest / gridDim.y);
+  const int tile = (int)(tiles - 1 - (unsigned)(rank / hs)), h = (int)(rest % gridDim.y), s = (int)(rest / gridDim.y);
   const int row0 = cu_rows[s], n_q = cu_rows[s + 1] - row0;
   const int q0 = tile * TQ;
   const int slot = seq_slot[s];
@@ -107,7 +111,9 @@ attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
   const int rows_here = min(TQ, n_q - q0);
   const int last_pos = pos0 + q0 + rows_here - 1;                    // newest key any row sees
   const int first_key = (window > 0) ? max(0, pos0 + q0 + 1 - window) : 0;
-  const int p_begin = first_key / PAGE_TOKENS, p_end = last_pos / PAGE_TOKENS + 1;
+  const int p_first = first_key / PAGE_TOKENS, p_last = last_pos / PAGE_TOKENS + 1;
+  const int p_middle = cut > 1 ? p_first + (p_last - p_first + 1) / 2 : p_last;
+  const int p_begin = half ? p_middle : p_first, p_end = half ? p_last : p_middle;
   const int* table = kv.block_table + (size_t)slot * kv.max_pages;
 
   // Which pieces this thread turns over: a warp takes 8 source rows x 4 pieces at a time, so a row's 64
@@ -142,7 +148,7 @@ attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
     cp_async_commit();
   };
 
-  ask_keys(p_begin);
+  if (p_begin < p_end) ask_keys(p_begin);
   // the query tile; rows beyond the sequence are zero
 #pragma unroll 4
   for (int n = 0; n < NL; ++n) {
@@ -150,45 +156,44 @@ attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
     put(Qt, n, i < rows_here ? load4(q + (size_t)(row0 + q0 + i) * q_stride + q_col + (size_t)h * HD + turn_piece(n) * 4, vec & VEC_Q)
                              : zero4);
   }
+  if (p_begin < p_end) {
 #pragma unroll
-  for (int n = 0; n < NL; ++n) put(Kt, n, kn[n]);
+    for (int n = 0; n < NL; ++n) put(Kt, n, kn[n]);
+  }
   __syncthreads();
-  bring_values(p_begin);
+  if (p_begin < p_end) bring_values(p_begin);
 
-  f32x2 o[8][2 * CH];       // rows ty * 8 + i; columns tx * 4 + (0, 1), (2, 3), and HD / 2 further
+  f32x2 o[4][4 * CH];       // rows ty * 8 + 2 i, 2 i + 1; columns tx * 4 + (0 .. 3), and HD / 2 further
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int c = 0; c < 2 * CH; ++c) o[i][c] = 0ull;
+    for (int c = 0; c < 4 * CH; ++c) o[i][c] = 0ull;
   float m_run[8], l_run[8];  // the sum of this thread's keys only
 #pragma unroll
   for (int i = 0; i < 8; ++i) { m_run[i] = -INFINITY; l_run[i] = 0.0f; }
 
   for (int p = p_begin; p < p_end; ++p) {
-    // scores: rows ty * 8 + i, keys tx * 4 + (0 .. 3)
-    f32x2 sc[8][KP];
+    // scores: rows ty * 8 + 2 i, 2 i + 1, keys tx * 4 + (0 .. 3)
+    f32x2 sc[4][KPT];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int c = 0; c < KP; ++c) sc[i][c] = 0ull;
+      for (int c = 0; c < KPT; ++c) sc[i][c] = 0ull;
 #pragma unroll 4
     for (int d = 0; d < HD; ++d) {
-      const float4 a0 = *reinterpret_cast<const float4*>(Qt + piece_of(d, ty * 2));
-      const float4 a1 = *reinterpret_cast<const float4*>(Qt + piece_of(d, ty * 2 + 1));
-      f32x2 kk[KP];
-      const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(Kt + piece_of(d, tx));
-      kk[0] = t.x; kk[1] = t.y;
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+      const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(Qt + piece_of(d, ty * 2));
+      const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(Qt + piece_of(d, ty * 2 + 1));
+      const float4 k4 = *reinterpret_cast<const float4*>(Kt + piece_of(d, tx));
+      const f32x2 av[4] = {a0.x, a0.y, a1.x, a1.y};
+      const f32x2 kv2[4] = {pair_of(k4.x, k4.x), pair_of(k4.y, k4.y), pair_of(k4.z, k4.z), pair_of(k4.w, k4.w)};
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const f32x2 a2 = pair_of(av[i], av[i]);
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int c = 0; c < KP; ++c) fma2(sc[i][c], a2, kk[c]);
-      }
+        for (int c = 0; c < KPT; ++c) fma2(sc[i][c], av[i], kv2[c]);
     }
     // scale, causal limit, window; the row's maximum among the threads of the row
     const bool all = (p + 1) * PAGE_TOKENS <= pos0 + q0 + 1 && window <= 0;   // every row sees every key
-    float pr[8][KPT];
+    float pr[8][KPT], resc[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int qp = pos0 + q0 + ty * 8 + i;           // absolute position of the row's query
@@ -196,16 +201,16 @@ attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
 #pragma unroll
       for (int c = 0; c < KPT; ++c) {
         const int key = p * PAGE_TOKENS + tx * 4 + c;
-        const float2 v = unpair(sc[i][c >> 1]);
+        const float2 v = unpair(sc[i >> 1][c]);
         const bool ok = all || (key <= qp && (window <= 0 || key > qp - window));
-        pr[i][c] = ok ? ((c & 1) ? v.y : v.x) * scale : -INFINITY;
+        pr[i][c] = ok ? ((i & 1) ? v.y : v.x) * scale : -INFINITY;
         mx = fmaxf(mx, pr[i][c]);
       }
 #pragma unroll
       for (int off = TX / 2; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
       const float m_new = fmaxf(m_run[i], mx);
       const float m_use = (m_new == -INFINITY) ? 0.0f : m_new;
-      const float resc = (m_run[i] == -INFINITY) ? 0.0f : expf(m_run[i] - m_use);
+      resc[i] = (m_run[i] == -INFINITY) ? 0.0f : expf(m_run[i] - m_use);
       m_run[i] = m_new;
       float sum = 0.0f;
 #pragma unroll
@@ -213,10 +218,13 @@ attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
         pr[i][c] = (pr[i][c] == -INFINITY) ? 0.0f : expf(pr[i][c] - m_use);
         sum += pr[i][c];
       }
-      l_run[i] = l_run[i] * resc + sum;
-      const f32x2 r2 = pair_of(resc, resc);
+      l_run[i] = l_run[i] * resc[i] + sum;
+    }
 #pragma unroll
-      for (int c = 0; c < 2 * CH; ++c) mul2(o[i][c], r2);
+    for (int i = 0; i < 4; ++i) {
+      const f32x2 r2 = pair_of(resc[2 * i], resc[2 * i + 1]);
+#pragma unroll
+      for (int c = 0; c < 4 * CH; ++c) mul2(o[i][c], r2);
     }
     // a warp reads only what its own threads wrote (its rows)
     __syncwarp();
@@ -234,20 +242,17 @@ attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
     // o += P V
 #pragma unroll 4
     for (int j = 0; j < PAGE_TOKENS; ++j) {
-      const float4 a0 = *reinterpret_cast<const float4*>(Pt + prob_of(j, ty * 2));
-      const float4 a1 = *reinterpret_cast<const float4*>(Pt + prob_of(j, ty * 2 + 1));
-      f32x2 vv[2 * CH];
+      const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(Pt + prob_of(j, ty * 2));
+      const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(Pt + prob_of(j, ty * 2 + 1));
+      const f32x2 av[4] = {a0.x, a0.y, a1.x, a1.y};
 #pragma unroll
-      for (int c = 0; c < CH; ++c) {
-        const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(Vs + j * HD + c * (HD / 2) + tx * 4);
-        vv[2 * c] = t.x; vv[2 * c + 1] = t.y;
-      }
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+      for (int q4 = 0; q4 < CH; ++q4) {
+        const float4 t = *reinterpret_cast<const float4*>(Vs + j * HD + q4 * (HD / 2) + tx * 4);
+        const f32x2 vv[4] = {pair_of(t.x, t.x), pair_of(t.y, t.y), pair_of(t.z, t.z), pair_of(t.w, t.w)};
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const f32x2 a2 = pair_of(av[i], av[i]);
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int c = 0; c < 2 * CH; ++c) fma2(o[i][c], a2, vv[c]);
+          for (int c = 0; c < 4; ++c) fma2(o[i][q4 * 4 + c], av[i], vv[c]);
       }
     }
     if (more) {
@@ -259,23 +264,82 @@ attention_prefill_f32_kernel(const T* q, int q_stride, int q_col,
   }
 
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
+  for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int off = TX / 2; off > 0; off >>= 1) l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], off);
-    if (ty * 8 + i >= rows_here) continue;
-    const float inv = l_run[i] > 0.0f ? 1.0f / l_run[i] : 0.0f;
+  // The second CTA's maxima, sums and weighted values, where its tiles were (all pages are done with):
+  // [64 rows][HD], maxima [64], sums [64].
+  float* part = sm;
+  if (cut > 1) {
+    if (half) {
 #pragma unroll
-    for (int c = 0; c < CH; ++c) {
-      const float2 x = unpair(o[i][2 * c]), y = unpair(o[i][2 * c + 1]);
-      TOut* dst = out + (size_t)(row0 + q0 + ty * 8 + i) * out_stride + (size_t)h * HD + c * (HD / 2) + tx * 4;
-      if (sizeof(TOut) == 4 && (vec & VEC_OUT)) {
-        *reinterpret_cast<float4*>(dst) = make_float4(x.x * inv, x.y * inv, y.x * inv, y.y * inv);
-      } else {
-        dst[0] = nb_from_f32<TOut>(x.x * inv); dst[1] = nb_from_f32<TOut>(x.y * inv);
-        dst[2] = nb_from_f32<TOut>(y.x * inv); dst[3] = nb_from_f32<TOut>(y.y * inv);
+      for (int i = 0; i < 8; ++i) {
+        const int r = ty * 8 + i;
+#pragma unroll
+        for (int q4 = 0; q4 < CH; ++q4) {
+          float y[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const float2 v = unpair(o[i >> 1][q4 * 4 + c]);
+            y[c] = (i & 1) ? v.y : v.x;
+          }
+          *reinterpret_cast<float4*>(part + r * HD + q4 * (HD / 2) + tx * 4) = make_float4(y[0], y[1], y[2], y[3]);
+        }
+        if (tx == 0) { part[TQ * HD + r] = m_run[i]; part[TQ * HD + TQ + r] = l_run[i]; }
+      }
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  }
+  if (half == 0) {
+    uint32_t other = 0;
+    if (cut > 1) {
+      const uint32_t own = (uint32_t)__cvta_generic_to_shared(part);
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(other) : "r"(own), "r"(1));
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = ty * 8 + i;
+      if (r >= rows_here) continue;
+      float l = l_run[i], own = 1.0f, more = 0.0f;        // factors of the two parts
+      if (cut > 1) {
+        float m1, l1;
+        asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(m1) : "r"(other + (uint32_t)(TQ * HD + r) * 4u) : "memory");
+        asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(l1) : "r"(other + (uint32_t)(TQ * HD + TQ + r) * 4u) : "memory");
+        const float m = fmaxf(m_run[i], m1);
+        own = m_run[i] == -INFINITY ? 0.0f : expf(m_run[i] - m);
+        more = m1 == -INFINITY ? 0.0f : expf(m1 - m);
+        l = l * own + l1 * more;
+      }
+      const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+#pragma unroll
+      for (int q4 = 0; q4 < CH; ++q4) {
+        float y[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float2 v = unpair(o[i >> 1][q4 * 4 + c]);
+          y[c] = (i & 1) ? v.y : v.x;
+        }
+        if (cut > 1) {
+          float4 t;
+          asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];\n"
+                       : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w)
+                       : "r"(other + (uint32_t)(r * HD + q4 * (HD / 2) + tx * 4) * 4u)
+                       : "memory");
+          y[0] = y[0] * own + t.x * more; y[1] = y[1] * own + t.y * more;
+          y[2] = y[2] * own + t.z * more; y[3] = y[3] * own + t.w * more;
+        }
+        TOut* dst = out + (size_t)(row0 + q0 + r) * out_stride + (size_t)h * HD + q4 * (HD / 2) + tx * 4;
+        if (sizeof(TOut) == 4 && (vec & VEC_OUT)) {
+          *reinterpret_cast<float4*>(dst) = make_float4(y[0] * inv, y[1] * inv, y[2] * inv, y[3] * inv);
+        } else {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) dst[c] = nb_from_f32<TOut>(y[c] * inv);
+        }
       }
     }
   }
+  if (cut > 1)      // the second CTA stays until it has been read
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
 template <typename T, int HD, typename TOut>
@@ -293,10 +357,11 @@ int launch(const void* q, int q_stride, int q_col, const int* cu_rows, const int
   const bool vec_kv = (uintptr_t)kv.k % 16 == 0 && (uintptr_t)kv.v % 16 == 0;
   const bool vec_out = (uintptr_t)out % 16 == 0 && out_stride % 4 == 0;
   const int vec = (vec_q ? VEC_Q : 0) | (vec_kv ? VEC_KV : 0) | (vec_out ? VEC_OUT : 0);
-  dim3 grid((max_q_len + TQ - 1) / TQ, n_heads, n_seqs);
-  NB_CUDA(nb_launch(kern, grid, dim3(THREADS), smem, stream, (const T*)q, q_stride, q_col, cu_rows,
+  const int tiles = (max_q_len + TQ - 1) / TQ, cut = tiles > 1 && tiles < (1 << 30) ? 2 : 1;
+  dim3 grid(tiles * cut, n_heads, n_seqs);
+  NB_CUDA(nb_launch_clusters(kern, grid, dim3(THREADS), smem, stream, cut, (const T*)q, q_stride, q_col, cu_rows,
                     seq_slot, seq_pos0, kv, n_heads / kv.n_kv_heads, (TOut*)out, out_stride, scale,
-                    window, vec, nb_device_sms()));
+                    window, vec, nb_device_sms(), cut));
   return 0;
 }
 
