@@ -111,24 +111,6 @@ __device__ __forceinline__ void nb_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
 
-// Weights (constants) that a later product of the step will read: a product of a few rows asks for them
-// to be brought into L2 while it runs, so that DRAM works through the latencies of the chain of
-// launches and not only while a product streams.  A hint: results do not depend on it.
-struct NbAhead {
-  const void* p;         // 16-byte aligned, or null
-  long long bytes;       // a multiple of 16
-};
-// One thread of every CTA of a one-dimensional grid calls it: an equal share each.
-__device__ __forceinline__ void nb_fetch_ahead(const NbAhead& a) {
-  if (a.p == nullptr) return;
-  const long long share = ((a.bytes + gridDim.x - 1) / gridDim.x + 127) & ~127LL;
-  const long long end = min(a.bytes, share * (blockIdx.x + 1));
-  for (long long at = share * blockIdx.x; at < end; at += 16384) {
-    const unsigned n = (unsigned)min(16384LL, end - at);
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"((const char*)a.p + at), "r"(n) : "memory");
-  }
-}
-
 template <typename... KArgs, typename... Args>
 inline cudaError_t nb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                              cudaStream_t stream, Args... args) {

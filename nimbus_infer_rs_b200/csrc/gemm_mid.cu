@@ -38,7 +38,6 @@ struct MidShape {
   int split;         // CTAs of a cluster = runs of K
   int kb_per;        // blocks of K a CTA
   int stages, stage_bytes, smem;
-  NbAhead ahead;
 };
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
@@ -115,7 +114,6 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         if (++s == sh.stages) { s = 0; phase ^= 1u; }
       }
     }
-    if (lane == 0) nb_fetch_ahead(sh.ahead);
     __syncwarp();
     __syncthreads();
   } else {
@@ -279,7 +277,7 @@ bool plan_mid(int M, int N, int K, MidShape* out) {
   if (M < 1 || M > MAX_ROWS || N < 1 || K < 8 || K % 8 != 0) return false;
   const int sms = nb_device_sms(), blocks = (K + BK - 1) / BK;
   const int rows = (M <= 32 ? 4 : (M <= 64 ? 8 : 16)) * 8;
-  MidShape s = {};
+  MidShape s;
   s.wn = 4;
   bool cut = true;
   if (M > 64 && (N + 31) / 32 * 4 <= sms) s.wn = 2;
@@ -419,15 +417,13 @@ NB_EXPORT int nb_gemm_mid_force(int columns, int split) {
 NB_EXPORT int nb_gemm_mid_set_wait_budget(long long cycles) { return set_wait_budget(cycles); }
 
 NB_EXPORT int nb_gemm_mid(const void* X, const void* W, const float* bias, const float* residual, void* out,
-                          int out_dtype, int M, int N, int K, int act, const void* ahead, long long ahead_bytes,
-                          cudaStream_t stream) {
+                          int out_dtype, int M, int N, int K, int act, cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;
   MidShape sh;
   NB_REQUIRE(plan_mid(M, N, K, &sh), NB_ERR_UNSUPPORTED,
              "gemm_mid: takes 1 to %d rows and K a multiple of 8 (M=%d N=%d K=%d)", MAX_ROWS, M, N, K);
   NB_REQUIRE((uintptr_t)X % 16 == 0 && (uintptr_t)W % 16 == 0, NB_ERR_UNSUPPORTED,
              "gemm_mid: operands must be 16-byte aligned");
-  sh.ahead = {ahead, ahead_bytes};
   int rc;
   if (out_dtype == NB_F32) rc = launch_nt<float>(X, W, bias, residual, out, M, N, K, act, sh, stream);
   else if (out_dtype == NB_BF16) rc = launch_nt<bf16>(X, W, bias, residual, out, M, N, K, act, sh, stream);

@@ -67,12 +67,11 @@ NB_EXPORT int nb_gemm_stream_set_wait_budget(long long cycles) {
 // rows first (X must then be fp32); `residual` may alias `out` (fp32).
 NB_EXPORT int nb_gemm_stream(const void* X, int x_dtype, const float* gamma, const float* beta,
                              float eps, const void* W, const float* bias, const float* residual,
-                             void* out, int out_dtype, int M, int N, int K, int act, const void* ahead,
-                             long long ahead_bytes, cudaStream_t stream) {
+                             void* out, int out_dtype, int M, int N, int K, int act,
+                             cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;
   const bool ln = gamma != nullptr;
-  StreamPlan p = plan_stream(M, N, K, ln);
-  p.sh.ahead = {ahead, ahead_bytes};
+  const StreamPlan p = plan_stream(M, N, K, ln);
   NB_REQUIRE(p.ok, NB_ERR_UNSUPPORTED, "gemm_stream: does not take M=%d N=%d K=%d%s", M, N, K,
              ln ? " with a norm" : "");
   NB_REQUIRE(!ln || x_dtype == NB_F32, NB_ERR_BAD_ARG, "gemm_stream: a fused norm needs fp32 rows");

@@ -69,7 +69,6 @@ struct StreamShape {
   int tpr;        // threads that share a row while it is normalised
   int n16;        // groups of 16 columns of the whole product
   unsigned vpr_magic;   // ceil(2^32 / vectors per staged row): index / vectors = umulhi(index, magic)
-  NbAhead ahead;
 };
 
 // The tensor-core instruction takes 16 x 16 of one operand and 16 x 8 of the other.  The weights
@@ -219,7 +218,6 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const TX* X,
   // this kernel's weights were asked for long ago: the kernel behind it may start and ask for
   // its own (only now: see common.cuh on what a kernel may read before its wait)
   nb_launch_dependents();
-  if (tid == NT - 1) nb_fetch_ahead(sh.ahead);
 
   // what the first batch's epilogue adds, asked for before anything else
   float e_res[EPT];

@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(cta_threads(BN, EPI), 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ CUtensorMap map_out, const float* __restrict__ bias,
                     const float* residual, TOut* out, int M, int N, int K, int act, int tiles_n,
-                    int num_tiles, int a_box_bytes, int* err_word, int tune, NbAhead ahead) {
+                    int num_tiles, int a_box_bytes, int* err_word, int tune) {
   using L = SmemLayout<BN, EPI, (int)sizeof(TOut), PAIR>;
   constexpr int EW = L::EPI_WARPS;
   constexpr int ACC = acc_stride(BN);
@@ -239,7 +239,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   // take the count below zero for a while (the phase cannot end before the arming arrives).
   const bool split_xw = (tune >> 1) == 1;
   if (warp == 2 + EW && !split_xw) {
-    if (lane == 0) nb_fetch_ahead(ahead);      // no operand to bring in
+    // nothing to bring in
   } else if (split_xw && (warp == 0 || warp == 2 + EW)) {
     const bool rows_of_x = warp == 0;
     if (lane == 0) {
@@ -645,7 +645,7 @@ __global__ void wait_probe_kernel(int* err_word, int* status) {
 // ---------------------------------------------------------------------------------- host
 template <int BN, int EPI, typename TOut, int PAIR = 0>
 int launch(const void* X, const void* W, const float* bias, const float* residual, void* out, int M,
-           int N, int K, int act, const NbAhead& ahead, cudaStream_t stream) {
+           int N, int K, int act, cudaStream_t stream) {
   using L = SmemLayout<BN, EPI, (int)sizeof(TOut), PAIR>;
   static_assert(L::STAGES >= 2, "tile shape leaves no room for a pipeline");
   CUtensorMap mx, mw, mo;
@@ -688,7 +688,7 @@ int launch(const void* X, const void* W, const float* bias, const float* residua
     const int pairs = (int)(num_tiles < sms / 2 ? num_tiles : sms / 2);
     NB_CUDA(nb_launch_clusters(kern, dim3(2 * pairs), dim3(cta_threads(BN, EPI)), (size_t)smem, stream, 2, mx, mw,
                                mo, bias, residual, (TOut*)out, M, N, K, act, tiles_n, (int)num_tiles,
-                               a_rows * BK * 2, error_word(), 1 << 1, NbAhead{}));
+                               a_rows * BK * 2, error_word(), 1 << 1));
     return 0;
   }
   const int grid = (int)(num_tiles < sms ? num_tiles : sms);   // one CTA per SM walks the tiles
@@ -700,7 +700,7 @@ int launch(const void* X, const void* W, const float* bias, const float* residua
   const int tune = (g_dual ? 1 : 0) | ((g_lanes ? (M <= BM ? 2 : 1) : 0) << 1);
   NB_CUDA(nb_launch(kern, dim3(grid), dim3(cta_threads(BN, EPI)), (size_t)smem, stream, mx, mw, mo, bias,
                     residual, (TOut*)out, M, N, K, act, tiles_n, (int)num_tiles, a_rows * BK * 2,
-                    error_word(), tune, M <= BM ? ahead : NbAhead{}));
+                    error_word(), tune));
   return 0;
 }
 
@@ -808,8 +808,8 @@ NB_EXPORT int nb_wait_probe(int* status, cudaStream_t stream) {
 }
 
 NB_EXPORT int nb_gemm_tcgen05(const void* X, const void* W, const float* bias, const float* residual,
-                              void* out, int out_dtype, int M, int N, int K, int act, const void* ahead_of,
-                              long long ahead_bytes, cudaStream_t stream) {
+                              void* out, int out_dtype, int M, int N, int K, int act,
+                              cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;
   NB_REQUIRE(nb_gemm_tcgen05_supported(NB_BF16, NB_BF16, M, N, K), NB_ERR_UNSUPPORTED,
              "gemm_tcgen05: needs bf16 operands and a width that is a multiple of 8 (M=%d N=%d K=%d)",
@@ -822,7 +822,6 @@ NB_EXPORT int nb_gemm_tcgen05(const void* X, const void* W, const float* bias, c
   // itself; otherwise every thread stores its own row segment.
   const int esize = out_dtype == NB_F32 ? 4 : 2;
   const bool tma_epi = ((long long)N * esize) % 16 == 0 && (residual == nullptr || residual == out);
-  const NbAhead ahead = {ahead_of, ahead_bytes};
   TileCost tile = {M <= BM ? pick_stream_width(N) : 0, 0};
   if (M > BM) {
     if (!tma_epi) tile = pick_tile(COST_DIRECT, M, N, K, 0);
@@ -835,21 +834,21 @@ NB_EXPORT int nb_gemm_tcgen05(const void* X, const void* W, const float* bias, c
   if (pair_bn) {
     rc = NB_ERR_BAD_ARG;
     if (out_dtype == NB_F32) {
-      if (pair_bn == 256) rc = launch<256, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, ahead, stream);
-      else if (pair_bn == 192) rc = launch<192, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, ahead, stream);
-      else if (pair_bn == 128) rc = launch<128, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, ahead, stream);
-      else if (pair_bn == 96) rc = launch<96, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, ahead, stream);
+      if (pair_bn == 256) rc = launch<256, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, stream);
+      else if (pair_bn == 192) rc = launch<192, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, stream);
+      else if (pair_bn == 128) rc = launch<128, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, stream);
+      else if (pair_bn == 96) rc = launch<96, 1, float, 1>(X, W, bias, residual, out, M, N, K, act, stream);
     } else if (out_dtype == NB_BF16) {
-      if (pair_bn == 256) rc = launch<256, 1, bf16, 1>(X, W, bias, residual, out, M, N, K, act, ahead, stream);
-      else if (pair_bn == 192) rc = launch<192, 1, bf16, 1>(X, W, bias, residual, out, M, N, K, act, ahead, stream);
-      else if (pair_bn == 128) rc = launch<128, 1, bf16, 1>(X, W, bias, residual, out, M, N, K, act, ahead, stream);
+      if (pair_bn == 256) rc = launch<256, 1, bf16, 1>(X, W, bias, residual, out, M, N, K, act, stream);
+      else if (pair_bn == 192) rc = launch<192, 1, bf16, 1>(X, W, bias, residual, out, M, N, K, act, stream);
+      else if (pair_bn == 128) rc = launch<128, 1, bf16, 1>(X, W, bias, residual, out, M, N, K, act, stream);
     }
     NB_REQUIRE(rc != NB_ERR_BAD_ARG, NB_ERR_BAD_ARG, "gemm_tcgen05: no paired kernel of width %d", pair_bn);
     if (rc) return rc;
     NB_CHECK_LAUNCH("gemm_tcgen05");
     return 0;
   }
-#define NB_TC(BN_, EPI_, T_) rc = launch<BN_, EPI_, T_>(X, W, bias, residual, out, M, N, K, act, ahead, stream)
+#define NB_TC(BN_, EPI_, T_) rc = launch<BN_, EPI_, T_>(X, W, bias, residual, out, M, N, K, act, stream)
   if (out_dtype == NB_F32) {
     if (tma_epi) {
       if (bn == 128) NB_TC(128, 1, float); else if (bn == 96) NB_TC(96, 1, float); else NB_TC(64, 1, float);

@@ -115,10 +115,6 @@ def _ptr(t: torch.Tensor | None) -> int:
     return 0 if t is None else t.data_ptr()
 
 
-def _bytes(t: torch.Tensor | None) -> int:
-    return 0 if t is None else t.numel() * t.element_size()
-
-
 try:    # the current stream's handle without building a Stream object (a few hundred ns)
     _raw_stream = torch._C._cuda_getCurrentRawStream
 except AttributeError:   # pragma: no cover
@@ -397,8 +393,6 @@ class CudaBackend:
                 raise KernelError("linear: residual shape does not match")
         tensor_core = (x.dtype == torch.bfloat16 or norm is not None and norm[3] == torch.bfloat16) \
             and w.dtype == torch.bfloat16 and K % 8 == 0 and self.use_tcgen05
-        # weights that the step reads after these (a hint that the model leaves on its weights)
-        ahead = getattr(w, "ahead", None) if M <= ROWS_MAX_ROWS else None
         # 17 to 128 rows over few columns, and fewer with a long K: all rows and a few columns
         # a CTA, K cut among a cluster
         if norm is None and self.use_tcgen05 and M <= ROWS_MAX_ROWS \
@@ -406,7 +400,7 @@ class CudaBackend:
                 and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and (
                     self.lib.nb_gemm_mid_preferred(M, N, K, act, dtype_code(out.dtype)) if self.use_mid == 1
                     else self.lib.nb_gemm_mid_supported(M, N, K)):
-            self._gemm_mid(x, w, bias, residual, out, act, ahead)
+            self._gemm_mid(x, w, bias, residual, out, act)
             return
         # few rows: the weight-streaming kernel; from 17 rows on the tensor-core kernel streams
         # weights faster (TMA ring), where it applies
@@ -425,7 +419,7 @@ class CudaBackend:
                 gamma, beta, eps = (norm[0], norm[1], norm[2]) if norm is not None else (None, None, 0.0)
                 self._call("nb_gemm_stream", _ptr(x), dtype_code(x.dtype), _ptr(gamma), _ptr(beta), eps,
                            _ptr(w), _ptr(bias), _ptr(residual), _ptr(out), dtype_code(out.dtype), M, N,
-                           K, act, _ptr(ahead), _bytes(ahead), self._stream())
+                           K, act, self._stream())
                 return
         # a 32-bit decode step of a few sequences: the norm inside the product
         if norm is not None and norm[3] == torch.float32 and w.dtype == torch.float32 and x.dtype == torch.float32 \
@@ -465,7 +459,7 @@ class CudaBackend:
         if self.use_tcgen05 and self.lib.nb_gemm_tcgen05_supported(
                 dtype_code(x.dtype), dtype_code(w.dtype), M, N, K):
             self._call("nb_gemm_tcgen05", _ptr(x), _ptr(w), _ptr(bias), _ptr(residual), _ptr(out),
-                       dtype_code(out.dtype), M, N, K, act, _ptr(ahead), _bytes(ahead),
+                       dtype_code(out.dtype), M, N, K, act,
                        self._stream())
             return
         # a prompt in 32-bit: three bf16 pieces of every number on the tensor cores
@@ -482,10 +476,9 @@ class CudaBackend:
                    dtype_code(out.dtype), M, N, K, act,
                    self._stream())
 
-    def _gemm_mid(self, x, w, bias, residual, out, act, ahead=None) -> None:
+    def _gemm_mid(self, x, w, bias, residual, out, act) -> None:
         self._call("nb_gemm_mid", _ptr(x), _ptr(w), _ptr(bias), _ptr(residual), _ptr(out),
-                   dtype_code(out.dtype), x.shape[0], w.shape[0], x.shape[1], act, _ptr(ahead), _bytes(ahead),
-                   self._stream())
+                   dtype_code(out.dtype), x.shape[0], w.shape[0], x.shape[1], act, self._stream())
 
     # A kernel whose bounded wait on a barrier ran out says so in a word of pinned host memory
     # (one per kernel family); its results are not valid.

@@ -13,10 +13,8 @@ import torch
 
 from ..parts.base import ParamSpec, bind_params, build_part, collect_param_specs
 from ..parts.embedding import LMHead, TokenEmbedding
-from ..parts.linear import Linear
 from .spec import ModelSpec
 
-AHEAD_MAX_BYTES = 32 << 20   # of weights brought into L2 ahead of their product (126 MB, shared with the cache)
 EMBEDDING_ENTRY = -1     # the key of the embedding's state rows among the schedule entries
 
 PRECISIONS = {"bfloat16": torch.bfloat16, "bf16": torch.bfloat16,
@@ -104,21 +102,6 @@ class Model:
             bind_params(part, params, self.rt, prefix)
         if self.spec.tie_head:
             self.head.tie(self.embedding.table)
-        self._link_weights()
-
-    def _link_weights(self) -> None:
-        """Leaves on every layer's weights which weights to bring into L2 while they are multiplied: the
-        ones after the next (those of the next product are asked for by its own kernel before it waits),
-        in the order of the layers and their parts.  A hint for the kernels of few rows."""
-        order = []
-        for layer in self.layers:
-            for part in layer.parts().values():
-                order += [c.weight for c in part.children().values() if isinstance(c, Linear)]
-        order = [t for t in order if t is not None and t.is_cuda and t.dtype == torch.bfloat16
-                 and t.is_contiguous() and t.data_ptr() % 16 == 0 and t.numel() % 8 == 0]
-        for t, ahead in zip(order, order[2:]):
-            if ahead.numel() * 2 <= AHEAD_MAX_BYTES:
-                t.ahead = ahead
 
     def graph_safe(self) -> bool:
         """True if every part of the model may run under CUDA-graph capture."""
