@@ -14,11 +14,7 @@
 // 8x768x3072 6.3 (13.2), 8x50257x768 53 (91), 1x768x3072 5.9 (11.6), 32x768x3072 17 (40),
 // 64x768x768 11 (35).
 //
-// With a LayerNorm in front (NORM: up to 8 rows, K up to 1024) a CTA norms the rows itself: a thread
-// holds its pieces of all rows, the sums meet through shared memory, mean first and then the
-// centred squares as in the pass of its own (rowwise.cu), which this saves.
-//
-// Reference analogue: Mat::gemv_into (src/model.rs:65-86), layer norm src/ops.rs:32-40.
+// Reference analogue: Mat::gemv_into (src/model.rs:65-86).
 #include "gemm_f32.cuh"
 
 namespace {
@@ -41,44 +37,12 @@ __device__ __forceinline__ void deal_out(float (&v)[N], int lane) {
   }
 }
 
-// Sums of eight values over the CTA, the same for every thread; `red`: [warps][8].  Ends behind a barrier
-// that all threads have passed since they called.
-__device__ __forceinline__ void cta_sums(float (&v)[ROWS], float (*red)[ROWS], int warp, int lane, int warps) {
-#pragma unroll
-  for (int half = ROWS / 2, bit = 16; half > 0; half >>= 1, bit >>= 1) {
-    const bool up = lane & bit;
-#pragma unroll
-    for (int i = 0; i < half; ++i) {
-      const float send = up ? v[i] : v[half + i];
-      const float keep = up ? v[half + i] : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
-    }
-  }
-  float t = v[0];                     // row lane / 4
-  t += __shfl_xor_sync(0xffffffffu, t, 2);
-  t += __shfl_xor_sync(0xffffffffu, t, 1);
-  if ((lane & 3) == 0) red[warp][lane >> 2] = t;
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < ROWS; ++r) v[r] = 0.0f;
-  for (int w = 0; w < warps; ++w)
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) v[r] += red[w][r];
-}
-
-struct RowNorm {
-  const float* gamma;
-  const float* beta;       // or null
-  float eps;
-};
-
 // NQ: 16-byte pieces of a weight row that a thread holds.
-template <int COLS, int NQ, typename TOut, bool NORM>
+template <int COLS, int NQ, typename TOut>
 __global__ void __launch_bounds__(256)
-gemm_rows_f32_kernel(const float* X, RowNorm norm, const float* __restrict__ W, const float* __restrict__ bias,
+gemm_rows_f32_kernel(const float* X, const float* __restrict__ W, const float* __restrict__ bias,
                      const float* residual, TOut* out, int M, int N, int K, int act) {
   constexpr int VALUES = ROWS * COLS, EACH = VALUES / 32;
-  static_assert(!NORM || NQ == 1, "a thread holds its pieces of all rows");
   __shared__ float red[8][VALUES];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, threads = blockDim.x;
   const int quads = K >> 2;
@@ -97,41 +61,7 @@ gemm_rows_f32_kernel(const float* X, RowNorm norm, const float* __restrict__ W, 
       }
   };
   load_weights(blockIdx.x);
-  [[maybe_unused]] float4 gm, bt;
-  if constexpr (NORM) {
-    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    gm = tid < quads ? __ldg(reinterpret_cast<const float4*>(norm.gamma) + tid) : zero;
-    bt = norm.beta != nullptr && tid < quads ? __ldg(reinterpret_cast<const float4*>(norm.beta) + tid) : zero;
-  }
   nb_grid_dependency_wait();
-  nb_launch_dependents();
-  [[maybe_unused]] float4 xn[NORM ? ROWS : 1];         // the normed rows, zero beyond M and K
-  if constexpr (NORM) {
-    __shared__ __align__(16) float sums[2][8][ROWS];
-    float v[ROWS], mean[ROWS];
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r)
-      xn[r] = (r < M && tid < quads) ? *(reinterpret_cast<const float4*>(X + (size_t)r * K) + tid)
-                                     : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) v[r] = (xn[r].x + xn[r].y) + (xn[r].z + xn[r].w);
-    cta_sums(v, sums[0], warp, lane, threads >> 5);
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-      mean[r] = v[r] / (float)K;
-      xn[r].x -= mean[r]; xn[r].y -= mean[r]; xn[r].z -= mean[r]; xn[r].w -= mean[r];
-      v[r] = tid < quads ? (xn[r].x * xn[r].x + xn[r].y * xn[r].y) + (xn[r].z * xn[r].z + xn[r].w * xn[r].w) : 0.0f;
-    }
-    cta_sums(v, sums[1], warp, lane, threads >> 5);
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-      const float inv = 1.0f / sqrtf(v[r] / (float)K + norm.eps);
-      xn[r].x = xn[r].x * inv * gm.x + bt.x;
-      xn[r].y = xn[r].y * inv * gm.y + bt.y;
-      xn[r].z = xn[r].z * inv * gm.z + bt.z;
-      xn[r].w = xn[r].w * inv * gm.w + bt.w;
-    }
-  }
 
   for (int grp = blockIdx.x; grp < n_groups; grp += gridDim.x) {
     for (int m0 = 0; m0 < M; m0 += ROWS) {
@@ -145,8 +75,7 @@ gemm_rows_f32_kernel(const float* X, RowNorm norm, const float* __restrict__ W, 
         float4 x[ROWS];
 #pragma unroll
         for (int r = 0; r < ROWS; ++r)
-          if constexpr (NORM) x[r] = xn[r];
-          else x[r] = (r < rows && k < quads) ? *(reinterpret_cast<const float4*>(X + (size_t)(m0 + r) * K) + k)
+          x[r] = (r < rows && k < quads) ? *(reinterpret_cast<const float4*>(X + (size_t)(m0 + r) * K) + k)
                                          : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
         for (int r = 0; r < ROWS; ++r)
@@ -161,6 +90,7 @@ gemm_rows_f32_kernel(const float* X, RowNorm norm, const float* __restrict__ W, 
       }
       if (m0 + ROWS >= M) {
         if (grp + (int)gridDim.x < n_groups) load_weights(grp + gridDim.x);
+        else nb_launch_dependents();     // this CTA's weights are all in
       }
       deal_out(acc, lane);
       __syncthreads();                   // the sums before these have been read
@@ -184,13 +114,13 @@ gemm_rows_f32_kernel(const float* X, RowNorm norm, const float* __restrict__ W, 
 
 // Threads that share K, and CTAs of so many that fit on the GPU at once.
 int threads_for(int K, int nq) { return ((K / 4 + nq - 1) / nq + 31) / 32 * 32; }
-template <int COLS, int NQ, typename TOut, bool NORM>
+template <int COLS, int NQ, typename TOut>
 cudaError_t fitting(int threads, int* fit) {
   static int resident[9] = {};       // by warps
   if (resident[threads / 32] == 0) {
     int per_sm = 0;
     const cudaError_t e =
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemm_rows_f32_kernel<COLS, NQ, TOut, NORM>, threads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemm_rows_f32_kernel<COLS, NQ, TOut>, threads, 0);
     if (e != cudaSuccess) return e;
     resident[threads / 32] = (per_sm > 0 ? per_sm : 1) * nb_device_sms();
   }
@@ -198,32 +128,15 @@ cudaError_t fitting(int threads, int* fit) {
   return cudaSuccess;
 }
 
-template <int COLS, int NQ, typename TOut, bool NORM>
-cudaError_t launch(const float* X, const RowNorm& norm, const float* W, const float* bias, const float* residual, TOut* out,
+template <int COLS, int NQ, typename TOut>
+cudaError_t launch(const float* X, const float* W, const float* bias, const float* residual, TOut* out,
                    int M, int N, int K, int act, cudaStream_t stream) {
   const int threads = threads_for(K, NQ), n_groups = (N + COLS - 1) / COLS;
   int fit = 0;
-  const cudaError_t e = fitting<COLS, NQ, TOut, NORM>(threads, &fit);
+  const cudaError_t e = fitting<COLS, NQ, TOut>(threads, &fit);
   if (e != cudaSuccess) return e;
-  return nb_launch(gemm_rows_f32_kernel<COLS, NQ, TOut, NORM>, dim3(n_groups < fit ? n_groups : fit), dim3(threads), 0,
-                   stream, X, norm, W, bias, residual, out, M, N, K, act);
-}
-
-// eight columns a CTA where that leaves a CTA for every SM and all CTAs run at once, else four: a second
-// walk over groups of eight costs more than one over groups of four (1 row us, eight and four:
-// 2304x768 3.6 and 3.9, 1184x1024 2.5 and 3.0; but 3072x640 4.7 and 4.2, 50257x768 57 and 51, and above 768
-// of K, where the registers leave an SM one CTA of 256 threads, 1600x1024 4.4 and 3.1, 4096x1024 10.1
-// and 8.3, 50257x1024 98 and 70)
-template <typename TOut, bool NORM>
-cudaError_t launch_short(const float* X, const RowNorm& norm, const float* W, const float* bias, const float* residual,
-                         TOut* out, int M, int N, int K, int act, cudaStream_t stream) {
-  if (N >= 8 * nb_device_sms()) {
-    int fit = 0;
-    const cudaError_t e = fitting<8, 1, TOut, NORM>(threads_for(K, 1), &fit);
-    if (e != cudaSuccess) return e;
-    if ((N + 7) / 8 <= fit) return launch<8, 1, TOut, NORM>(X, norm, W, bias, residual, out, M, N, K, act, stream);
-  }
-  return launch<4, 1, TOut, NORM>(X, norm, W, bias, residual, out, M, N, K, act, stream);
+  return nb_launch(gemm_rows_f32_kernel<COLS, NQ, TOut>, dim3(n_groups < fit ? n_groups : fit), dim3(threads), 0,
+                   stream, X, W, bias, residual, out, M, N, K, act);
 }
 
 }  // namespace
@@ -235,10 +148,23 @@ bool nb_gemm_f32_rows(const float* X, const float* W, const float* bias, const f
   // 16-byte pieces; a row of weights is held in at most three of them a thread (with more the weights
   // of four columns no longer fit beside the rows in registers)
   if (K % 4 || K < 4 || K > 3 * 1024 || (uintptr_t)X % 16 || (uintptr_t)W % 16) return false;
-  const RowNorm none = {};
-  if (K <= 1024) *err = launch_short<TOut, false>(X, none, W, bias, residual, out, M, N, K, act, stream);
-  else if (K <= 2048) *err = launch<4, 2, TOut, false>(X, none, W, bias, residual, out, M, N, K, act, stream);
-  else *err = launch<4, 3, TOut, false>(X, none, W, bias, residual, out, M, N, K, act, stream);
+  // eight columns a CTA where that leaves a CTA for every SM and all CTAs run at once, else four: a second
+  // walk over groups of eight costs more than one over groups of four (1 row us, eight and four:
+  // 2304x768 3.6 and 3.9, 1184x1024 2.5 and 3.0; but 3072x640 4.7 and 4.2, 50257x768 57 and 51, and above 768
+  // of K, where the registers leave an SM one CTA of 256 threads, 1600x1024 4.4 and 3.1, 4096x1024 10.1
+  // and 8.3, 50257x1024 98 and 70)
+  bool wide = false;
+  if (K <= 1024 && N >= 8 * nb_device_sms()) {
+    int fit = 0;
+    *err = fitting<8, 1, TOut>(threads_for(K, 1), &fit);
+    if (*err != cudaSuccess) return true;
+    wide = (N + 7) / 8 <= fit;
+  }
+#define NB_GO(C_, Q_) *err = launch<C_, Q_, TOut>(X, W, bias, residual, out, M, N, K, act, stream)
+  if (K <= 1024) { if (wide) NB_GO(8, 1); else NB_GO(4, 1); }
+  else if (K <= 2048) NB_GO(4, 2);
+  else NB_GO(4, 3);
+#undef NB_GO
   return true;
 }
 
@@ -247,25 +173,3 @@ template bool nb_gemm_f32_rows<float>(const float*, const float*, const float*, 
 template bool nb_gemm_f32_rows<__nv_bfloat16>(const float*, const float*, const float*, const float*,
                                               __nv_bfloat16*, int, int, int, int, cudaStream_t,
                                               cudaError_t*);
-
-// 1 where a product of fp32 rows takes the LayerNorm in front of it along (see the head of the file).
-NB_EXPORT int nb_gemm_rows_f32_norm_supported(int M, int N, int K) {
-  return M >= 1 && M <= ROWS && N >= 1 && K >= 4 && K % 4 == 0 && K <= 1024 ? 1 : 0;
-}
-
-// out = act(layernorm(X) W^T + bias) (+ residual), everything in fp32; beta may be null.
-NB_EXPORT int nb_gemm_rows_f32_norm(const float* X, const float* gamma, const float* beta, float eps, const float* W,
-                                    const float* bias, const float* residual, void* out, int out_dtype, int M,
-                                    int N, int K, int act, cudaStream_t stream) {
-  if (M == 0 || N == 0) return 0;
-  NB_REQUIRE(nb_gemm_rows_f32_norm_supported(M, N, K), NB_ERR_UNSUPPORTED,
-             "gemm_rows_f32_norm: does not take M=%d N=%d K=%d", M, N, K);
-  NB_REQUIRE((uintptr_t)X % 16 == 0 && (uintptr_t)W % 16 == 0 && (uintptr_t)gamma % 16 == 0 && (uintptr_t)beta % 16 == 0,
-             NB_ERR_UNSUPPORTED, "gemm_rows_f32_norm: rows, weights and the norm's vectors must be 16-byte aligned");
-  const RowNorm norm = {gamma, beta, eps};
-  NB_REQUIRE(out_dtype == NB_F32 || out_dtype == NB_BF16, NB_ERR_BAD_ARG, "gemm_rows_f32_norm: unknown output type %d", out_dtype);
-  if (out_dtype == NB_F32) NB_CUDA((launch_short<float, true>(X, norm, W, bias, residual, (float*)out, M, N, K, act, stream)));
-  else NB_CUDA((launch_short<__nv_bfloat16, true>(X, norm, W, bias, residual, (__nv_bfloat16*)out, M, N, K, act, stream)));
-  NB_CHECK_LAUNCH("gemm_rows_f32_norm");
-  return 0;
-}

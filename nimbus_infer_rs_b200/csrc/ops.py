@@ -421,13 +421,6 @@ class CudaBackend:
                            _ptr(w), _ptr(bias), _ptr(residual), _ptr(out), dtype_code(out.dtype), M, N,
                            K, act, self._stream())
                 return
-        # a 32-bit decode step of a few sequences: the norm inside the product
-        if norm is not None and norm[3] == torch.float32 and w.dtype == torch.float32 and x.dtype == torch.float32 \
-                and self.lib.nb_gemm_rows_f32_norm_supported(M, N, K) \
-                and all(t is None or t.data_ptr() % 16 == 0 for t in (x, w, norm[0], norm[1])):
-            self._call("nb_gemm_rows_f32_norm", _ptr(x), _ptr(norm[0]), _ptr(norm[1]), norm[2], _ptr(w), _ptr(bias),
-                       _ptr(residual), _ptr(out), dtype_code(out.dtype), M, N, K, act, self._stream())
-            return
         if skinny:
             if norm is not None and (M > FUSED_NORM_MAX_ROWS or N > FUSED_NORM_MAX_COLS
                                      or w.dtype != torch.bfloat16
