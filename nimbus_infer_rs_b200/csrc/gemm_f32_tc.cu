@@ -59,18 +59,12 @@ typedef __nv_bfloat16 bf16;
 
 constexpr int BM = 128, BK = 64;
 constexpr int STAGES = 2;                   // blocks of K in flight
+constexpr int SMALL = 8;                    // blocks of K whose small terms are added up in one place
 
 template <int BN>                           // columns of a tile
 struct Tile {
   static constexpr int XPIECE = BM * BK * 2, WPIECE = BN * BK * 2;        // bytes of the boxes
   static constexpr int BLOCK_BYTES = 3 * (XPIECE + WPIECE);               // X's three pieces, W's three pieces
-  // Two pieces of W in one instruction of twice the width, the small terms in two halves that are
-  // added up when they are taken out: fewer instructions, which pays up to 96 columns (2024x768x3072
-  // with 96 columns MEASURED_96); 256 wide they take so much longer that nothing is left of it (2024x2304x768
-  // 64 us against 47, x3072 88 against 72).
-  static constexpr bool DOUBLE = BN <= 96;
-  // blocks of K whose small terms are added up in one place: about as many terms an accumulator either way
-  static constexpr int SMALL = DOUBLE ? 8 : 4;
   static constexpr int EPI = 4 * (BN / 32);                               // warps of the epilogue
   static constexpr int THREADS = 64 + 32 * EPI;
   static constexpr int OLD = BN + 4;                                      // floats between rows of the finished tile
@@ -168,8 +162,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                    const float* __restrict__ bias, const float* residual, TOut* out, int ld, int M, int N,
                    int K, int act, int tiles_n, int run, int* err_word) {
   constexpr int XPIECE = Tile<BN>::XPIECE, WPIECE = Tile<BN>::WPIECE, BLOCK_BYTES = Tile<BN>::BLOCK_BYTES;
-  constexpr int EPI = Tile<BN>::EPI, OLD = Tile<BN>::OLD, SMALL = Tile<BN>::SMALL;
-  constexpr bool DOUBLE = Tile<BN>::DOUBLE;
+  constexpr int EPI = Tile<BN>::EPI, OLD = Tile<BN>::OLD;
   extern __shared__ unsigned char smem_dyn[];
   const uint32_t raw = smem_u32(smem_dyn);
   const uint32_t base = (raw + 1023u) & ~1023u;          // swizzle atoms are 1024 bytes
@@ -177,10 +170,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   const uint32_t bars = base + STAGES * BLOCK_BYTES;
   auto full = [&](int s, int p) { return bars + 8u * (s * 3 + p); };       // one a piece
   auto empty = [&](int s) { return bars + 8u * (3 * STAGES + s); };
-  // accumulators 0 and 1: large terms, 2 and 3 small ones, in turn; DOUBLE: 2 alone, in two halves
+  // accumulators 0 and 1: large terms, 2: small terms, in two halves
   auto acc_full = [&](int b) { return bars + 8u * (4 * STAGES + b); };
-  auto acc_empty = [&](int b) { return bars + 8u * (4 * STAGES + 4 + b); };
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_dyn + (bars - raw) + 8 * (4 * STAGES + 8));
+  auto acc_empty = [&](int b) { return bars + 8u * (4 * STAGES + 3 + b); };
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_dyn + (bars - raw) + 8 * (4 * STAGES + 6));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = (int)(blockIdx.x / tiles_n) * BM, n0 = (int)(blockIdx.x % tiles_n) * BN;
@@ -191,7 +184,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       for (int p = 0; p < 3; ++p) mbar_init(full(s, p), 1);
       mbar_init(empty(s), 1);
     }
-    for (int b = 0; b < 4; ++b) {
+    for (int b = 0; b < 3; ++b) {
       mbar_init(acc_full(b), 1);
       mbar_init(acc_empty(b), EPI);
     }
@@ -231,8 +224,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       constexpr uint32_t one = instr_desc_bf16(BM, BN), two = instr_desc_bf16(BM, 2 * BN);
       bool ok = true;
       for (int kb = 0; kb < blocks; ++kb) {
-        const int s = kb % STAGES, g = kb / SMALL, small = DOUBLE ? 2 : 2 + (g & 1);
-        const uint32_t small_phase = (uint32_t)(DOUBLE ? g : g >> 1) & 1u;
+        const int s = kb % STAGES, g = kb / SMALL;
         const bool first = kb % SMALL == 0, last = kb % SMALL == SMALL - 1 || kb + 1 == blocks;
         const uint32_t phase = (uint32_t)(kb / STAGES) & 1u;
         const uint32_t st = base + (uint32_t)(s * BLOCK_BYTES);
@@ -244,50 +236,33 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
           tc05_mma_bf16(tmem + (uint32_t)col, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc,
                         fresh ? 0u : 1u);
         };
-        // the large terms of half a block, for the epilogue to take out
-        auto large = [&](int b) {
-          if (!mbar_wait(acc_empty(b), ((uint32_t)kb & 1u) ^ 1u, abort_flag)) return false;
+        // the large terms, half a block at a time, for the epilogue to take out
+        ok = mbar_wait(full(s, 0), phase, abort_flag);
+        for (int b = 0; b < 2 && ok; ++b) {
+          ok = mbar_wait(acc_empty(b), ((uint32_t)kb & 1u) ^ 1u, abort_flag);
+          if (!ok) break;
           tc05_fence_after();
           product(one, 0, 0, 2 * b, b * 128, true);
           product(one, 0, 0, 2 * b + 1, b * 128, false);
           tc05_commit(acc_full(b));
-          return true;
-        };
-        ok = mbar_wait(full(s, 0), phase, abort_flag) && large(0);
-        if (DOUBLE) ok = ok && large(1);
-        if (first && ok) ok = mbar_wait(acc_empty(small), small_phase ^ 1u, abort_flag);
+        }
+        if (first && ok) ok = mbar_wait(acc_empty(2), ((uint32_t)g & 1u) ^ 1u, abort_flag);
         ok = ok && mbar_wait(full(s, 1), phase, abort_flag);
         if (!ok) break;
         tc05_fence_after();
-        const int at = small * 128;
 #pragma unroll
-        for (int k = 0; k < BK / 16; ++k) {
-          if constexpr (DOUBLE) {
-            product(two, 1, 0, k, at, first && k == 0);        // mh' | mm'
-          } else {
-            product(one, 0, 1, k, at, first && k == 0);
-            product(one, 1, 0, k, at, false);
-            product(one, 1, 1, k, at, false);
-          }
-        }
-        if (!DOUBLE) ok = large(1);
-        ok = ok && mbar_wait(full(s, 2), phase, abort_flag);
+        for (int k = 0; k < BK / 16; ++k) product(two, 1, 0, k, 256, first && k == 0);      // mh' | mm'
+        ok = mbar_wait(full(s, 2), phase, abort_flag);
         if (!ok) break;
         tc05_fence_after();
 #pragma unroll
         for (int k = 0; k < BK / 16; ++k) {
-          if constexpr (DOUBLE) {
-            product(two, 0, 1, k, at, false);         // hm' | hl'
-            product(two, 2, 0, k, at, false);         // lh' | lm'
-          } else {
-            product(one, 0, 2, k, at, false);
-            product(one, 2, 0, k, at, false);
-            product(one, 2, 1, k, at, false);
-          }
-          product(one, 1, 2, k, at, false);           // ml'
+          product(two, 0, 1, k, 256, false);         // hm' | hl'
+          product(two, 2, 0, k, 256, false);         // lh' | lm'
+          product(one, 1, 2, k, 256, false);         // ml'
         }
         tc05_commit(empty(s));
-        if (last) tc05_commit(acc_full(small));
+        if (last) tc05_commit(acc_full(2));
       }
     }
     __syncwarp();
@@ -305,7 +280,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       for (int q = 0; q < 2; ++q) {
         uint32_t v[16];
         tc05_ld_32x32b_x16(lanes + (uint32_t)(b * 128 + q * 16), v);
-        if (DOUBLE && b == 2) {      // the two halves are added up first: that rounds 2^-8 of the result
+        if (b == 2) {      // the two halves are added up first: that rounds 2^-8 of the result
           uint32_t w[16];
           tc05_ld_32x32b_x16(lanes + (uint32_t)(b * 128 + BN + q * 16), w);
           tc05_wait_ld();
@@ -325,7 +300,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     for (int kb = 0, left = run; kb < blocks && ok; ++kb) {
       const int g = kb / SMALL;
       ok = take_out(0, (uint32_t)kb & 1u) && take_out(1, (uint32_t)kb & 1u);
-      if (ok && (kb % SMALL == SMALL - 1 || kb + 1 == blocks)) ok = take_out(DOUBLE ? 2 : 2 + (g & 1), (uint32_t)(DOUBLE ? g : g >> 1) & 1u);
+      if (ok && (kb % SMALL == SMALL - 1 || kb + 1 == blocks)) ok = take_out(2, (uint32_t)g & 1u);
       if (--left == 0 || kb + 1 == blocks) {
         left = run;
 #pragma unroll
@@ -503,7 +478,7 @@ int launch_tiles(const float* X, const float* W, const bf16* xp, const bf16* wp,
 
 // Columns of a tile: the width with the least waves of tiles x time of a block of K in it.
 int g_force_bn = 0;
-double block_us(int bn) { return bn == 96 ? 1.53 : 1.65; }
+double block_us(int bn) { return bn == 96 ? 1.15 : 1.4; }
 double waves(long long M, long long N, int bn) {
   return ceil((double)((M + BM - 1) / BM) * (double)((N + bn - 1) / bn) / nb_device_sms());
 }
