@@ -19,10 +19,11 @@
 //     cluster barrier each CTA takes its share of the rows from all of them, 512 consecutive bytes a
 //     warp, adds in rank order (the result does not depend on timing), applies bias,
 //     activation and residual and stores 16 bytes a thread.  (Sent out instead with `st.async`, 16
-//     bytes a store, the exchange went at 8 bytes a clock and SM: SLOW_FIGURES)
+//     bytes a store, the exchange went at 8 bytes a clock and SM: 64x2304x1600 15.2 us for 7.2 now,
+//     64x768x3072 8.5 for 6.2, 128x1600x6400 18.3 for 11.4)
 // Warp 0 issues the TMA loads (128 x 64 boxes of W, rows x 64 boxes of X, 128-byte
-// swizzled) into a ring of stages of 104 KB at most, so that a CTA of the next launch fits beside it; the
-// weights of the first stages are asked for before the wait on the kernel in front (they are
+// swizzled) into a ring of stages of 200 KB at most (a block of cold weights is 1.5 us away: 128x1600x6400
+// 13.4 us with 104 KB); the weights of the first stages are asked for before the wait on the kernel in front (they are
 // constants).  Warp 1 owns the tensor memory and issues the MMAs.  Warps 2 to 9 are the epilogue, two per
 // quarter of the lanes.
 //
@@ -375,9 +376,8 @@ NB_EXPORT int nb_gemm_tc_rows_supported(int M, int N, int K) {
 
 // 1 where this kernel is the faster one of the two tensor-core products (measured on a B200 at
 // 32, 64 and 128 rows on GPT-2 124M's and XL's shapes): a long K (24 blocks and more) over
-// few columns, where the tiled kernel has few CTAs and each a long walk.  Elsewhere the
-// exchange between the CTAs of a cluster (about 8 bytes a clock and SM) costs more than the
-// shorter walk saves.
+// few columns, where the tiled kernel has few CTAs and each a long walk.  (Measured with the exchange
+// that this kernel had first; with the present one 64x4800x1600 takes 9.7 us, the tiled kernel 9.0.)
 NB_EXPORT int nb_gemm_tc_rows_preferred(int M, int N, int K) {
   RowsShape sh;
   if (!plan_rows(M, N, K, &sh)) return 0;
