@@ -18,6 +18,13 @@ def ops():
     return ops_mod.backend()
 
 
+@pytest.fixture(autouse=True)
+def own_random_numbers():
+    """What is drawn here moves no other test's numbers."""
+    with torch.random.fork_rng():
+        yield
+
+
 @pytest.mark.parametrize("width, pair", [(96, 1), (128, 1), (192, 1), (256, 1), (96, 0), (128, 0)])
 @pytest.mark.parametrize("M, N, K", [(129, 260, 8), (257, 1600, 136), (511, 52, 640), (2900, 516, 72)])
 def test_tiles_of_every_width_with_32_bit_results(ops, width, pair, M, N, K):
