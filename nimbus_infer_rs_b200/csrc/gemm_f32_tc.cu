@@ -478,7 +478,7 @@ int launch_tiles(const float* X, const float* W, const bf16* xp, const bf16* wp,
 
 // Columns of a tile: the width with the least waves of tiles x time of a block of K in it.
 int g_force_bn = 0;
-double block_us(int bn) { return bn == 96 ? 1.53 : 1.65; }
+double block_us(int bn) { return bn == 96 ? 1.15 : 1.4; }
 double waves(long long M, long long N, int bn) {
   return ceil((double)((M + BM - 1) / BM) * (double)((N + bn - 1) / bn) / nb_device_sms());
 }

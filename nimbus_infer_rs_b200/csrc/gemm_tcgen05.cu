@@ -57,7 +57,6 @@ __host__ __device__ constexpr int cta_threads(int bn, int epi) { return 96 + 32 
 // the next tile's products, and the 64 KB it saves are two stages of the ring.
 // PAIR 1: two CTAs of a cluster share 256 x BN tiles (`cta_group::2`): each brings its 128
 // rows of X and half of the tile's rows of W, so a stage holds BN / 2 rows of W.
-constexpr int TURN_LD = 33;      // floats between rows of such a block: neither way meets in a bank
 template <int BN, int EPI, int ESIZE, int PAIR>
 struct SmemLayout {
   static constexpr int A_BYTES = BM * BK * 2;
@@ -66,8 +65,7 @@ struct SmemLayout {
   static constexpr int EPI_WARPS = epi_warps(BN, EPI);
   // fp32 tiles wider than 128 columns: one 32-column box a warp, used twice a tile
   static constexpr int BOXES = ESIZE == 4 && BN <= 128 ? 2 : 1;
-  // direct stores: a 32 x 32 block of fp32 sums, turned over on its way out
-  static constexpr int STG_PER_WARP = EPI ? BOXES * 4096 : 32 * TURN_LD * 4;
+  static constexpr int STG_PER_WARP = EPI ? BOXES * 4096 : 0;
   static constexpr int STG_BYTES = EPI_WARPS * STG_PER_WARP;
   static constexpr int BUDGET = 222 * 1024;   // of the 227 KB a CTA may have
   static constexpr int STAGES_RAW = (BUDGET - STG_BYTES) / STAGE_BYTES;
@@ -501,7 +499,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     const int quarter = warp & 3;   // the 32 tensor-memory lanes this warp may read
     const int half = (warp - 2) >> 2;   // which share of the tile's columns it takes
     constexpr int CHUNKS = BN / 32 / (EW / 4);   // 32-column chunks per warp
-    float* turn = reinterpret_cast<float*>(gen + L::TILES_BYTES + (warp - 2) * L::STG_PER_WARP);
     uint32_t t = 0;
     if (dual) {   // the second issuing thread, before its warp turns to the epilogue
       if (warp == 2 && lane == 0) dual_walk(1);
@@ -549,44 +546,47 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 #pragma unroll
         for (int q = 1; q < CHUNKS; ++q)
           if (c - half * CHUNKS == q) bias_l = bias_pre[q];
-        if (m0 + quarter * 32 >= M) continue;         // a short last tile: nothing to store
         // The accumulator comes with a lane per row and a register per column; stored that way
         // a warp's instruction would touch 32 rows, four bytes each.  The 32 x 32 block is
-        // turned over through shared memory, after which lane l holds column l and register i row i: an
-        // instruction then writes 32 consecutive columns of one row, whatever the width of the output
-        // (the logits' 50,257 columns are no multiple of anything).  (Turned over by five rounds of
-        // exchanges across the warp a tile took its warps some 1,300 instructions a block and 16
-        // clocks each, which bounded the output head: HEAD_FIGURES)
+        // transposed across the warp (five rounds of exchanges between lanes 16, 8, 4, 2, 1
+        // apart), after which lane l holds column l and register i row i: an instruction then
+        // writes 32 consecutive columns of one row, whatever the width of the output (the
+        // logits' 50,257 columns are no multiple of anything).
         float f[32];
-        __syncwarp();                                 // the block before this one has been read
 #pragma unroll
-        for (int j = 0; j < 32; ++j) turn[lane * TURN_LD + j] = __uint_as_float(v[j]);
-        __syncwarp();
+        for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) f[i] = turn[i * TURN_LD + lane];
+        for (int s2 = 16; s2 >= 1; s2 >>= 1) {
+          const bool upper = (lane & s2) != 0;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            if (j & s2) continue;
+            const float send = upper ? f[j] : f[j + s2];
+            const float got = __shfl_xor_sync(0xffffffffu, send, s2);
+            if (upper) f[j] = got; else f[j + s2] = got;
+          }
+        }
         const int col = nb + lane;
         const int row0 = m0 + quarter * 32;
         if (col < N) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) f[i] += bias_l;
           nb_apply_act_fast_all(f, act);
-          if (residual)                       // may be `out` itself: all of it before the first store
+          float rs[32];   // `residual` may be `out` itself: all of it before the first store
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (row0 + i < M) f[i] += residual[(size_t)(row0 + i) * N + col];
-          TOut* to = out + (size_t)row0 * N + col;
-          if (row0 + 32 <= M) {
+          for (int i = 0; i < 32; ++i)
+            rs[i] = (residual && row0 + i < M) ? residual[(size_t)(row0 + i) * N + col] : 0.0f;
 #pragma unroll
-            for (int i = 0; i < 32; ++i) to[(size_t)i * N] = nb_from_f32<TOut>(f[i]);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (row0 + i < M) to[(size_t)i * N] = nb_from_f32<TOut>(f[i]);
+          for (int i = 0; i < 32; ++i) {
+            if (row0 + i >= M) break;
+            const float y = f[i] + rs[i];
+            if constexpr (sizeof(TOut) == 4) reinterpret_cast<float*>(out)[(size_t)(row0 + i) * N + col] = y;
+            else reinterpret_cast<bf16*>(out)[(size_t)(row0 + i) * N + col] = __float2bfloat16_rn(y);
           }
         }
-        __syncwarp();
       }
     }
+  
   }
 
   tc05_fence_before();
