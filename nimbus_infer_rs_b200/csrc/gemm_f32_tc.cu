@@ -13,7 +13,7 @@
 // instruction (16 of K) cuts its sum instead of rounding it, so that errors of one sign pile up in an
 // accumulator that is left alone (over 6,400 numbers of one sign 8.0e-7 of the result, where
 // multiply-adds have 0.9e-7).  So the large terms hh' are taken out of tensor memory every 32 of K, and
-// the small ones, in which the same error counts 2^-8 as much or less, every 256; both are
+// the small ones, in which the same error counts 2^-8 as much or less, every 512; both are
 // added up in registers, rounded, in runs of about sqrt(K / 64) blocks whose sums are added up in turn
 // (one chain of K / 32 additions would round as often as the multiply-adds do).
 //
@@ -37,14 +37,19 @@
 // (Cut in parts, over so few tiles that they are the faster ones, multiply-adds come nearer: numbers
 // of one sign at K = 128 in two parts 5.4.)
 //
-// A CTA takes a 128 x 128 tile.  A block of 64 of K takes 3,200 clocks: its 32 instructions read 256 KB of
-// operands out of shared memory and its loads write 96 KB there, 2,800 clocks at 128 bytes a
-// clock.  (With six products, ml' and lm' left out, and the large terms taken out every 128 of K it took
-// 2,800: 2024x2304x768 55 us against 60, 2024x768x3072 94 against 115.  Large terms taken out every 16 of K
-// by eight warps: 84 and 151.)
+// A CTA takes a tile of 128 rows and 128 columns, or 96 where that takes no more waves of tiles.  What
+// bounds a block of 64 of K is the shared memory that its instructions read their operands from and its
+// loads write to, and the instructions' number: W's neighbouring pieces lie behind one another and are
+// taken as one operand of twice the width, hm' beside hl', mh' beside mm', lh' beside lm', into two halves
+// of the small terms' accumulator, which are added up when they are taken out: 20 instructions a block
+// that read 208 KB, where one at a time took 32 and 256 KB (us, split_kernel included, now and then:
+// 2024x2304x768 57 and 63, 2024x3072x768 82 and 88; with 96 columns 2024x768x768 28 and 35, 2024x768x3072 85 and
+// 115).  (With six products, ml' and lm' left out, and the large terms taken out every 128 of K, one piece
+// at a time: 2024x2304x768 55, 2024x768x3072 94.  Large terms taken out every 16 of K by eight warps:
+// 2024x768x3072 151.)
 // Warp 0 brings the pieces of 64 columns of K by TMA (six 128 x 64
-// boxes a block, two blocks in flight), warp 1 issues the MMAs, sixteen warps take the
-// accumulators (two for the large terms, two for the small) out and finish the tile through shared
+// boxes a block, two blocks in flight), warp 1 issues the MMAs, sixteen or twelve warps take the
+// accumulators (two for the large terms, one in two halves for the small) out and finish the tile through shared
 // memory.  Every wait has a clock budget.
 //
 // Reference analogue: Mat::gemm_into (src/model.rs:88-133).
@@ -478,7 +483,7 @@ int launch_tiles(const float* X, const float* W, const bf16* xp, const bf16* wp,
 
 // Columns of a tile: the width with the least waves of tiles x time of a block of K in it.
 int g_force_bn = 0;
-double block_us(int bn) { return bn == 96 ? 1.15 : 1.4; }
+double block_us(int bn) { return bn == 96 ? 1.53 : 1.65; }
 double waves(long long M, long long N, int bn) {
   return ceil((double)((M + BM - 1) / BM) * (double)((N + bn - 1) / bn) / nb_device_sms());
 }
@@ -533,7 +538,7 @@ NB_EXPORT int nb_gemm_f32_tc_supported(int M, int N, int K) {
 // block of 16 of its part of K 1.03 up to 1.75 CTAs an SM, 1.8 up to 3.5, and beyond 0.46 a CTA and SM,
 // or 0.62 where K is cut (clusters leave SMs out); where it leaves K of under 256 to gemm_simt.cu that
 // one's 4 and 0.045 a number of K.  Measured, this kernel and the other:
-// 2024x2304x768 60 and 173, 2024x3072x768 85 and 251, 2024x768x3072 115 and 320, 1000x768x768 30 and 49,
+// 2024x2304x768 57 and 173, 2024x3072x768 82 and 251, 2024x768x3072 85 and 320, 1000x768x768 30 and 49,
 // 333x2304x768 31 and 48, 200x2304x768 31 and 40, 66x50257x768 155 and 243, 128x4800x1600 70 and 92; but
 // 512x768x768 29 and 26.5, 333x768x768 29 and 23, 997x512x512 23 and 21, 300x1600x6400 202 and 190,
 // 128x768x3072 93 and 30.  Not below 128 of K, where gemm_simt.cu's tiles take as long as a wave here or
