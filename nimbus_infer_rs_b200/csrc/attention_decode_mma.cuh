@@ -70,7 +70,7 @@ attention_decode_mma_kernel(const __nv_bfloat16* q, int q_stride, int q_col,
   constexpr int NT = NW * 32;          // threads
   constexpr int PPI = NW > 4 ? NW / 4 : 1;   // pages per turn of the loop
   constexpr int QPW = NW < 4 ? 4 / NW : 1;   // quarters of a page a warp takes
-  static_assert((NW == 1 || NW == 2 || NW == 4 || NW == 8) && MMA_STAGES % PPI == 0, "one to eight warps");
+  static_assert((NW == 2 || NW == 4 || NW == 8) && MMA_STAGES % PPI == 0, "two, four or eight warps");
   const int dk = MIXED ? kv.head_dim : HD, dv = MIXED ? kv.value_dim : HD;
   const int KTILE = PAGE_TOKENS * dk, VTILE = PAGE_TOKENS * dv;    // elements of one page of one head
   constexpr int STILE = PAGE_TOKENS * ROW;
@@ -262,7 +262,7 @@ attention_decode_mma_kernel(const __nv_bfloat16* q, int q_stride, int q_col,
     const int p = p0 + po;                            // this warp's page
     bf16* kt = tiles + (size_t)(stage + po) * 2 * STILE;
     bf16* vt = kt + STILE;
-    const int key0 = p * PAGE_TOKENS + wq * 16;       // first key of this warp's 16 (or 32, 64)
+    const int key0 = p * PAGE_TOKENS + wq * 16;       // first key of this warp's 16 (or 32)
     if (p < p_end && key0 < kv_len && (key0 + QPW * 16 > j_begin || key0 < keep_first)) {   // warp-uniform: something to attend to
       float sc[QPW][4];
 #pragma unroll
@@ -597,12 +597,12 @@ int launch_mma(const void* q, int q_stride, int q_col, const int* row_slot, cons
     // Heads of 64: four warps and two pages where splits share a sequence or the CTAs are few (us, one
     // sequence of 900 tokens x 12 heads in eight splits 3.5, with eight warps and four pages 3.9; 4 x 450 tokens
     // 4.7 and 5.2); whole sequences in so many CTAs that latencies overlap among them by
-    // two warps with 32 keys each and, where that puts all of them on the GPU, one page (64
-    // sequences of 97 to 152 tokens x 25 heads 13.1, with two pages 16.0, with four warps 16.2; x 12 heads
-    // 9.5, 9.0 and 9.3; of 500 to 1,000 tokens x 25 heads 54.1, 53.4 and 52.9).
+    // two warps with 32 keys each (us; x 25 heads: 64 sequences of 1,000 tokens 66.9, with four warps 67.6, of
+    // 97 to 152 tokens 15.4 and 15.7, 36 of 128 to 1,024 tokens 29.6 and 30.4).  Not by two warps and one
+    // page, though all CTAs are on the GPU at once that way: 64 short sequences 13.0, but 64 long ones 70.0 and
+    // the 36 unequal ones 38.3, and a launch does not know how long its sequences are.
     if (n_splits > 1 || ctas <= 4LL * sms) NB_GO(2, 4);
-    if (ctas <= 6LL * sms) NB_GO(2, 2);
-    NB_GO(1, 2);
+    NB_GO(2, 2);
   } else {
     if (ctas <= per_sm * sms) NB_GO(4, 8);
     NB_GO(2, 4);

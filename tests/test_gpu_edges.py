@@ -136,3 +136,43 @@ def test_a_session_that_runs_ahead_of_the_device(tmp_path):
         session.close()
         for s in slots:
             engine.free_slot(s)
+
+
+@pytest.mark.parametrize("rows, H, Hk", [(50, 12, 12), (74, 12, 12), (64, 25, 25), (60, 24, 12)])
+@pytest.mark.parametrize("window", [0, 70])
+@pytest.mark.parametrize("append", [False, True])
+def test_decode_attention_of_large_batches_over_heads_of_64(ops, rows, H, Hk, window, append):
+    """Whole sequences in more than four CTAs an SM (two warps, 32 keys each), below and beyond what is on
+    the GPU at once: lengths around a page's end and of one to six pages, a padding row, NaN in every row of
+    a page that holds no key, the step's own keys and values from its rows or from the cache.  Off by at
+    most the rounding of probabilities and results to 8 bits: 2^-9 of the largest value and of the
+    result."""
+    hd, dtype = 64, torch.bfloat16
+    lens = [(1, 63, 64, 65, 129, 200, 333, 128)[i % 8] for i in range(rows)]
+    kv, dk, dv = _paged_cache(rows, lens, Hk, hd, dtype, seed=rows + H, stale_nan=True)
+    lay = build_layout([(s + 1, [0], []) for s in range(rows)], [n - 1 for n in lens], DEV)
+    lay.row_slot[2] = -1
+    torch.manual_seed(8)
+    qkv = torch.randn(rows, (H + 2 * Hk) * hd, device=DEV).to(dtype)
+    pages = kv.block_table[torch.arange(1, rows + 1, device=DEV), torch.tensor([(n - 1) // 64 for n in lens], device=DEV)].long()
+    at = torch.tensor([(n - 1) % 64 for n in lens], device=DEV)
+    if append:
+        own = [t.view(rows, Hk, hd) for t in (qkv[:, H * hd:(H + Hk) * hd], qkv[:, (H + Hk) * hd:])]
+        for dense, mine, plane in zip((dk, dv), own, (kv.k, kv.v)):
+            plane[pages, :, at] = float("nan")
+            for s in range(rows):
+                dense[s][-1] = mine[s].cpu()
+    out = torch.full((rows, H * hd), 7.0, device=DEV, dtype=dtype)
+    scale = 0.5 / math.sqrt(hd)
+    ops.attention(qkv, 0, lay, kv, H, out, scale, window, append=(H * hd, (H + Hk) * hd) if append else None)
+    for s, n in enumerate(lens):
+        if s == 2:
+            assert (out[s] == 0).all()
+            continue
+        ref = _attention_ref(qkv[s, :H * hd].view(H, hd).cpu(), dk[s], dv[s], n - 1, scale, H // Hk, window)
+        err = (out[s].view(H, hd).double().cpu() - ref).abs().max()
+        assert err <= 2.0 ** -9 * float(dv[s].double().abs().max() + ref.abs().max()) + 1e-4, s
+    if append:      # the cache holds them now; the padding row has written nothing
+        live = [s for s in range(rows) if s != 2]
+        for mine, plane in zip(own, (kv.k, kv.v)):
+            assert torch.equal(plane[pages, :, at][live], mine[live]) and plane[pages, :, at][2].isnan().all()
