@@ -176,3 +176,25 @@ def test_decode_attention_of_large_batches_over_heads_of_64(ops, rows, H, Hk, wi
         live = [s for s in range(rows) if s != 2]
         for mine, plane in zip(own, (kv.k, kv.v)):
             assert torch.equal(plane[pages, :, at][live], mine[live]) and plane[pages, :, at][2].isnan().all()
+
+
+@pytest.mark.parametrize("rows, H, Hk, longest", [(2, 2, 2, 1530), (3, 16, 4, 1100), (40, 16, 4, 330), (9, 16, 2, 700),
+                                                  (5, 8, 1, 961), (12, 12, 6, 577)])
+def test_decode_attention_of_small_batches_over_heads_of_64(ops, rows, H, Hk, longest):
+    """Splits by eight warps (shared key heads in up to a CTA an SM; more than two pages a split) and by
+    four, over one long sequence among short ones, an odd number of pages, and a split whose pages lie beyond
+    most sequences.  Bound as above."""
+    hd, dtype = 64, torch.bfloat16
+    lens = [longest if s == rows // 2 else (1, 65, 130, 64, 257)[s % 5] for s in range(rows)]
+    kv, dk, dv = _paged_cache(rows, lens, Hk, hd, dtype, seed=rows + H, stale_nan=True)
+    lay = build_layout([(s + 1, [0], []) for s in range(rows)], [n - 1 for n in lens], DEV)
+    lay.max_kv_len = longest
+    torch.manual_seed(8)
+    q = torch.randn(rows, H * hd, device=DEV).to(dtype)
+    out = torch.full((rows, H * hd), 7.0, device=DEV, dtype=dtype)
+    scale = 0.5 / math.sqrt(hd)
+    ops.attention(q, 0, lay, kv, H, out, scale)
+    for s, n in enumerate(lens):
+        ref = _attention_ref(q[s].view(H, hd).cpu(), dk[s], dv[s], n - 1, scale, H // Hk)
+        err = (out[s].view(H, hd).double().cpu() - ref).abs().max()
+        assert err <= 2.0 ** -9 * float(dv[s].double().abs().max() + ref.abs().max()) + 1e-4, s
