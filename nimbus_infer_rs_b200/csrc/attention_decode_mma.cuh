@@ -601,13 +601,14 @@ int launch_mma(const void* q, int q_stride, int q_col, const int* row_slot, cons
     // 97 to 152 tokens 15.4 and 15.7, 36 of 128 to 1,024 tokens 29.6 and 30.4).  Not by two warps and one
     // page, though all CTAs are on the GPU at once that way: 64 short sequences 13.0, but 64 long ones 70.0 and
     // the 36 unequal ones 38.3, and a launch does not know how long its sequences are.
-    // Eight warps and four pages stay for up to a CTA an SM where query heads share a key head, since
-    // merging takes group times as long and eight warps halve it (us; 4 key heads of 4 query heads: one
-    // sequence of 2,048 tokens in eight splits 4.4 and, with four warps, 6.0; 4 of 1,024 tokens in
-    // eight 4.6 and 5.8, 8 in four 5.2 and 6.5), and for eight splits of more than two pages each (12
-    // heads, one sequence of 2,048 tokens 4.4 and 5.5; 25 heads 6.3 and 7.2).
+    // Eight warps and four pages stay for up to a CTA an SM (1.3 from four query heads to a key head on) where
+    // query heads share a key head, since merging takes group times as long and eight warps halve it
+    // (us; 4 key heads of 4 query heads: one sequence of 2,048 tokens in eight splits 4.4 and, with four warps,
+    // 6.0; 4 of 1,024 tokens in eight 4.6 and 5.8, 8 in six 6.3 and 6.3, but of 576 in eight 6.5 and 7.4), and
+    // for eight splits of more than two pages each (12 heads, one sequence of 2,048 tokens 4.4 and 5.5; 25
+    // heads 6.3 and 7.2).
     const bool long_runs = n_splits == MAX_CLUSTER && kv.max_pages > 2 * MAX_CLUSTER;
-    if (group > 1 ? ctas <= sms : long_runs && 5 * ctas <= 7LL * sms) NB_GO(4, 8);
+    if (group > 1 ? 10 * ctas <= (group > 2 ? 13LL : 10LL) * sms : long_runs && 5 * ctas <= 7LL * sms) NB_GO(4, 8);
     if (n_splits > 1 || ctas <= 4LL * sms) NB_GO(2, 4);
     NB_GO(2, 2);
   } else {
