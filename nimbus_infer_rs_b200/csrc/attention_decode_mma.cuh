@@ -605,10 +605,10 @@ int launch_mma(const void* q, int q_stride, int q_col, const int* row_slot, cons
     // query heads share a key head, since merging takes group times as long and eight warps halve it
     // (us; 4 key heads of 4 query heads: one sequence of 2,048 tokens in eight splits 4.4 and, with four warps,
     // 6.0; 4 of 1,024 tokens in eight 4.6 and 5.8, 8 in six 6.3 and 6.3, but of 576 in eight 6.5 and 7.4), and
-    // for eight splits of more than two pages each (12 heads, one sequence of 2,048 tokens 4.4 and 5.5; 25
-    // heads 6.3 and 7.2).
+    // for up to a CTA an SM in eight splits of more than two pages each (12 heads, one sequence of 2,048 tokens
+    // 4.4 and 5.5; two unequal ones, 192 CTAs, 4.9 and 3.9).
     const bool long_runs = n_splits == MAX_CLUSTER && kv.max_pages > 2 * MAX_CLUSTER;
-    if (group > 1 ? 10 * ctas <= (group > 2 ? 13LL : 10LL) * sms : long_runs && 5 * ctas <= 7LL * sms) NB_GO(4, 8);
+    if ((group > 1 || long_runs) && 10 * ctas <= (group > 2 ? 13LL : 10LL) * sms) NB_GO(4, 8);
     if (n_splits > 1 || ctas <= 4LL * sms) NB_GO(2, 4);
     NB_GO(2, 2);
   } else {
