@@ -41,6 +41,11 @@ ROWS_MAX_ROWS = 128    # up to this many rows a product's weights are the tensor
 MOE_TC_MIN_PLACES = 1024   # from this many (token, choice) pairs on the experts' products take tcgen05 tiles
 
 
+def fewest_splits(pages: int, splits: int) -> int:
+    """The smallest count whose longest split is no longer than with ``splits`` of them."""
+    return -(-pages // -(-pages // splits))
+
+
 def decode_splits(base_ctas: int, pages: int, page: int, head_dim: int, sms: int, most: int) -> int:
     """Splits of a sequence's pages in the tensor-core decode attention (swept on a B200 at
     contexts of 256 and 1,024 and batches of 1 to 32).  Four pages a split: eight warps take
@@ -62,16 +67,23 @@ def decode_splits(base_ctas: int, pages: int, page: int, head_dim: int, sms: int
     return s
 
 
-def decode_splits_64(base_ctas: int, pages: int, sms: int, most: int) -> int:
-    """The same for heads of 64 (four warps and two pages a CTA, six CTAs an SM): the most splits that
-    deal the pages out evenly and leave the launch at four CTAs an SM, or two splits where that
-    fills it to six (us; 12 heads, 16 pages: one sequence in 8 splits 3.5, in 4 4.0; 4 sequences 4.7 and
-    5.0; 8 in 4 8.1, in 8 over 8.9; 24 in 2 10.8, whole 12.3; 32 in 2 11.5, whole 13.2; 25 heads: 16 in 2
-    8.4, whole 9.8; 24 in 2 19.3, whole 18.7)."""
-    for s in (8, 4, 2):
-        if s <= most and pages % s == 0 and s * base_ctas <= (4 if s > 2 else 6) * sms:
-            return s
-    return 1
+def decode_splits_64(base_ctas: int, pages: int, group: int, sms: int, most: int) -> int:
+    """The same for heads of 64, ``group`` query heads to a key head.  What a launch takes goes with the
+    pages that a split walks over and, once the GPU is full, with its CTAs: of the counts that leave the
+    launch at 4.4 CTAs an SM, or two splits at 6, the one with the shortest walk, and of those the smallest.
+    Shared key heads merge ``group`` times as much: 1.3 CTAs an SM in more than five splits, 3 in three to
+    five, 4 in two.  (us, 12 heads: one sequence of 9 pages in 5 splits 3.4, whole 8.8, of 15 in 8 3.6,
+    whole 12.9, of 33 in 7 6.2, whole 25.6; 8 sequences of 9 in 5 5.4, in 8 9.8, whole 10.2, of 16 in 6 7.7,
+    in 4 7.6, in 8 10.4; 32 of 16 in 2 20.7, whole 22.6, of 5 in 2 10.1, whole 9.1; 25 heads, 16 of 9 in 2
+    13.2, whole 18.0, 24 of 16 in 2 33.1, whole 29.9; 16 heads over 4 key heads, 8 of 16 in 6 6.3, in 8 7.4,
+    whole 14.1.  Over 600 launches of 1 to 96 sequences of 2 to 33 pages, equal and unequal, 1.5 to 4 %
+    above the fastest count.)"""
+    def room(s):      # tenths of a CTA an SM
+        if group > 1:
+            return 13 if s > 5 else 30 if s > 2 else 40
+        return 44 if s > 2 else 60
+    s = next((s for s in range(min(most, pages), 1, -1) if 10 * s * base_ctas <= room(s) * sms), 1)
+    return fewest_splits(pages, s)
 
 
 def decode_splits_f32(base_ctas: int, pages: int, page: int, head_dim: int, sms: int, cluster: int) -> int:
@@ -514,15 +526,15 @@ class CudaBackend:
         return int(status.item())
 
     # -- cache and attention ----------------------------------------------------------
-    def _decode_splits(self, base_ctas: int, pages: int, kv, dtype) -> int:
+    def _decode_splits(self, base_ctas: int, pages: int, kv, dtype, group: int) -> int:
         """Into how many splits a decode launch cuts each sequence's pages (`base_ctas`: rows x
-        key-value heads): `decode_splits_f32` and, on the tensor cores, `decode_splits_64` or
-        `decode_splits`."""
+        key-value heads; `group`: query heads to each of these): `decode_splits_f32` and, on the tensor
+        cores, `decode_splits_64` or `decode_splits`."""
         if dtype != torch.bfloat16:
             return decode_splits_f32(base_ctas, pages, kv.page, kv.head_dim, self._sms,
                                      self._cluster_limit if self.decode_clusters else 0)
         if kv.head_dim == 64 and self.decode_clusters:
-            return decode_splits_64(base_ctas, pages, self._sms, self._cluster_limit)
+            return decode_splits_64(base_ctas, pages, group, self._sms, self._cluster_limit)
         return decode_splits(base_ctas, pages, kv.page, kv.head_dim, self._sms,
                              self._cluster_limit if self.decode_clusters else 16)
 
@@ -604,7 +616,8 @@ class CudaBackend:
                 dtype_code(q_src.dtype), kv.head_dim, n_heads,
                 kv.n_kv_heads, kv.page):
             pages = max(1, -(-layout.max_kv_len // kv.page))
-            n_splits = self._decode_splits(n_rows * kv.n_kv_heads, pages, kv, q_src.dtype)
+            n_splits = self._decode_splits(n_rows * kv.n_kv_heads, pages, kv, q_src.dtype,
+                                           n_heads // kv.n_kv_heads)
             acc, ml, counters = self._decode_scratch(q_src.device, n_rows, n_heads, kv.n_kv_heads,
                                                      kv.head_dim, n_splits)
             if capped:
@@ -916,7 +929,8 @@ class CudaBackend:
             pages = max(1, -(-layout.max_kv_len // k_store.page))
             if look_back > 0:
                 pages = min(pages, (look_back + k_store.page - 1) // k_store.page + 1)
-            n_splits = self._decode_splits(n * k_store.n_kv_heads, pages, k_store, q.dtype) + (1 if keeps else 0)
+            n_splits = self._decode_splits(n * k_store.n_kv_heads, pages, k_store, q.dtype,
+                                           n_heads // k_store.n_kv_heads) + (1 if keeps else 0)
             acc, ml, counters = self._decode_scratch(q.device, n, n_heads, k_store.n_kv_heads, d, n_splits)
             self._call("nb_attention_decode_capped", _ptr(q), code, q.shape[1], 0,
                        _ptr(layout.row_slot), _ptr(layout.row_pos), _ptr(k_store.k), _ptr(k_store.v),
@@ -1033,7 +1047,7 @@ class CudaBackend:
             pages = max(1, -(-layout.max_kv_len // page))
             if window > 0:
                 pages = min(pages, (window + page - 1) // page + 1)
-            n_splits = self._decode_splits(n * G, pages, k_store, q.dtype)
+            n_splits = self._decode_splits(n * G, pages, k_store, q.dtype, 2 * n_heads // G)
             acc, ml, counters = self._decode_scratch(q.device, n, 2 * n_heads, G, d2, n_splits)
             self._call("nb_attention_decode_maps", _ptr(q), q.shape[1], _ptr(layout.row_slot),
                        _ptr(layout.row_pos), _ptr(k_store.k), _ptr(v_plane), _ptr(k_store.block_table),

@@ -196,9 +196,9 @@ def test_a_preset_name_builds_a_model_with_no_file_on_disk(cpu_backend):
 
 
 def test_splits_of_the_decode_attention():
-    """How many CTAs share a sequence's pages (GPT-2 small's 12 heads of 64, a B200's 148 SMs,
-    pages of 64 tokens): the rule's answers where a sweep on the GPU gave the best or nearly
-    the best count."""
+    """How many CTAs share a sequence's pages (12 heads of 64, a B200's 148 SMs, pages of 64
+    tokens): the rule's answers where a sweep on the GPU gave the best or nearly the best count.
+    The launches it decides are those of other head sizes, and of heads of 64 without clusters."""
     from nimbus_infer_rs_b200.csrc.ops import decode_splits
 
     def s(batch, pages, heads=12, most=8):
@@ -213,6 +213,33 @@ def test_splits_of_the_decode_attention():
     assert s(8, 16, heads=16) == 4 and s(12, 16, heads=16) == 2
     # without clusters up to 16 splits
     assert s(1, 64, most=16) == 16 and s(1, 64) == 8
+
+
+def test_splits_of_the_decode_attention_over_heads_of_64():
+    """Any number of pages, odd ones (every window of whole even pages) and primes among them: one
+    more page never shortens the longest split and adds at most a page to it, no split is
+    empty, and a launch with room on the GPU is cut."""
+    from nimbus_infer_rs_b200.csrc.ops import decode_splits_64
+
+    def s(batch, pages, heads=12, group=1, most=8):
+        return decode_splits_64(batch * heads, pages, group, 148, most)
+    assert [s(1, p) for p in (1, 2, 3, 5, 9, 15, 16, 17, 31, 33)] == [1, 2, 3, 5, 5, 8, 8, 6, 8, 7]
+    assert [s(8, p) for p in (9, 15, 16, 17, 33)] == [5, 5, 6, 6, 6]
+    assert [s(b, 16) for b in (1, 4, 8, 16, 32, 64)] == [8, 8, 6, 3, 2, 1]
+    # 16 heads over 4 key heads, windows of 512 (9 pages) and blocks of 2,048 positions (33)
+    assert [s(b, 9, 4, 4) for b in (1, 4, 8, 16, 32)] == [5, 5, 5, 5, 3]
+    assert [s(b, 33, 4, 4) for b in (1, 4, 8, 16, 32)] == [7, 7, 6, 5, 3]
+    assert s(1, 33, most=4) == 4 and s(1, 1) == 1 and s(200, 16) == 1
+    for group in (1, 2, 8):
+        for base in (1, 4, 12, 25, 60, 96, 192, 300, 444, 445, 900):
+            walk = 0
+            for pages in range(1, 70):
+                n = decode_splits_64(base, pages, group, 148, 8)
+                now = -(-pages // n)
+                assert 1 <= n <= min(8, pages) and walk <= now <= walk + 1
+                assert (n - 1) * now < pages                      # the last split has a page
+                assert n > 1 or pages == 1 or 2 * base > (6 if group == 1 else 4) * 148
+                walk = now
 
 
 def test_every_row_of_a_packed_step_says_where_it_belongs():
