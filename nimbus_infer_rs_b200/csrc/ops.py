@@ -87,19 +87,27 @@ def decode_splits_64(base_ctas: int, pages: int, group: int, sms: int, most: int
 
 
 def decode_splits_f32(base_ctas: int, pages: int, page: int, head_dim: int, sms: int, cluster: int) -> int:
-    """Splits of a sequence's pages in the 32-bit decode attention: as many as put one launch on the
-    GPU at once (a CTA keeps two pages of keys and values, 64 KB with heads of 64).  What merges inside
-    a cluster (up to `cluster` splits, 0: none do) deals the pages out evenly, and is preferred unless
-    a split would then walk over more than four pages (us; 12 heads of 64, 16 pages: one sequence in 8
-    splits 5.0, in 16 7.1; 5 sequences in 4 7.8, in 7 8.9; 8 in 4 12.3, in 3 13.9; 24 in 2, a third more than
-    fit, 20.5, whole 23.4; 32 in 2 24.1, whole 23.7)."""
+    """Splits of a sequence's pages in the 32-bit decode attention.  A CTA keeps two pages of keys and
+    values (64 KB with heads of 64), and a launch that does not fit on the GPU at once takes twice as long:
+    of up to `cluster` splits, which merge inside a cluster (0: none do), the shortest walk that
+    leaves the launch at nine tenths of what fits, at three quarters in more than six (clusters of seven
+    and eight leave SMs out), at all of it in two.  Where a split would walk over more than five
+    pages, as many as fit, merged through scratch memory.  (us, 12 heads of 64: one sequence of 9 pages in 5
+    splits 5.8, in 9 6.6, whole 13.2, of 15 in 8 6.4, in 15 8.3, of 16 in 8 6.3, in 16 7.7; 4 of 16 in 6 9.6,
+    in 8 11.4; 5 of 16 in 6 10.1, in 7 15.9; 8 of 9 in 3 9.9, in 6 13.5, of 16 in 4 12.8, in 5 20.1; 12 of 16
+    in 2 19.1, in 3 24.9, whole 26.9; 24 of 16 in 2 39.0, whole 34.0; 8 heads of 128: one of 31 in 16 12.5,
+    in 8 14.5, two in 9 17.2, in 6 20.1, in 8 27.1.)"""
     room = max(1, min(8, (228 * 1024) // (4 * page * head_dim * 4 + 4096))) * sms
-    if 0 < cluster and pages <= 4 * cluster:
-        for s in (8, 4, 2):
-            if s <= cluster and pages % s == 0 and s * base_ctas <= (room if s > 2 else room * 4 // 3):
-                return s
-        return 1
-    return max(1, min(pages, room // base_ctas))
+
+    def share(s):     # hundredths of what fits
+        return 75 if s > 6 else 90 if s > 2 else 100
+    s = next((s for s in range(min(cluster, pages), 1, -1) if 100 * s * base_ctas <= share(s) * room), 1)
+    s = fewest_splits(pages, s)
+    if cluster == 0 or -(-pages // s) > 5:
+        fit = max(1, min(pages, room // base_ctas))
+        if fit > cluster:
+            return max(cluster + 1, fewest_splits(pages, fit))
+    return s
 
 
 def latent_splits(ctas: int, pages: int, sms: int) -> int:

@@ -242,6 +242,31 @@ def test_splits_of_the_decode_attention_over_heads_of_64():
                 walk = now
 
 
+def test_splits_of_the_32_bit_decode_attention():
+    """The same in 32-bit: any number of pages, within what is on the GPU at once (three CTAs an SM
+    with heads of 64, one with 128), beyond eight splits only where those would walk far, and without
+    clusters as many as fit."""
+    from nimbus_infer_rs_b200.csrc.ops import decode_splits_f32
+
+    def s(batch, pages, heads=12, hd=64, cluster=8):
+        return decode_splits_f32(batch * heads, pages, 64, hd, 148, cluster)
+    assert [s(1, p) for p in (1, 2, 3, 6, 9, 15, 16, 17, 18, 31, 33)] == [1, 2, 3, 6, 5, 8, 8, 6, 6, 8, 7]
+    assert [s(8, p) for p in (5, 9, 15, 16, 17, 33)] == [3, 3, 4, 4, 4, 4]
+    assert [s(b, 16) for b in (2, 4, 5, 10, 16, 24, 32)] == [8, 6, 6, 3, 2, 1, 1]
+    assert [s(1, p, heads=8, hd=128) for p in (9, 16, 31, 64)] == [5, 8, 8, 16]
+    assert [s(2, p, heads=8, hd=128) for p in (9, 16, 31, 48)] == [5, 6, 9, 9]
+    assert [s(1, p, cluster=0) for p in (1, 3, 9, 16, 33, 100)] == [1, 3, 9, 16, 33, 34]
+    for cluster in (0, 8):
+        for hd in (16, 64, 128):
+            room = {16: 8, 64: 3, 128: 1}[hd] * 148
+            for base in (1, 4, 12, 25, 60, 96, 148, 192, 300, 444, 445, 900):
+                for pages in range(1, 70):
+                    n = decode_splits_f32(base, pages, 64, hd, 148, cluster)
+                    assert 1 <= n <= pages and (n == 1 or n * base <= room)
+                    assert n > 8 or (n - 1) * -(-pages // n) < pages       # the last split has a page
+                    assert n > 1 or pages == 1 or 2 * base > room
+
+
 def test_every_row_of_a_packed_step_says_where_it_belongs():
     """Any batch, any padding: row r of sequence i carries its token, the position
     ``pos0[i] + offset`` and the sequence's slot; ``cu_rows`` cuts the rows into the sequences;
