@@ -750,6 +750,13 @@ TileCost pick_tile(const TileCost (&cost)[COUNT], int M, int N, int K, int pairs
   return best;
 }
 
+template <int COUNT>
+bool has_tile(const TileCost (&cost)[COUNT], int bn, int pair) {
+  for (const TileCost& c : cost)
+    if (c.bn == bn && c.pair == pair) return true;
+  return false;
+}
+
 }  // namespace
 
 // 1 if the tensor-core kernel takes this product.
@@ -765,8 +772,11 @@ NB_EXPORT int nb_gemm_tcgen05_tune(int dual, int lanes) {
   return 0;
 }
 
-// Tuning and tests: a tile width and whether pairs of CTAs take it (0: choose).
+// Tuning and tests: a tile width and whether pairs of CTAs take it (0: choose).  While one is set, products
+// that have no kernel of it (of that result type, of up to 128 rows, with direct stores) are refused.
 NB_EXPORT int nb_gemm_tcgen05_force(int width, int pair) {
+  NB_REQUIRE(width == 0 || has_tile(COST_F32, width, pair) || has_tile(COST_B16, width, pair), NB_ERR_BAD_ARG,
+             "gemm_tcgen05: no tile of %d columns%s", width, pair ? " for pairs of CTAs" : "");
   g_force_bn = width;
   g_force_pair = pair;
   return 0;
@@ -822,6 +832,9 @@ NB_EXPORT int nb_gemm_tcgen05(const void* X, const void* W, const float* bias, c
   // itself; otherwise every thread stores its own row segment.
   const int esize = out_dtype == NB_F32 ? 4 : 2;
   const bool tma_epi = ((long long)N * esize) % 16 == 0 && (residual == nullptr || residual == out);
+  NB_REQUIRE(g_force_bn == 0 || (M > BM && tma_epi && (out_dtype == NB_F32 ? has_tile(COST_F32, g_force_bn, g_force_pair)
+                                                                         : has_tile(COST_B16, g_force_bn, g_force_pair))),
+             NB_ERR_BAD_ARG, "gemm_tcgen05: this product has no kernel of the %d columns that are set", g_force_bn);
   TileCost tile = {M <= BM ? pick_stream_width(N) : 0, 0};
   if (M > BM) {
     if (!tma_epi) tile = pick_tile(COST_DIRECT, M, N, K, 0);

@@ -51,6 +51,22 @@ def test_tiles_of_every_width_with_32_bit_results(ops, width, pair, M, N, K):
     assert (stream.double() - want).abs().max() <= tol + 1e-6 * float(want.abs().max())
 
 
+def test_a_product_without_a_kernel_of_the_width_that_is_set_is_refused(ops):
+    """By the result's type, by its rows (up to 128 take tiles of their own), by rows that TMA cannot store."""
+    x, w = (torch.randn(n, 64, device=DEV).bfloat16() for n in (300, 260))
+    for (width, pair), rows, columns, dtype in (((96, 0), 300, 260, torch.bfloat16), ((192, 0), 300, 260, torch.float32),
+                                                ((128, 0), 100, 260, torch.float32), ((128, 0), 300, 257, torch.float32)):
+        out = torch.zeros(rows, columns, device=DEV, dtype=dtype)
+        assert ops.lib.nb_gemm_tcgen05_force(width, pair) == 0
+        try:
+            with pytest.raises(ops_mod.KernelError):
+                ops._call("nb_gemm_tcgen05", x.data_ptr(), w.data_ptr(), 0, 0, out.data_ptr(), int(dtype == torch.bfloat16),
+                          rows, columns, 64, 0, torch.cuda.current_stream().cuda_stream)
+        finally:
+            ops.lib.nb_gemm_tcgen05_force(0, 0)
+        assert (out == 0).all()
+
+
 @pytest.mark.parametrize("columns", [96, 128])
 @pytest.mark.parametrize("M, N, K", [(65, 95, 64), (128, 97, 520), (129, 193, 1032), (70, 300, 4104)])
 def test_32_bit_products_in_tiles_of_either_width(ops, columns, M, N, K):
