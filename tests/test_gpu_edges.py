@@ -26,7 +26,8 @@ def own_random_numbers():
 
 
 @pytest.mark.parametrize("width, pair", [(96, 1), (128, 1), (192, 1), (256, 1), (96, 0), (128, 0)])
-@pytest.mark.parametrize("M, N, K", [(129, 260, 8), (257, 1600, 136), (511, 52, 640), (2900, 516, 72)])
+@pytest.mark.parametrize("M, N, K", [(129, 260, 8), (257, 1600, 136), (511, 52, 640), (2900, 516, 72), (5000, 2052, 72),
+                                     (5000, 2052, 648)])
 def test_tiles_of_every_width_with_32_bit_results(ops, width, pair, M, N, K):
     """One tile and several a CTA, rows and columns that end inside a 32 x 32 box, K shorter and longer
     than the ring; the residual added in place.  Sums of K products in fp32: 3e-6 of the largest for

@@ -262,13 +262,11 @@ def test_a_row_that_stops_becomes_padding_while_the_others_cross_a_page(model_di
 def test_the_sessions_logits_equal_the_plain_implementations(model_dirs, name, dtype, clusters):
     """Not only ids: after N replayed steps of a session (N chosen so that a page end lies
     behind every row) the logits the session holds are the plain implementation's last-row
-    logits of each sequence, at the tolerance of every other logits test.  In bfloat16 the
+    logits of each sequence, at the tolerance of every other logits test.  The
     splits of a sequence's pages (2 for A, 5 for D) merge inside thread-block clusters, or
     with `clusters` off through scratch memory: both inside the replayed graph."""
     from gpu_helpers import assert_close
     from nimbus_infer_rs_b200.engine.decode import DecodeSession
-    if dtype == "float32" and not clusters:
-        pytest.skip("the 32-bit kernel has one way to merge")
     W = P.PlainWeights(model_dirs[name])
     e = Engine.load(model_dirs[name], dtype=dtype, cache_tokens=4096)
     was = e.ops.decode_clusters
