@@ -5,12 +5,12 @@
 // contiguous) into shared memory with 16-byte cp.async copies, two or four pages in flight (the
 // first ones asked for before the kernel's wait on its predecessor), and all query heads that
 // share the key/value head are served from the same staged page.  Scores, softmax and the
-// weighted sum are fp32; every warp keeps a running (max, sum, accumulator) for its quarter of
-// a page (the bfloat16 kernel has four warps on a page, or eight on two pages at a time), the
-// warps are merged at the end of the split, and the splits are merged either inside a
-// thread-block cluster (2 to 8 splits of the bfloat16 kernel: partial results into the first
-// CTA's shared memory, one cluster barrier) or by whichever CTA of the (row, head) finishes
-// last (a counter in scratch memory that it leaves at zero again).
+// weighted sum are fp32; every warp keeps a running (max, sum, accumulator) for its share of
+// a page (four warps on a page; the bfloat16 kernel also has two on a page, or eight on two pages at
+// a time), the warps are merged at the end of the split, and the splits are merged either inside a
+// thread-block cluster (2 to 8 splits: partial results into the first CTA's shared memory, one
+// cluster barrier) or by whichever CTA of the (row, head) finishes last (a counter in scratch
+// memory that it leaves at zero again).
 //
 // Scratch (caller-allocated): part_acc [rows][heads][splits][head_dim] fp32, part_ml
 // [rows][heads][splits][2] fp32, counters [rows][kv_heads] int32, zero before the first use.
@@ -565,7 +565,7 @@ NB_EXPORT int nb_attention_decode_maps(const void* q, int q_stride, const int* r
                           /*append=*/-1, 0, 0, g_cluster_merge.load(), stream);
 }
 
-// How the splits of the bfloat16 kernel merge: 0 always through the scratch arrays; otherwise
+// How the splits merge: 0 always through the scratch arrays; otherwise
 // (the default) through a cluster's shared memory where there are 2 to 8 of them.  Returns the
 // earlier setting.
 NB_EXPORT int nb_attention_decode_cluster_merge(int mode) {

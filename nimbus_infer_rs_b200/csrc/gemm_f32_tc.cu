@@ -17,7 +17,7 @@
 // added up in registers, rounded, in runs of about sqrt(K / 64) blocks whose sums are added up in turn
 // (one chain of K / 32 additions would round as often as the multiply-adds do).
 //
-// A pass of its own (split_kernel, a warp a row) writes the three pieces of the rows of X and of W
+// A pass of its own (split_kernel, a warp a row, four beyond 1,024 of K) writes the three pieces of the rows of X and of W
 // into scratch memory, every time: nothing is kept from one call to the next.  Rows all of whose numbers
 // are below 2^-30 are split times a power of two that brings the largest into [1, 2), and the result is
 // multiplied back: their small terms would be subnormal, where every cut is of 2^-149 (both operands of
@@ -538,10 +538,12 @@ NB_EXPORT int nb_gemm_f32_tc_supported(int M, int N, int K) {
 // block of 16 of its part of K 1.03 up to 1.75 CTAs an SM, 1.8 up to 3.5, and beyond 0.46 a CTA and SM,
 // or 0.62 where K is cut (clusters leave SMs out); where it leaves K of under 256 to gemm_simt.cu that
 // one's 4 and 0.045 a number of K.  Measured, this kernel and the other:
-// 2024x2304x768 57 and 173, 2024x3072x768 82 and 251, 2024x768x3072 85 and 320, 1000x768x768 30 and 49,
-// 333x2304x768 31 and 48, 200x2304x768 31 and 40, 66x50257x768 155 and 243, 128x4800x1600 70 and 92; but
-// 512x768x768 29 and 26.5, 333x768x768 29 and 23, 997x512x512 23 and 21, 300x1600x6400 202 and 190,
-// 128x768x3072 93 and 30.  Not below 128 of K, where gemm_simt.cu's tiles take as long as a wave here or
+// 2024x2304x768 57 and 173, 2024x3072x768 82 and 251, 2024x768x3072 84 and 320, 1000x768x768 26 and 49,
+// 333x2304x768 27 and 49, 200x2304x768 26 and 40, 66x50257x768 138 and 244, 128x4800x1600 55 and 92,
+// 512x768x3072 76 and 88; but 333x768x768 25 and 23.5, 100x2304x768 25 and 23.6, 256x768x3072 75 and 47,
+// 128x768x3072 74 and 30.  (The line's constants are from before the tiles of 96 columns and rows split in one
+// reading.  It leaves a few to the multiply-adds that are faster here now: 512x768x768 25.3 and 26.7,
+// 997x512x512 19.9 and 21.8, 300x1600x1600 46 and 52, 300x1600x6400 161 and 191.)  Not below 128 of K, where gemm_simt.cu's tiles take as long as a wave here or
 // less (512x768x64 6.8 and 9.5) and, with a step or two of 16, the one cut a step leaves more than the few
 // roundings of multiply-adds (K = 8, one large term a row: 5.7e-8 against 4.8e-8).
 NB_EXPORT int nb_gemm_f32_tc_preferred(int M, int N, int K) {

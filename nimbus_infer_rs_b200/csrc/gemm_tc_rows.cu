@@ -374,10 +374,15 @@ NB_EXPORT int nb_gemm_tc_rows_supported(int M, int N, int K) {
   return plan_rows(M, N, K, &sh) ? 1 : 0;
 }
 
-// 1 where this kernel is the faster one of the two tensor-core products (measured on a B200 at
-// 32, 64 and 128 rows on GPT-2 124M's and XL's shapes): a long K (24 blocks and more) over
-// few columns, where the tiled kernel has few CTAs and each a long walk.  (Measured with the exchange
-// that this kernel had first; with the present one 64x4800x1600 takes 9.7 us, the tiled kernel 9.0.)
+// 1 where this kernel is taken before the tiled one: a long K (24 blocks and more) over few columns,
+// where the tiled kernel has few CTAs and each a long walk.  The line is from measurements with an exchange that
+// this kernel no longer has.  Chains of products over cold weights, 32-bit results added in place (bf16 with
+// GELU), us, here and tiled: 64x2304x1600 7.3 and 9.6 (7.3 and 8.6), 96x4096x3072 11.0 and 17.0 (11.0 and 15.0),
+// 128x4096x6400 17.0 and 32.4; over the 144 shapes between 2,304 and 4,736 columns that it gives this kernel 0.83
+// (0.95) of the tiled one's time.  But it takes some that the tiled kernel is faster at, near its end in columns
+// and at some cuts of K (64x4736x1600 13.7 and 9.9, 96x2304x1600 12.7 and 9.9, 64x3072x2048 13.2 and
+// 11.9), and leaves some beyond it (64x4800x3072 12.4 and 16.9, 128x4800x6400 21.2 and 33.1); up to 64
+// rows gemm_mid.cu is as fast as this kernel or faster at most of them (64x3072x3072 9.9 and 14.8).
 NB_EXPORT int nb_gemm_tc_rows_preferred(int M, int N, int K) {
   RowsShape sh;
   if (!plan_rows(M, N, K, &sh)) return 0;

@@ -187,7 +187,7 @@ class CudaBackend:
         # NIMBUS_B200_F32_TC=0/1/2: 32-bit products as eight products of bf16 pieces on the tensor
         # cores: never / where that is the faster way / wherever it applies
         self.use_f32_tc = int(os.environ.get("NIMBUS_B200_F32_TC", "1") or 1)
-        # NIMBUS_B200_DECODE_CLUSTERS=0: the splits of the bfloat16 decode attention merge through
+        # NIMBUS_B200_DECODE_CLUSTERS=0: the splits of the decode attention merge through
         # scratch memory and a counter instead of a thread-block cluster's shared memory
         self._cluster_limit = int(self.lib.nb_attention_decode_cluster_limit())
         self._sms = torch.cuda.get_device_properties(self._device_index).multi_processor_count
